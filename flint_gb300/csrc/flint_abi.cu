@@ -71,6 +71,218 @@ struct flint_mech_s {
 
 namespace flint {
 
+// Append the fixed-point image (ImageLayout::fix and the f_ offsets) when the
+// mechanism fits it: NASA-7 thermo, reactions whose rate is a product of at most
+// three concentrations a side (with the reverse Gibbs sum over the same
+// factors), non-zero A, and every coefficient and exponent within its format
+// from fix_Tlo <= 600 K up to fix_Thi >= 3000 K.  Coefficients are formed in long double.
+static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, ImageLayout& L,
+                     std::vector<uint8_t>& img) {
+  typedef long double ld;
+  const ld LOG2E = 1.0L / logl(2.0L);
+  const int ns = L.ns, nr = L.nr, S = L.nsp, P = L.nrpad, dummy = fix_dummy(S);
+  L.fix = 0;
+  if (d->nasa9 || nr < 1 || ns > dummy || L.nfall > 16) return;
+  bool ok = true;
+  auto q = [&](ld x, int bits, ld limit) -> int64_t {   // to fixed point, checked against the format's range
+    if (!(fabsl(x) < limit)) { ok = false; return 0; }
+    return (int64_t)llrintl(ldexpl(x, bits));
+  };
+  // ---- species polynomials; t = T / 2^11 below tmid, T / 2^13 above
+  std::vector<int64_t> G(14 * S, 0), H(12 * S, 0), C(10 * S, 0);
+  std::vector<double> tmid(S, 0.0);
+  double Thi = 8192.0;
+  for (int k = 0; k < ns; ++k) {
+    const double* c = d->nasa7 + 17 * k;
+    // a low range that reaches beyond 2048 K serves both sections, up to Thi
+    const bool wide = !(c[1] < 2048.0);
+    tmid[k] = wide ? 2000.0 : c[1];
+    if (wide) Thi = std::min(Thi, c[1]);
+    for (int rg = 0; rg < 2; ++rg) {
+      const double* a = c + 3 + (wide ? 0 : 7 * rg);
+      const ld s = rg == 0 ? 2048.0L : 8192.0L;
+      int64_t* g = &G[7 * rg * S + k];
+      g[0] = q(LOG2E * ((ld)a[0] * (1.0L - logl(1024.0L)) - (ld)a[6]), 52, 1000.0L) - 1;   // -1: the products below floor
+      g[S] = q(a[0], 54, 500.0L);
+      int64_t* h = &H[6 * rg * S + k];
+      int64_t* cp = &C[5 * rg * S + k];
+      h[0] = q(a[0], 52, 1000.0L);
+      cp[0] = h[0];
+      // coefficient of t^j in Q(52 - j) (Q(53 - j) in g, whose polynomial starts
+      // at t): one more integer bit per order, for the steep quartics; every
+      // Horner stage is checked over the range
+      ld sk = 1.0L;
+      for (int j = 1; j <= 4; ++j) {
+        sk *= s;
+        g[(1 + j) * S] = q(LOG2E * a[j] * sk / (j * (j + 1)), 53 - j, ldexpl(1.0L, 9 + j));
+        h[j * S] = q(a[j] * sk / (j + 1), 52 - j, ldexpl(1.0L, 10 + j));
+        cp[j * S] = q(a[j] * sk, 52 - j, ldexpl(1.0L, 10 + j));
+      }
+      g[6 * S] = q(LOG2E * a[5], 45, 260000.0L);
+      h[5 * S] = q(a[5], 45, 260000.0L);
+      const double t0 = (rg == 0 ? 128.0 : tmid[k]) / s, t1 = (rg == 0 ? tmid[k] : Thi) / s;
+      for (int i = 0; i <= 32; ++i) {   // (in double: a check of magnitudes with 10 % to spare)
+        const double t = t0 + (t1 - t0) * i / 32;
+        double sg = 0, sh = 0, sc = 0;
+        for (int j = 4; j >= 0; --j) {
+          if (j) sg = std::ldexp((double)g[(1 + j) * S], j - 53) + t * sg;
+          sh = std::ldexp((double)h[j * S], j - 52) + t * sh;
+          sc = std::ldexp((double)cp[j * S], j - 52) + t * sc;
+          const double lim = 0.9 * (1 << (10 + j));
+          if (!(std::fabs(sg) < lim && std::fabs(sh) < 2 * lim && std::fabs(sc) < 2 * lim)) ok = false;
+        }
+      }
+    }
+  }
+  // ---- reactions
+  std::vector<int64_t> fa(P, 0), fb(P, 0), fe(P, 0), ra(16, 0), rb(16, 0), re(16, 0);
+  std::vector<uint64_t> ix(P, 0);
+  std::vector<double> tr(5 * 16, 0.0);
+  std::vector<std::vector<int>> lists_r(nr), lists_p(nr);
+  bool w3 = false;
+  int tb = 0;
+  for (int rr = 0; rr < nr && ok; ++rr) {
+    const int r = order[rr], t = d->rtype[r];
+    const double A = d->arrh[3 * r], b = d->arrh[3 * r + 1], E = d->arrh[3 * r + 2];
+    if (A == 0.0 || !std::isfinite(A)) ok = false;
+    std::vector<int> rs, ps;
+    for (int s = 0; s < 3; ++s) {
+      const int i = d->rsp[3 * r + s], j = d->psp[3 * r + s];
+      if (i >= 0) {
+        const double o = d->rord[3 * r + s], nu = d->rnu[3 * r + s];
+        if (!(o == 0.0 || o == 1.0 || o == 2.0 || o == 3.0) || (d->reversible[r] && o != nu)) { ok = false; break; }
+        for (int u = 0; u < (int)o; ++u) rs.push_back(i);
+      }
+      if (j >= 0 && d->reversible[r]) {
+        const double nu = d->pnu[3 * r + s];
+        if (!(nu == 0.0 || nu == 1.0 || nu == 2.0 || nu == 3.0)) { ok = false; break; }
+        for (int u = 0; u < (int)nu; ++u) ps.push_back(j);
+      }
+    }
+    if (rs.size() > 3 || ps.size() > 3) ok = false;
+    if (!ok) break;
+    lists_r[rr] = rs; lists_p[rr] = ps;
+    w3 |= rs.size() > 2 || ps.size() > 2;
+    const int dn = d->reversible[r] ? (int)ps.size() - (int)rs.size() : 0;
+    uint64_t w = 0;
+    for (int s = 0; s < 3; ++s) {
+      w |= (uint64_t)(s < (int)rs.size() ? rs[s] : dummy) << (6 * s);
+      w |= (uint64_t)(s < (int)ps.size() ? ps[s] : dummy) << (18 + 6 * s);
+    }
+    w |= (uint64_t)(dn + 8) << 36 | (uint64_t)t << 40 | (uint64_t)(d->reversible[r] ? 1 : 0) << 42 |
+         (uint64_t)(A < 0.0 ? 1 : 0) << 43;
+    if (t) { w |= (uint64_t)tb << 48; ++tb; }
+    ix[rr] = w;
+    // +1.5 units of 2^-52: the mean of the two floored products added to it
+    fa[rr] = q(log2l(fabsl((ld)A)) + 10.0L * (ld)b + ldexpl(1.5L, -52), 52, 2000.0L);
+    fb[rr] = q(b, 55, 250.0L);
+    fe[rr] = q(-LOG2E * (ld)E, 45, 260000.0L);
+    if (t >= 2) {
+      const int i = rr - (nr - L.nfall);
+      const ld A0r = (ld)d->arrh0[3 * r] / (ld)A, b0r = (ld)d->arrh0[3 * r + 1] - (ld)b, E0r = (ld)d->arrh0[3 * r + 2] - (ld)E;
+      if (!(A0r > 0.0L) || A < 0.0) { ok = false; break; }
+      ra[i] = q(log2l(A0r) + 10.0L * b0r + ldexpl(1.5L, -52), 52, 2000.0L);
+      rb[i] = q(b0r, 55, 250.0L);
+      re[i] = q(-LOG2E * E0r, 45, 260000.0L);
+      if (t == 3) {
+        const double* z = d->troe + 4 * r;
+        tr[i] = (double)(1.0L - (ld)z[0]);
+        tr[16 + i] = z[0];
+        tr[32 + i] = (double)(LOG2E / (ld)z[1]);
+        tr[48 + i] = (double)(LOG2E / (ld)z[2]);
+        tr[64 + i] = (double)(LOG2E * (ld)z[3]);
+        for (int u = 0; u < 5; ++u) if (std::isnan(tr[16 * u + i])) ok = false;
+      }
+    }
+  }
+  const ld lC = log2l((ld)d->p_ref / (ld)d->r_thermo) - 10.0L;
+  if (!(fabsl(lC) < 1000.0L)) ok = false;
+  if (!ok) return;
+  // ---- the range of T over which every exponent stays in format (in double:
+  // magnitudes against limits 2 % inside the formats')
+  double Tlo = 1e30;
+  const double l2e = (double)LOG2E, lC0 = (double)(lC + 10.0L);
+  std::vector<double> g(ns), lA(nr), lA0(nr);
+  for (int rr = 0; rr < nr; ++rr) {
+    lA[rr] = std::log2(std::fabs(d->arrh[3 * order[rr]]));
+    lA0[rr] = d->rtype[order[rr]] >= 2 ? std::log2(d->arrh0[3 * order[rr]]) : 0.0;
+  }
+  for (double T = Thi; T >= 125.0; T *= 0.97) {
+    const double lg = std::log2(T);
+    bool in = true;
+    for (int k = 0; k < ns && in; ++k) {
+      const double* c = d->nasa7 + 17 * k;
+      const double* a = c + (T <= c[1] ? 3 : 10);
+      double cp = 0, h = 0, ss = 0, Tj = 1;
+      for (int j = 0; j < 5; ++j) {
+        cp += a[j] * Tj; h += a[j] * Tj / (j + 1); ss += j ? a[j] * Tj / j : a[0] * std::log(T);
+        Tj *= T;
+      }
+      h += a[5] / T; ss += a[6];
+      g[k] = l2e * (h - ss);
+      in = std::fabs(cp) < 1000.0 && std::fabs(h) < 1000.0 && std::fabs(g[k]) < 1000.0;
+    }
+    for (int rr = 0; rr < nr && in; ++rr) {
+      const int r = order[rr];
+      const double f = lA[rr] + d->arrh[3 * r + 1] * lg - l2e * d->arrh[3 * r + 2] / T;
+      double v = 0;
+      if (d->reversible[r]) {
+        for (int i : lists_p[rr]) v += g[i];
+        for (int i : lists_r[rr]) v -= g[i];
+        v -= ((int)lists_p[rr].size() - (int)lists_r[rr].size()) * (lC0 - lg);
+      }
+      in = std::fabs(f) < 2000.0 && std::fabs(v) < 2000.0 && std::fabs(f + v) < 2000.0;
+      if (d->rtype[r] >= 2) {
+        const double f0 = lA0[rr] + d->arrh0[3 * r + 1] * lg - l2e * d->arrh0[3 * r + 2] / T;
+        in = in && std::fabs(f0 - f) < 2000.0;
+      }
+    }
+    if (!in) break;
+    Tlo = T;
+  }
+  if (!(Tlo <= 600.0 && Thi >= 3000.0)) return;
+  L.fix = 1;
+  L.fix_w3 = w3 ? 1 : 0;
+  L.fix_Tlo = std::max(Tlo, 129.0);
+  L.fix_Thi = Thi;
+  L.fix_lC = (int64_t)llrintl(ldexpl(lC, 52));
+  // ---- sections
+  int off = 0;
+  auto sec = [&](int bytes) { int o = off; off = rup(off + bytes, 16); return o; };
+  const int ntbl = (L.o_tbv - L.o_tbs) / 4, nlist = std::max(L.nlist, 1);
+  L.f_mw = sec(8 * S); L.f_invmw = sec(8 * S); L.f_tmid = sec(8 * S);
+  L.f_g = sec(8 * 14 * S); L.f_h = sec(8 * 12 * S); L.f_c = sec(8 * 10 * S);
+  L.f_a = sec(8 * P); L.f_b = sec(8 * P); L.f_e = sec(8 * P); L.f_ix = sec(8 * P);
+  L.f_ra = sec(8 * 16); L.f_rb = sec(8 * 16); L.f_re = sec(8 * 16); L.f_tr = sec(8 * 5 * 16);
+  L.f_tbd = sec(8 * L.ntb); L.f_tbp = sec(4 * (L.ntb + 1)); L.f_tbs = sec(4 * ntbl); L.f_tbv = sec(8 * ntbl);
+  L.f_exp = sec(8 * FIX_EXP2); L.f_log = sec(8 * 2 * FIX_LOG2);
+  L.f_cstart = sec(4 * (S + 1)); L.f_lr = sec(4 * nlist); L.f_lnu = sec(8 * nlist);
+  L.o_fix = L.bytes;
+  L.fix_bytes = off;
+  img.resize((size_t)L.bytes + off, 0);
+  uint8_t* F = img.data() + L.o_fix;
+  auto put = [&](int o, const void* src, size_t bytes) { memcpy(F + o, src, bytes); };
+  put(L.f_mw, img.data() + L.o_mw, 8 * S);
+  put(L.f_invmw, img.data() + L.o_invmw, 8 * S);
+  put(L.f_tmid, tmid.data(), 8 * S);
+  put(L.f_g, G.data(), 8 * G.size()); put(L.f_h, H.data(), 8 * H.size()); put(L.f_c, C.data(), 8 * C.size());
+  put(L.f_a, fa.data(), 8 * P); put(L.f_b, fb.data(), 8 * P); put(L.f_e, fe.data(), 8 * P); put(L.f_ix, ix.data(), 8 * P);
+  put(L.f_ra, ra.data(), 8 * 16); put(L.f_rb, rb.data(), 8 * 16); put(L.f_re, re.data(), 8 * 16);
+  put(L.f_tr, tr.data(), 8 * 5 * 16);
+  put(L.f_tbd, img.data() + L.o_tbd, 8 * L.ntb); put(L.f_tbp, img.data() + L.o_tbp, 4 * (L.ntb + 1));
+  put(L.f_tbs, img.data() + L.o_tbs, 4 * ntbl); put(L.f_tbv, img.data() + L.o_tbv, 8 * (size_t)((L.o_cstart - L.o_tbv) / 8));
+  put(L.f_cstart, img.data() + L.o_cstart, 4 * (S + 1)); put(L.f_lr, img.data() + L.o_lr, 4 * nlist);
+  put(L.f_lnu, img.data() + L.o_lnu, 8 * nlist);
+  int64_t* et = reinterpret_cast<int64_t*>(F + L.f_exp);
+  for (int j = 0; j < FIX_EXP2; ++j) et[j] = (int64_t)llrintl(ldexpl(exp2l((j + 0.5L) / FIX_EXP2), 62));
+  int64_t* lt = reinterpret_cast<int64_t*>(F + L.f_log);
+  for (int j = 0; j < FIX_LOG2; ++j) {
+    const uint64_t c = (uint64_t)ldexpl(1.0L / (1.0L + (j + 0.5L) / FIX_LOG2), 64);
+    lt[2 * j] = (int64_t)c;
+    lt[2 * j + 1] = (int64_t)llrintl(ldexpl(-log2l(ldexpl((ld)c, -64)), 62));
+  }
+}
+
 // Pack a mechanism description into the device image (see ImageLayout).
 static int pack(const flint_mech_desc* d, ImageLayout& L, std::vector<uint8_t>& img) {
   const int ns = d->ns, nr = d->nr;
@@ -252,6 +464,7 @@ static int pack(const flint_mech_desc* d, ImageLayout& L, std::vector<uint8_t>& 
     D(L.o_logtab)[3 * j + 1] = hi;
     D(L.o_logtab)[3 * j + 2] = (double)(l - (long double)hi);
   }
+  pack_fix(d, order, L, img);
   return FLINT_OK;
 }
 

@@ -16,6 +16,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "flint_fix.cuh"
 
 namespace flint {
 
@@ -68,6 +69,21 @@ struct ImageLayout {
   int nfall;                     // falloff reactions (the last nfall after sorting; <= 16)
   int o_nasa9;                   // NASA-9 thermo [32][nsp] (nranges, T0..T3, 3 x 9 coefficients); -1 = none
   int o_logtab;                  // double [129][3]: c_j ~ 1/(1 + j/128), -ln c_j as hi + lo (flog)
+  // Fixed-point image (flint_fix.cuh, flint_fixkin.cuh): present when fix != 0,
+  // at o_fix, 16-byte aligned, fix_bytes long; the f_ offsets are relative to
+  // o_fix.  `bytes` above counts the FP64 sections only.
+  int fix, o_fix, fix_bytes;
+  int fix_w3;                    // some reaction has a third factor on a side
+  double fix_Tlo, fix_Thi;       // cells with T in [fix_Tlo, fix_Thi) take the fixed-point path
+  int64_t fix_lC;                // log2(p_ref / r_thermo) - 10, Q52
+  int f_mw, f_invmw, f_tmid;     // [nsp]
+  int f_g, f_h, f_c;             // int64 [2][7][nsp], [2][6][nsp], [2][5][nsp]: g/RT (octaves), h/RT, cp/R; low, high range
+  int f_a, f_b, f_e, f_ix;       // int64 [nrpad]: log2|A| + 10 b, b, -E log2e; packed indices (fix_ix_*)
+  int f_ra, f_rb, f_re;          // int64 [16]: k0/kinf of the falloff reactions
+  int f_tr;                      // double [5][16]: 1 - a, a, log2e/T3, log2e/T1, T2 log2e (0: none)
+  int f_tbd, f_tbp, f_tbs, f_tbv;   // as the o_ ones
+  int f_exp, f_log;              // int64 [256], [128][2]
+  int f_cstart, f_lr, f_lnu;     // as the o_ ones
 };
 
 struct MechView {
@@ -284,8 +300,13 @@ struct WarpScratch {
 // 31 species, in a per-warp slot of global memory (L2-resident) for 32-63.
 // The falloff pre-pass of a Jacobian evaluation uses Jr (written only after the
 // rates of progress are done).
+// c, hRT and gRT have two more entries than species slots: the fixed-point path
+// reads index `dummy` (c = 1, g = 0) for a missing reactant or product.
+__host__ __device__ inline int species_stride(int nsp) { return nsp + 2; }
+// (63 rather than 64 for the larger size: the packed index has 6 bits, and 63 species leave slot 63 free)
+__host__ __device__ inline int fix_dummy(int nsp) { return nsp == 64 ? 63 : nsp; }
 __host__ __device__ inline int scratch_small_doubles(int nsp, int nrpad) {
-  return (3 * nsp + nrpad + 8 * 32 + 1) & ~1;   // keep 16-byte alignment
+  return (3 * species_stride(nsp) + nrpad + 8 * 32 + 1) & ~1;   // keep 16-byte alignment
 }
 __host__ __device__ inline int scratch_jac_doubles(int nsp, int nrpad) {
   return (8 * nrpad + (nsp + 1) * (nsp + 1) + 1) & ~1;
@@ -295,12 +316,14 @@ __host__ __device__ inline int scratch_jac_doubles(int nsp, int nrpad) {
 // calls without the Jacobian (in the Jacobian call it lives in Jr), and dq only
 // inside a Jacobian call, so the two may share (8 nrpad >= 256 doubles).
 __host__ __device__ inline int scratch_doubles(int nsp, int nrpad, bool jac) {
-  return jac ? ((3 * nsp + nrpad + 8 * nrpad + (nsp + 1) * (nsp + 1) + 1) & ~1) : scratch_small_doubles(nsp, nrpad);
+  return jac ? ((3 * species_stride(nsp) + nrpad + 8 * nrpad + (nsp + 1) * (nsp + 1) + 1) & ~1)
+             : scratch_small_doubles(nsp, nrpad);
 }
 
 __device__ inline WarpScratch carve2(double* small, double* jacbuf, int nsp, int nrpad) {
   WarpScratch s;
-  s.c = small; s.hRT = small + nsp; s.gRT = small + 2 * nsp; s.q = small + 3 * nsp;
+  const int ss = species_stride(nsp);
+  s.c = small; s.hRT = small + ss; s.gRT = small + 2 * ss; s.q = small + 3 * ss;
   s.fo = s.q + nrpad;
   s.ldj = nsp + 1;
   s.dq = jacbuf;
@@ -310,7 +333,7 @@ __device__ inline WarpScratch carve2(double* small, double* jacbuf, int nsp, int
 
 // Both parts contiguous in one buffer (shared memory, up to 31 species).
 __device__ inline WarpScratch carve(double* p, int nsp, int nrpad, bool jac) {
-  return carve2(p, jac ? p + 3 * nsp + nrpad : nullptr, nsp, nrpad);
+  return carve2(p, jac ? p + 3 * species_stride(nsp) + nrpad : nullptr, nsp, nrpad);
 }
 
 // Cell-level results held per lane: lane k (< ns) gets species k, the T-row

@@ -1,0 +1,470 @@
+// flint_fixkin.cuh -- warp-per-cell kinetics on the fixed-point image.
+//
+// The same quantities as warp_kinetics (flint_dev.cuh), with every exponent,
+// exponential and logarithm and the thermo polynomials in 64-bit fixed point
+// (flint_fix.cuh).  What remains on the FP64 pipe per cell: the concentrations,
+// four products per reaction round, the falloff blend, the species sums, and
+// (JAC) the Jacobian.  A mechanism without the fixed-point image, and a cell
+// outside its temperature range, go through warp_kinetics.
+#pragma once
+#include "flint_dev.cuh"
+
+namespace flint {
+
+// Index word of a reaction: bits 0-17 three reactant factors, 18-35 three
+// product factors (6 bits each, `dummy` where absent), 36-39 dn + 8, 40-41
+// type, 42 reversible, 43 A < 0, 48-55 third-body row.
+__device__ __forceinline__ int fix_type(uint64_t w) { return (int)(w >> 40) & 3; }
+__device__ __forceinline__ bool fix_rev(uint64_t w) { return (w >> 42) & 1; }
+__device__ __forceinline__ int fix_tbrow(uint64_t w) { return (int)(w >> 48) & 0xff; }
+__device__ __forceinline__ int fix_idx(uint64_t w, int slot) { return (int)(w >> (6 * slot)) & 63; }
+__device__ __forceinline__ int fix_dn(uint64_t w) { return ((int)(w >> 36) & 15) - 8; }
+
+struct FixView {
+  int ns, nr, nrpad, nsp, nfall, dummy, w3;
+  double inv_r_eos, r_eos, r_thermo, Tlo, Thi;
+  int64_t lC;
+  const double *mw, *invmw, *tr, *tbd, *tbv, *lnu;
+  const int64_t *tmid, *g, *h, *c, *a, *b, *e, *ra, *rb, *re, *et, *lt;
+  const uint64_t* ix;
+  const int *tbp, *tbs, *cstart, *lr;
+  __device__ __forceinline__ void bind(const ImageLayout& L, const uint8_t* base) {
+    ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; nfall = L.nfall; dummy = fix_dummy(L.nsp); w3 = L.fix_w3;
+    inv_r_eos = L.inv_r_eos; r_eos = L.r_eos; r_thermo = L.r_thermo; Tlo = L.fix_Tlo; Thi = L.fix_Thi; lC = L.fix_lC;
+    auto D = [&](int o) { return (const double*)(base + o); };
+    auto I = [&](int o) { return (const int64_t*)(base + o); };
+    mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv); lnu = D(L.f_lnu);
+    tmid = I(L.f_tmid); g = I(L.f_g); h = I(L.f_h); c = I(L.f_c); a = I(L.f_a); b = I(L.f_b); e = I(L.f_e);
+    ra = I(L.f_ra); rb = I(L.f_rb); re = I(L.f_re); et = I(L.f_exp); lt = I(L.f_log);
+    ix = (const uint64_t*)(base + L.f_ix);
+    tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
+    cstart = (const int*)(base + L.f_cstart); lr = (const int*)(base + L.f_lr);
+  }
+  __device__ __forceinline__ bool covers(double T) const { return T >= Tlo && T < Thi; }
+};
+
+// Sum over the warp in 64-bit integers: every lane's value aligned to the
+// largest exponent of the warp (58 bits below it), three 32-bit warp reductions
+// of its 24-bit pieces, one rounding at the end.  The result is the exact sum to
+// 2^-57 of the largest term, the same on every lane, with no FP64 instruction
+// (the FP64 butterfly took five DADDs of 19 cycles and ten shuffles).
+static __device__ __noinline__ double warp_sum_slow(double v) { return warp_sum(v); }
+__device__ __forceinline__ double warp_isum(double v) {
+  const int64_t b = __double_as_longlong(v);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  const unsigned emax = __reduce_max_sync(FULL, e);
+  if (emax - 128u > 1900u) return warp_sum_slow(v);   // zeros, subnormal, huge, inf, NaN
+  int64_t m = (b & 0xfffffffffffffll) | (e ? ONE52 : 0);
+  const unsigned sh = emax - (e ? e : 1u);
+  m = sh < 58 ? (m << 5) >> sh : 0;
+  m = b < 0 ? -m : m;
+  const unsigned lo = __reduce_add_sync(FULL, (unsigned)m & 0xffffffu);
+  const unsigned mi = __reduce_add_sync(FULL, (unsigned)(m >> 24) & 0xffffffu);
+  const int hi = __reduce_add_sync(FULL, (int)(m >> 48));
+  const int64_t S = ((int64_t)hi << 48) + ((int64_t)mi << 24) + (int64_t)lo;
+  return fix2d(S, 1080 - (int)emax);
+}
+
+// Polynomial c0 + t (c1 + t (...)) in t (Q63); coefficients (stride S) in Q52,
+// Q51, Q50, ... by order (see pack_fix), the result in Q52.
+template <int N>
+__device__ __forceinline__ int64_t fix_poly(const int64_t* __restrict__ c, int S, int64_t t) {
+  int64_t a = c[(N - 1) * S];
+#pragma unroll
+  for (int j = N - 2; j >= 0; --j) a = c[j * S] + (mulhi_s(a, t) << 2);
+  return a;
+}
+
+__device__ __forceinline__ double fix_tb_conc(const FixView& m, int t, double ctot, const double* c) {
+  double M = m.tbd[t] * ctot;
+  for (int e = m.tbp[t]; e < m.tbp[t + 1]; ++e) M = fma(m.tbv[e], c[m.tbs[e]], M);
+  return M;
+}
+
+// Constants of the Troe blend with all logarithms in octaves (base 2): x = log Pr
+// - 0.4 - 0.67 log Fc, n = 0.75 - 1.27 log Fc, den = n - 0.14 x and log F = log Fc
+// den^2 / (den^2 + x^2); x, n and den carry the factor log2(10), which cancels.
+constexpr int64_t TROE_C40 = 5984253652114523ll;        // 0.40 log2(10)  Q52
+constexpr int64_t TROE_C75 = 11220475597714730ll;       // 0.75 log2(10)  Q52
+constexpr int64_t TROE_M67 = 6179659264692699791ll;     // 0.67  Q63
+constexpr int64_t TROE_M127 = 5856841243402782638ll;    // 1.27  Q62
+constexpr int64_t TROE_M14 = 1291272085159668613ll;     // 0.14  Q63
+
+// One cell (see warp_kinetics for the meaning of pr, cv and s.Jr).  RHS: form
+// out.f and out.fT; want_h: form out.cp_mass and out.h_mass.  img: the global
+// image, for the Jacobian's FP64 coefficients.
+template <bool JAC, int SPL, bool RHS>
+__device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
+                                             const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
+                                             double pr, CellOutT<SPL>& out, bool cv, bool want_h) {
+  const int ns = m.ns, nsp = m.nsp, nrpad = m.nrpad;
+  const bool thermo = JAC || RHS || want_h;
+  int64_t* G = reinterpret_cast<int64_t*>(s.gRT);
+  double yw[SPL];
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    yw[j] = k < ns ? Yk[j] * m.invmw[k] : 0.0;
+  }
+  const double sumYW = warp_isum(SPL == 1 ? yw[0] : yw[0] + yw[SPL - 1]);
+  const FixT f = fix_T(T, m.lt);
+  const double X = T * sumYW;
+  const double rho = cv ? pr : pr * m.inv_r_eos * recip(X);
+  const double ctot = rho * sumYW;
+  // ---- species k = lane + 32 j
+  double my_cpR[SPL], my_hRT[SPL], my_c[SPL];
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    my_cpR[j] = 0.0; my_hRT[j] = 0.0; my_c[j] = 0.0;
+    int64_t gk = 0;
+    double ck = k == m.dummy ? 1.0 : 0.0;
+    if (k < ns) {
+      ck = rho * yw[j];
+      my_c[j] = ck;
+      const bool lo = __double_as_longlong(T) <= m.tmid[k];
+      const int64_t t = lo ? f.t11 : f.t13;
+      const int64_t* c = m.g + (lo ? 0 : 7 * nsp) + k;
+      gk = c[0] - (mulhi_s(c[nsp], f.L) << 1) - (mulhi_s(fix_poly<4>(c + 2 * nsp, nsp, t), t) << 1) +
+           (mulhi_s(c[6 * nsp], f.v) << 1);
+      if (thermo) {
+        const int64_t* h = m.h + (lo ? 0 : 6 * nsp) + k;
+        my_hRT[j] = fix2d(fix_poly<5>(h, nsp, t) + (mulhi_s(h[5 * nsp], f.v) << 1), 52);
+        my_cpR[j] = fix2d(fix_poly<5>(m.c + (lo ? 0 : 5 * nsp) + k, nsp, t), 52);
+      }
+    }
+    if (k < nsp) {
+      s.c[k] = ck;
+      G[k] = gk;
+      if (JAC) s.hRT[k] = my_hRT[j];
+    }
+  }
+  if (lane == 0 && m.dummy == nsp) { s.c[nsp] = 1.0; G[nsp] = 0; if (JAC) s.hRT[nsp] = 0.0; }
+  __syncwarp();
+  double invT = 0.0;
+  const double *gb = nullptr, *gE = nullptr, *gb0 = nullptr, *gE0 = nullptr;   // FP64 Arrhenius data (JAC)
+  if (JAC) {
+    invT = recip(T);
+    gb = (const double*)(img + L.o_b); gE = (const double*)(img + L.o_E);
+    gb0 = (const double*)(img + L.o_b0); gE0 = (const double*)(img + L.o_E0);
+  }
+  // ---- falloff: the last nfall reactions (<= 16), as in warp_kinetics.  Pass 1
+  // spreads their five exponentials each over the lanes, pass 2 forms M, Pr and
+  // Fcent on lane i, pass 3 takes log2 of Fcent (lane i) and Pr (lane nfall + i)
+  // together, pass 4 blends.
+  const int NF = m.nfall, f0 = m.nr - NF;
+  double* fo = JAC ? s.Jr : s.fo;
+  if (NF > 0) {
+    const double Tinv = JAC ? invT : fix2d(f.v, 70);
+    for (int jb = lane; jb < 5 * NF; jb += WARP) {
+      const int i = jb / 5, kind = jb - 5 * i, r = f0 + i;
+      int64_t x;
+      double keep = 1.0;
+      if (kind < 2) {
+        const int64_t a = kind == 0 ? m.a[r] : m.ra[i], b = kind == 0 ? m.b[r] : m.rb[i], e = kind == 0 ? m.e[r] : m.re[i];
+        x = a + mulhi_s(b, f.L) + (mulhi_s(e, f.v) << 1);
+      } else {
+        const double z = m.tr[16 * kind + i];      // log2e/T3, log2e/T1, T2 log2e
+        x = -d2fix52(z * (kind == 4 ? Tinv : T));
+        if (kind == 4 && z == 0.0) keep = 0.0;
+      }
+      const double v = exp2_q52(x, m.et);
+      fo[kind * WARP + i] = keep != 0.0 ? v : 0.0;
+    }
+    __syncwarp();
+    double Pr = 1.0, Fc = 1.0, kinf = 0.0, kratio = 0.0;
+    bool troe = false;
+    if (lane < NF) {
+      const uint64_t w = m.ix[f0 + lane];
+      troe = fix_type(w) == 3;
+      kinf = fo[lane];
+      kratio = fo[WARP + lane];
+      Pr = kratio * fix_tb_conc(m, fix_tbrow(w), ctot, s.c);
+      if (troe) Fc = fma(m.tr[lane], fo[2 * WARP + lane], fma(m.tr[16 + lane], fo[3 * WARP + lane], fo[4 * WARP + lane]));
+    }
+    const double Pr_src = __shfl_sync(FULL, Pr, lane >= NF && lane < 2 * NF ? lane - NF : 0);
+    double lg_in = lane < NF ? Fc : (lane < 2 * NF ? Pr_src : 1.0);
+    lg_in = lg_in > 1e-300 ? lg_in : 1e-300;
+    // octaves; Pr = inf or NaN gives a finite garbage exponent, and the NaN of
+    // Pr / (1 + Pr) below makes the rate NaN as before
+    const int64_t lg = log2_q52(lg_in, m.lt);
+    const int64_t lgP = __shfl_sync(FULL, lg, lane < NF ? lane + NF : 0);
+    if (lane < NF) {
+      double Fb = 1.0, R = 0.0, dx = 0.0, dden = 1.0, Qr = 1.0, lgd = 0.0, nnd = 0.0;
+      if (troe) {
+        const int64_t xx = lgP - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
+        const int64_t nn = TROE_C75 - (mulhi_s(lg, TROE_M127) << 2);
+        const int64_t den = nn - (mulhi_s(xx, TROE_M14) << 1);
+        dx = fix2d(xx, 52);
+        dden = fix2d(den, 52);
+        lgd = fix2d(lg, 52);
+        const double d2 = dden * dden;
+        Qr = recip(fma(dx, dx, d2));
+        R = d2 * Qr;
+        Fb = exp2_q52(d2fix52(lgd * R), m.et);
+        if (JAC) nnd = fix2d(nn, 52);
+      }
+      const double iopr = recip(1.0 + Pr);
+      fo[5 * WARP + lane] = kinf * (Pr * iopr) * Fb;
+      if (JAC) {
+        const int r = f0 + lane;
+        const double dlnkinf = fma(gE[r], invT, gb[r]) * invT, dlnPr = fma(gE0[r], invT, gb0[r]) * invT;
+        double Gf = 0.0, dlnF_T = 0.0;
+        if (troe) {
+          // d ln F: with f1 = x/den, Aq = 2 lgF f1 / ((1 + f1^2)^2 den^2) and
+          // 1 + f1^2 = (den^2 + x^2)/den^2; lgF, x, n, den all carry the factor
+          // log2(10), and Aq n, Aq x are free of it
+          const double iden = recip(dden);
+          const double f1 = dx * iden;
+          const double Aq = 2.0 * lgd * f1 * (R * R) * (iden * iden);
+          Gf = -Aq * nnd;
+          const double e3 = fo[2 * WARP + lane], e1 = fo[3 * WARP + lane], e2 = fo[4 * WARP + lane];
+          constexpr double LN2 = 0.6931471805599453;
+          const double k3 = m.tr[32 + lane] * LN2, k1 = m.tr[48 + lane] * LN2, k2 = m.tr[64 + lane] * LN2;
+          const double dFc = -m.tr[lane] * k3 * e3 - m.tr[16 + lane] * k1 * e1 + k2 * invT * invT * e2;
+          dlnF_T = (R + Aq * (0.67 * nnd - 1.27 * dx)) * dFc / Fc;
+        }
+        fo[6 * WARP + lane] = dlnkinf + dlnPr * iopr + Gf * dlnPr + dlnF_T;
+        fo[7 * WARP + lane] = kinf * Fb * iopr * (iopr + Gf) * kratio;
+      }
+    }
+    __syncwarp();
+  }
+  // ---- reactions: rates of progress
+  for (int r = lane; r < nrpad; r += WARP) {
+    double q = 0.0;
+    if (r < m.nr) {
+      const uint64_t w = m.ix[r];
+      const int type = fix_type(w);
+      const bool rev = fix_rev(w);
+      const int r0 = fix_idx(w, 0), r1 = fix_idx(w, 1), p0 = fix_idx(w, 3), p1 = fix_idx(w, 4);
+      const double c0 = s.c[r0], c1 = s.c[r1], d0 = s.c[p0], d1 = s.c[p1];
+      int64_t a = m.a[r] + mulhi_s(m.b[r], f.L) + (mulhi_s(m.e[r], f.v) << 1);
+      a = type >= 2 ? 0 : a;
+      // 1/Kc = 2^(dG - dn log2(p_ref/RT)), kr = kf / Kc
+      int64_t ar = a + G[p0] + G[p1] - G[r0] - G[r1] - (int64_t)fix_dn(w) * (m.lC - (f.L >> 9));
+      double c2 = 1.0, d2 = 1.0;
+      if (m.w3) {
+        const int r2 = fix_idx(w, 2), p2 = fix_idx(w, 5);
+        ar += G[p2] - G[r2];
+        c2 = s.c[r2];
+        d2 = s.c[p2];
+      }
+      double kf = exp2_q52(a, m.et);
+      double kr = rev ? exp2_q52(ar, m.et) : 0.0;
+      const int sgn = ((int)(w >> 43) & 1) << 31;
+      kf = __hiloint2double(__double2hiint(kf) ^ sgn, __double2loint(kf));
+      kr = __hiloint2double(__double2hiint(kr) ^ sgn, __double2loint(kr));
+      const double iKc = kr;                      // (falloff reactions: a = 0)
+      double Mfac = 1.0;
+      if (type == 1) {
+        Mfac = fix_tb_conc(m, fix_tbrow(w), ctot, s.c);
+      } else if (type >= 2) {
+        kf = fo[5 * WARP + r - f0];
+        kr *= kf;
+      }
+      double Pf = c0 * c1, Pr = d0 * d1;
+      if (m.w3) { Pf *= c2; Pr *= d2; }
+      const double fwd = kf * Pf;
+      q = fma(-kr, Pr, fwd);
+      if (JAC) {
+        const double kfM = type == 1 ? kf * Mfac : kf, krM = type == 1 ? kr * Mfac : kr;
+        s.dq[r] = kfM * c1;
+        s.dq[nrpad + r] = kfM * c0;
+        s.dq[3 * nrpad + r] = -krM * d1;
+        s.dq[4 * nrpad + r] = -krM * d0;
+        if (m.w3) {
+          s.dq[r] *= c2;
+          s.dq[nrpad + r] *= c2;
+          s.dq[2 * nrpad + r] = kfM * (c0 * c1);
+          s.dq[3 * nrpad + r] *= d2;
+          s.dq[4 * nrpad + r] *= d2;
+          s.dq[5 * nrpad + r] = -krM * (d0 * d1);
+        }
+        double dlnk, tb = 0.0;
+        if (type >= 2) {
+          dlnk = fo[6 * WARP + r - f0];
+          tb = fo[7 * WARP + r - f0] * fma(-iKc, Pr, Pf);
+        } else {
+          dlnk = fma(gE[r], invT, gb[r]) * invT;
+          if (type == 1) tb = q;
+        }
+        double dH = s.hRT[p0] + s.hRT[p1] - s.hRT[r0] - s.hRT[r1];
+        if (m.w3) dH += s.hRT[fix_idx(w, 5)] - s.hRT[fix_idx(w, 2)];
+        const double dlnKc = rev ? (dH - (double)fix_dn(w)) * invT : 0.0;
+        // fwd dlnk - rvs (dlnk - dlnKc) = q dlnk + rvs dlnKc
+        s.dq[6 * nrpad + r] = tb;
+        s.dq[7 * nrpad + r] = Mfac * fma(q, dlnk, kr * Pr * dlnKc);
+      }
+      if (type == 1) q *= Mfac;
+    }
+    s.q[r] = q;
+  }
+  __syncwarp();
+  // ---- species: production rates
+  const double cvone = cv ? 1.0 : 0.0;
+  double wm[SPL];
+  double Ql = 0.0, Dl = 0.0, cpl = 0.0, hl = 0.0;
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    wm[j] = 0.0;
+    if (k < ns) {
+      for (int e = m.cstart[k]; e < m.cstart[k + 1]; ++e) wm[j] = fma(m.lnu[e], s.q[m.lr[e]], wm[j]);
+      if (RHS || JAC) {
+        // constant volume: u_k/RT = h_k/RT - 1, cv_k/R = cp_k/R - 1
+        Ql = fma(cv ? my_hRT[j] - 1.0 : my_hRT[j], wm[j], Ql);
+        Dl = fma(my_c[j], cv ? my_cpR[j] - 1.0 : my_cpR[j], Dl);
+      }
+      if (want_h) {
+        cpl = fma(yw[j], my_cpR[j], cpl);
+        hl = fma(yw[j], my_hRT[j], hl);
+      }
+    }
+    out.wmol[j] = wm[j];
+  }
+  out.rho = rho;
+  if (want_h) {
+    out.cp_mass = warp_isum(cpl) * m.r_thermo;
+    out.h_mass = warp_isum(hl) * m.r_thermo * T;
+  }
+  if (!RHS && !JAC) return;
+  const double Q = warp_isum(Ql), D = warp_isum(Dl);
+  const double invD = recip(D);
+  const double fT = -T * Q * invD;
+  const double irho = recip(rho);
+  out.fT = fT;
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    out.cpR[j] = my_cpR[j];
+    out.f[j] = (k < ns) ? m.mw[k] * wm[j] * irho : (k == ns ? fT : 0.0);
+  }
+  if (!JAC) return;
+
+  // ---- Jacobian in concentration space: row k = species k ------------------
+  const int ld = s.ldj, nslot = m.w3 ? 3 : 2;
+  double JT[SPL];
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    JT[j] = 0.0;
+    if (k < ns) {
+      double* Jrow = s.Jr + k * ld;
+      for (int jj = 0; jj < ns; ++jj) Jrow[jj] = 0.0;
+      double tball = 0.0;   // third-body terms common to every column
+      for (int e = m.cstart[k]; e < m.cstart[k + 1]; ++e) {
+        const int r = m.lr[e];
+        const double nu = m.lnu[e];
+        const uint64_t w = m.ix[r];
+        for (int sl = 0; sl < nslot; ++sl) {
+          const int sp = fix_idx(w, sl), sq = fix_idx(w, 3 + sl);
+          if (sp != m.dummy) Jrow[sp] = fma(nu, s.dq[sl * nrpad + r], Jrow[sp]);
+          if (sq != m.dummy) Jrow[sq] = fma(nu, s.dq[(3 + sl) * nrpad + r], Jrow[sq]);
+        }
+        if (fix_type(w) != 0) {
+          const double t = nu * s.dq[6 * nrpad + r];
+          const int row = fix_tbrow(w);
+          tball = fma(t, m.tbd[row], tball);
+          for (int q = m.tbp[row]; q < m.tbp[row + 1]; ++q) Jrow[m.tbs[q]] = fma(t, m.tbv[q], Jrow[m.tbs[q]]);
+        }
+        JT[j] = fma(nu, s.dq[7 * nrpad + r], JT[j]);
+      }
+      if (tball != 0.0)
+        for (int jj = 0; jj < ns; ++jj) Jrow[jj] += tball;
+    }
+  }
+  __syncwarp();
+  // S_k = sum_j c_j Jc[k][j] (row k); HJ_m = sum_k hRT_k Jc[k][m] (column m)
+  double Sk[SPL], HJ[SPL];
+  double HSl = 0.0, dQTl = 0.0, dDTl = 0.0;
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    Sk[j] = 0.0; HJ[j] = 0.0;
+    if (k < ns) {
+      const double* Jrow = s.Jr + k * ld;
+      const double* a = (const double*)(img + L.o_nasa) + (__double_as_longlong(T) <= m.tmid[k] ? 0 : 7 * nsp) + k;
+      const double dcp = a[nsp] + T * (2.0 * a[2 * nsp] + T * (3.0 * a[3 * nsp] + T * 4.0 * a[4 * nsp]));
+      if (cv) {
+        // rho fixed: no dependence of c on T or through rho on Y (Sk = 0)
+        for (int kk = 0; kk < ns; ++kk) HJ[j] += (s.hRT[kk] - 1.0) * s.Jr[kk * ld + k];
+        dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + (my_hRT[j] - 1.0) * JT[j];
+        dDTl += my_c[j] * dcp;
+      } else {
+        for (int jj = 0; jj < ns; ++jj) Sk[j] = fma(s.c[jj], Jrow[jj], Sk[j]);
+        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk], s.Jr[kk * ld + k], HJ[j]);
+        HSl += my_hRT[j] * Sk[j];
+        dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + my_hRT[j] * (JT[j] - Sk[j] * invT);
+        dDTl += my_c[j] * (dcp - my_cpR[j] * invT);
+      }
+    }
+  }
+  const double HS = warp_isum(HSl);
+  __syncwarp();
+  const double wbar = recip(sumYW);
+  const double wr = cv ? 0.0 : wbar * irho;
+  const double dQT = warp_isum(dQTl), dDT = warp_isum(dDTl);
+  const double QD = Q * invD, TD = T * invD;
+  const double JTT = -QD - TD * (dQT - QD * dDT);
+  double JTm[SPL];
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    JTm[j] = 0.0;
+    if (k < ns) {
+      const double rw = rho * m.invmw[k], ww = cv ? 0.0 : wbar * m.invmw[k];
+      const double dQ = rw * HJ[j] - ww * HS;
+      const double dD = rw * (my_cpR[j] - cvone) - ww * D;
+      JTm[j] = -TD * (dQ - QD * dD);
+      // species row k in (Y, T) variables
+      const double tk = Sk[j] - wm[j];
+      const double Wk = m.mw[k];
+      const double wt = wr * tk;
+      double* Jrow = s.Jr + k * ld;
+      for (int jj = 0; jj < ns; ++jj) Jrow[jj] = Wk * m.invmw[jj] * (Jrow[jj] - wt);
+      Jrow[ns] = (Wk * irho) * (cv ? JT[j] : JT[j] - tk * invT);
+    }
+  }
+  __syncwarp();
+  // T row (row ns)
+  double* JrowT = s.Jr + ns * ld;
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) {
+    const int k = lane + 32 * j;
+    if (k < ns) JrowT[k] = JTm[j];
+  }
+  if (lane == 0) JrowT[ns] = JTT;
+  __syncwarp();
+}
+
+// The FP64 path of one cell for kernels whose shared memory holds the
+// fixed-point image: the mechanism is read from global memory.
+template <bool JAC, int SPL>
+__device__ __noinline__ void kinetics_general(const uint8_t* __restrict__ img, const ImageLayout& L,
+                                              const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
+                                              double pr, CellOutT<SPL>& out, bool cv) {
+  MechView g;
+  g.bind(L, img);
+  warp_kinetics<JAC, SPL>(g, s, lane, Yk, T, pr, out, cv);
+}
+
+// The fixed-point path where the cell's temperature allows it.
+template <bool JAC, int SPL, bool RHS>
+__device__ __forceinline__ void kinetics_cell(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
+                                              const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
+                                              double pr, CellOutT<SPL>& out, bool cv, bool want_h) {
+  if (m.covers(T)) {
+    kinetics_fix<JAC, SPL, RHS>(m, img, L, s, lane, Yk, T, pr, out, cv, want_h);
+  } else {
+    CellOutT<SPL> o;
+    double yk[SPL];
+#pragma unroll
+    for (int j = 0; j < SPL; ++j) yk[j] = Yk[j];
+    WarpScratch sc = s;
+    kinetics_general<JAC, SPL>(img, L, sc, lane, yk, T, pr, o, cv);
+    out = o;
+  }
+}
+
+}  // namespace flint

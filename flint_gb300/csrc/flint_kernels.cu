@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <atomic>
 #include "flint_dev.cuh"
+#include "flint_fixkin.cuh"
 #include "flint_host.h"
 
 namespace flint {
@@ -144,30 +145,37 @@ k_wdot_small(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, int layo
 // ---------------------------------------------------------------- warp
 // SPL species per lane; GJ: the Jacobian work area is a per-warp slot of
 // global memory (mechanisms of 33-63 species, and smaller ones whose shared
-// memory layout would not fit a block).
-template <bool JAC, int SPL, bool GJ>
-__global__ void __launch_bounds__(WARP_THREADS)
-k_wdot_warp(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, int layout,
+// memory layout would not fit a block).  FIX: the fixed-point kinetics
+// (flint_fixkin.cuh); the block then stages only that image.  RHS: rhs_out is
+// wanted.
+template <bool JAC, int SPL, bool GJ, bool FIX, bool RHS>
+__global__ void __launch_bounds__(WARP_THREADS, JAC ? 1 : 2)
+k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, int layout,
             const double* __restrict__ Tg, const double* __restrict__ pg,
             const double* __restrict__ Yg, double* __restrict__ wdot, double* __restrict__ cpo,
             double* __restrict__ ho, double* __restrict__ jac, double* __restrict__ rhs_out,
             double* __restrict__ gscratch, int cv) {
   extern __shared__ __align__(16) uint8_t smem[];
-  stage_image(smem, img, L.bytes);
+  const int base = FIX ? L.fix_bytes : L.bytes;
+  stage_image(smem, FIX ? img + L.o_fix : img, base);
   MechView m;
-  m.bind(L, smem);
+  FixView x;
+  if (FIX) x.bind(L, smem);
+  else m.bind(L, smem);
+  const double* mw = FIX ? x.mw : m.mw;
+  const int nsp = L.nsp, nrpad = L.nrpad;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpScratch s;
   if (!GJ) {
-    const int sd = scratch_doubles(m.nsp, m.nrpad, JAC);
-    s = carve(reinterpret_cast<double*>(smem + L.bytes) + wid * sd, m.nsp, m.nrpad, JAC);
+    const int sd = scratch_doubles(nsp, nrpad, JAC);
+    s = carve(reinterpret_cast<double*>(smem + base) + wid * sd, nsp, nrpad, JAC);
   } else {
-    const int sd = scratch_small_doubles(m.nsp, m.nrpad);
+    const int sd = scratch_small_doubles(nsp, nrpad);
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
-    s = carve2(reinterpret_cast<double*>(smem + L.bytes) + wid * sd,
-               JAC ? gscratch + gw * scratch_jac_doubles(m.nsp, m.nrpad) : nullptr, m.nsp, m.nrpad);
+    s = carve2(reinterpret_cast<double*>(smem + base) + wid * sd,
+               JAC ? gscratch + gw * scratch_jac_doubles(nsp, nrpad) : nullptr, nsp, nrpad);
   }
-  const int ns = m.ns, nv = ns + 1;
+  const int ns = L.ns, nv = ns + 1;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t cell = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid; cell < n; cell += nwarps) {
     const double T = Tg[cell], p = pg[cell];
@@ -179,16 +187,17 @@ k_wdot_warp(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, int layou
       if (k < ns) Yk[j] = (layout == 1) ? Yg[(int64_t)k * n + cell] : Yg[cell * ns + k];
     }
     CellOutT<SPL> o;
-    warp_kinetics<JAC, SPL>(m, s, lane, Yk, T, p, o, cv != 0);
+    if (FIX) kinetics_cell<JAC, SPL, RHS>(x, img, L, s, lane, Yk, T, p, o, cv != 0, cpo != nullptr || ho != nullptr);
+    else warp_kinetics<JAC, SPL>(m, s, lane, Yk, T, p, o, cv != 0);
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int k = lane + 32 * j;
       if (wdot && k < ns) {
-        const double v = m.mw[k] * o.wmol[j];
+        const double v = mw[k] * o.wmol[j];
         if (layout == 1) wdot[(int64_t)k * n + cell] = v;
         else wdot[cell * ns + k] = v;
       }
-      if (rhs_out && k < nv) rhs_out[cell * nv + k] = o.f[j];
+      if (RHS && k < nv) rhs_out[cell * nv + k] = o.f[j];
     }
     if (lane == 0) {
       if (cpo) cpo[cell] = o.cp_mass;
@@ -385,18 +394,21 @@ size_t small_smem(const ImageLayout& L) { return L.bytes + 3 * SMALL_NSMAX * SMA
 // Jacobian work area in global memory: 33-63 species, or a shared-memory
 // layout too large for a block of 256 threads (the choice does not depend on
 // the block size a caller tunes, so one kernel serves every block size).
+// The image a block of the warp kernels stages.
+static size_t image_bytes(const ImageLayout& L) { return L.fix ? L.fix_bytes : L.bytes; }
 static bool warp_gj(const ImageLayout& L, bool jac) {
   if (L.nsp > 32) return true;
   if (!jac) return false;
-  return L.bytes + (WARP_THREADS / 32) * scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) > device_smem_optin();
+  return image_bytes(L) + (WARP_THREADS / 32) * scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) >
+         device_smem_optin();
 }
 
 static int warp_block(int threads) { return threads == 64 || threads == 128 ? threads : WARP_THREADS; }
 
 size_t warp_smem(const ImageLayout& L, bool jac, int threads) {
   const int wpb = warp_block(threads) / 32;
-  if (warp_gj(L, jac)) return L.bytes + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
-  return L.bytes + wpb * scratch_doubles(L.nsp, L.nrpad, jac) * sizeof(double);
+  if (warp_gj(L, jac)) return image_bytes(L) + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
+  return image_bytes(L) + wpb * scratch_doubles(L.nsp, L.nrpad, jac) * sizeof(double);
 }
 
 int warp_block_candidates(int* out) {
@@ -404,10 +416,14 @@ int warp_block_candidates(int* out) {
   return 3;
 }
 
-template <bool JAC>
-static const void* warp_fn(const ImageLayout& L) {
-  if (L.nsp > 32) return (const void*)k_wdot_warp<JAC, 2, true>;
-  return warp_gj(L, JAC) ? (const void*)k_wdot_warp<JAC, 1, true> : (const void*)k_wdot_warp<JAC, 1, false>;
+typedef void (*WarpKernel)(const uint8_t*, ImageLayout, int64_t, int, const double*, const double*, const double*,
+                           double*, double*, double*, double*, double*, double*, int);
+
+template <bool JAC, bool RHS>
+static WarpKernel warp_fn(const ImageLayout& L) {
+  if (L.nsp > 32) return L.fix ? k_wdot_warp<JAC, 2, true, true, RHS> : k_wdot_warp<JAC, 2, true, false, RHS>;
+  if (JAC && warp_gj(L, JAC)) return L.fix ? k_wdot_warp<JAC, 1, true, true, RHS> : k_wdot_warp<JAC, 1, true, false, RHS>;
+  return L.fix ? k_wdot_warp<JAC, 1, false, true, RHS> : k_wdot_warp<JAC, 1, false, false, RHS>;
 }
 
 // Global Jacobian work area needed by the warp kernels (doubles), for a grid
@@ -415,7 +431,7 @@ static const void* warp_fn(const ImageLayout& L) {
 // (enough for the resident warps of every block size)
 int64_t warp_jac_scratch_doubles(const ImageLayout& L) {
   if (!warp_gj(L, true)) return 0;
-  const void* fn = warp_fn<true>(L);
+  const void* fn = (const void*)warp_fn<true, false>(L);
   int64_t most = 0;
   int cand[4];
   const int nc = warp_block_candidates(cand);
@@ -430,27 +446,19 @@ int64_t warp_jac_scratch_doubles(const ImageLayout& L) {
   return most * scratch_jac_doubles(L.nsp, L.nrpad);
 }
 
-template <bool JAC>
+template <bool JAC, bool RHS>
 static cudaError_t launch_warp(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
                                const double* p, const double* Y, double* wdot, double* cp, double* h, double* jac,
                                double* rhs, double* gscratch, cudaStream_t st, int cv = 0, int threads = 0) {
   const int bt = warp_block(threads);
   size_t sm = warp_smem(L, JAC, bt);
-  const void* fn = warp_fn<JAC>(L);
-  cudaError_t e = set_smem(fn, sm);
+  const WarpKernel fn = warp_fn<JAC, RHS>(L);
+  cudaError_t e = set_smem((const void*)fn, sm);
   if (e != cudaSuccess) return e;
   const bool gj = warp_gj(L, JAC);
   if (gj && JAC && !gscratch) return cudaErrorInvalidValue;
-  int64_t g = grid_for(fn, bt, sm, n * 32);
-  if (L.nsp > 32)
-    k_wdot_warp<JAC, 2, true><<<(unsigned)g, bt, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, jac, rhs,
-                                                            gscratch, cv);
-  else if (gj)
-    k_wdot_warp<JAC, 1, true><<<(unsigned)g, bt, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, jac, rhs,
-                                                            gscratch, cv);
-  else
-    k_wdot_warp<JAC, 1, false><<<(unsigned)g, bt, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, jac, rhs,
-                                                             nullptr, cv);
+  int64_t g = grid_for((const void*)fn, bt, sm, n * 32);
+  fn<<<(unsigned)g, bt, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, jac, rhs, gj ? gscratch : nullptr, cv);
   count_launch();
   return cudaGetLastError();
 }
@@ -469,7 +477,7 @@ cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int
     count_launch();
     return cudaGetLastError();
   }
-  return launch_warp<false>(img, L, n, layout, T, p, Y, wdot, cp, h, nullptr, nullptr, nullptr, st, 0, threads);
+  return launch_warp<false, false>(img, L, n, layout, T, p, Y, wdot, cp, h, nullptr, nullptr, nullptr, st, 0, threads);
 }
 
 cudaError_t launch_thermo(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
@@ -510,14 +518,14 @@ cudaError_t launch_wdot_jac(const uint8_t* img, const ImageLayout& L, int64_t n,
                             const double* p, const double* Y, double* wdot, double* jac, double* gscratch,
                             cudaStream_t st, int cv, int threads) {
   if (n <= 0) return cudaSuccess;
-  return launch_warp<true>(img, L, n, layout, T, p, Y, wdot, nullptr, nullptr, jac, nullptr, gscratch, st, cv,
-                           threads);
+  return launch_warp<true, false>(img, L, n, layout, T, p, Y, wdot, nullptr, nullptr, jac, nullptr, gscratch, st, cv,
+                                  threads);
 }
 
 cudaError_t launch_rhs(const uint8_t* img, const ImageLayout& L, int64_t n, const double* T, const double* p,
                        const double* Y, double* f, cudaStream_t st, int cv) {
   if (n <= 0) return cudaSuccess;
-  return launch_warp<false>(img, L, n, 0, T, p, Y, nullptr, nullptr, nullptr, nullptr, f, nullptr, st, cv);
+  return launch_warp<false, true>(img, L, n, 0, T, p, Y, nullptr, nullptr, nullptr, nullptr, f, nullptr, st, cv);
 }
 
 }  // namespace flint

@@ -30,6 +30,7 @@
 #include <mutex>
 
 #include "flint_dev.cuh"
+#include "flint_fixkin.cuh"
 #include "flint_host.h"
 
 namespace flint {
@@ -208,12 +209,14 @@ __device__ inline void warp_lu_solve(const double* A, int ld, int nv, int lane, 
 // pivot step to pivs[32 SPL + row].  Inlined: an out-of-line version (to keep
 // the Newton loop's code compact) measured 3 % slower on the 31-species
 // workload and equal on the 54-species one.
-template <int SPL>
-__device__ __forceinline__ void refresh_newton_matrix(MechView m, WarpScratch s, int lane, double p, bool cv,
+template <int SPL, bool FIX>
+__device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const FixView& x,
+                                                   const uint8_t* __restrict__ img, const ImageLayout& L,
+                                                   const WarpScratch& s, int lane, double p, bool cv,
                                                    double gamma, int eval_J, double ya, double yb, double* Jg,
                                                    int* pivs) {
   constexpr int JW = 32 * SPL;
-  const int ns = m.ns, nv = ns + 1, ld = s.ldj;
+  const int ns = L.ns, nv = ns + 1, ld = s.ldj;
   const int Tslot = ns >> 5, Tlane = ns & 31;
   if (eval_J) {
     const double Tv = __shfl_sync(FULL, (SPL == 1 || Tslot == 0) ? ya : yb, Tlane);
@@ -221,7 +224,8 @@ __device__ __forceinline__ void refresh_newton_matrix(MechView m, WarpScratch s,
     yk[0] = (lane < ns) ? ya : 0.0;
     if (SPL > 1) yk[SPL - 1] = (lane + 32 < ns) ? yb : 0.0;
     CellOutT<SPL> co;
-    warp_kinetics<true, SPL>(m, s, lane, yk, Tv, p, co, cv);
+    if (FIX) kinetics_cell<true, SPL, false>(x, img, L, s, lane, yk, Tv, p, co, cv, false);
+    else warp_kinetics<true, SPL>(m, s, lane, yk, Tv, p, co, cv);
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int r = lane + 32 * j;
@@ -260,8 +264,11 @@ __device__ __forceinline__ void refresh_newton_matrix(MechView m, WarpScratch s,
 // memory (SPL = 1 and the block fits), or in the warp's global slot (GJ).
 static int spl_of(const ImageLayout& L) { return L.nsp / 32; }
 
+// The image a block stages.
+static size_t staged_bytes(const ImageLayout& L) { return L.fix ? L.fix_bytes : L.bytes; }
+
 static size_t reactor_smem_spl1(const ImageLayout& L) {
-  return L.bytes + (REACTOR_THREADS / 32) * (scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) + 64 * sizeof(int));
+  return staged_bytes(L) + (REACTOR_THREADS / 32) * (scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) + 64 * sizeof(int));
 }
 
 // layout: REACTOR_LAYOUT_AUTO picks shared memory whenever the block fits;
@@ -284,18 +291,23 @@ static int64_t reactor_slot_doubles_of(const ImageLayout& L, int layout = REACTO
   return (int64_t)(32 * spl) * (32 * spl) + (reactor_gj(L, layout) ? scratch_jac_doubles(L.nsp, L.nrpad) : 0);
 }
 
-template <int SPL, bool GJ, int MINB = 1>
+template <int SPL, bool GJ, int MINB, bool FIX>
 __global__ void __launch_bounds__(REACTOR_THREADS, MINB)
-k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __restrict__ Tg,
+k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, double* __restrict__ Tg,
           const double* __restrict__ pg, double* __restrict__ Yg, const double* __restrict__ dtg,
           flint_reactor_opts o, int* __restrict__ status_g, int* __restrict__ nsteps_g,
           unsigned long long* __restrict__ counter, double* __restrict__ jsave, int64_t slot_doubles,
           const unsigned long long* __restrict__ n_dev) {
   extern __shared__ __align__(16) uint8_t smem[];
   if (n_dev) n = min(n, (int64_t)*n_dev);   // cell count produced on the device
-  stage_image(smem, img, L.bytes);
+  const int base = FIX ? L.fix_bytes : L.bytes;
+  stage_image(smem, FIX ? img + L.o_fix : img, base);
   MechView m;
-  m.bind(L, smem);
+  FixView x;
+  if (FIX) x.bind(L, smem);
+  else m.bind(L, smem);
+  const double* invmw = FIX ? x.invmw : m.invmw;
+  const int nsp = L.nsp, nrpad = L.nrpad;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t slot = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
   double* Jg = jsave + slot * slot_doubles;
@@ -303,17 +315,17 @@ k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __r
   WarpScratch s;
   int* pivs;
   if (!GJ) {
-    const int sd = scratch_doubles(m.nsp, m.nrpad, true);
-    double* wbase = reinterpret_cast<double*>(smem + L.bytes) + wid * sd;
-    s = carve(wbase, m.nsp, m.nrpad, true);
-    pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + L.bytes) + (blockDim.x >> 5) * sd) + wid * 64;
+    const int sd = scratch_doubles(nsp, nrpad, true);
+    double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
+    s = carve(wbase, nsp, nrpad, true);
+    pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
   } else {
-    const int sd = scratch_small_doubles(m.nsp, m.nrpad);
-    double* wbase = reinterpret_cast<double*>(smem + L.bytes) + wid * sd;
-    s = carve2(wbase, Jg + JW * JW, m.nsp, m.nrpad);
-    pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + L.bytes) + (blockDim.x >> 5) * sd) + wid * 64 * SPL;
+    const int sd = scratch_small_doubles(nsp, nrpad);
+    double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
+    s = carve2(wbase, Jg + JW * JW, nsp, nrpad);
+    pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64 * SPL;
   }
-  const int ns = m.ns, nv = ns + 1;
+  const int ns = L.ns, nv = ns + 1;
   const double inv_nv = 1.0 / nv;
   const int ld = s.ldj;
   const BdfL& B = c_bdf;
@@ -347,8 +359,8 @@ k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __r
       double yw = 0.0;
 #pragma unroll
       for (int j = 0; j < SPL; ++j)
-        if (lane + 32 * j < ns) yw += y[j] * m.invmw[lane + 32 * j];
-      pr = p / (m.r_eos * T0 * warp_sum(yw));
+        if (lane + 32 * j < ns) yw += y[j] * invmw[lane + 32 * j];
+      pr = p / (L.r_eos * T0 * warp_sum(yw));
     }
     int status = FLINT_CELL_OK, nst = 0;
     if (bad) status = FLINT_CELL_NAN_INPUT;
@@ -380,7 +392,8 @@ k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __r
         double yk[SPL];
 #pragma unroll
         for (int j = 0; j < SPL; ++j) yk[j] = (lane + 32 * j < ns) ? yv[j] : 0.0;
-        warp_kinetics<false, SPL>(m, s, lane, yk, Tv, pr, co, cv);
+        if (FIX) kinetics_cell<false, SPL, true>(x, img, L, s, lane, yk, Tv, pr, co, cv, false);
+        else warp_kinetics<false, SPL>(m, s, lane, yk, Tv, pr, co, cv);
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < SPL; ++j) fo[j] = co.f[j];
@@ -453,7 +466,7 @@ k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __r
               ++n_jac;
               have_J = 1; jfresh = 1; nstJ = nst; need_J = 0;
             }
-            refresh_newton_matrix<SPL>(m, s, lane, pr, cv, gamma, eval_J, ypred[0], ypred[SPL - 1], Jg, pivs);
+            refresh_newton_matrix<SPL, FIX>(m, x, img, L, s, lane, pr, cv, gamma, eval_J, ypred[0], ypred[SPL - 1], Jg, pivs);
 #pragma unroll
             for (int j = 0; j < SPL; ++j) mystep[j] = pivs[32 * SPL + lane + 32 * j];
             ++n_lu;
@@ -625,20 +638,29 @@ k_reactor(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, double* __r
 
 size_t reactor_smem(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
   if (!reactor_gj(L, layout)) return reactor_smem_spl1(L);
-  return L.bytes + (reactor_threads(layout) / 32) *
+  return staged_bytes(L) + (reactor_threads(layout) / 32) *
                        (scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double) + 64 * spl_of(L) * sizeof(int));
 }
 
-static const void* reactor_fn(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
+typedef void (*ReactorKernel)(const uint8_t*, ImageLayout, int64_t, double*, const double*, double*, const double*,
+                              flint_reactor_opts, int*, int*, unsigned long long*, double*, int64_t,
+                              const unsigned long long*);
+
+template <bool FIX>
+static ReactorKernel reactor_kernel(const ImageLayout& L, int layout) {
   const bool two = layout == REACTOR_LAYOUT_GLOBAL2B;
-  if (spl_of(L) > 1) return two ? (const void*)k_reactor<2, true, 2> : (const void*)k_reactor<2, true>;
-  if (two) return (const void*)k_reactor<1, true, 2>;
-  return reactor_gj(L, layout) ? (const void*)k_reactor<1, true> : (const void*)k_reactor<1, false>;
+  if (spl_of(L) > 1) return two ? k_reactor<2, true, 2, FIX> : k_reactor<2, true, 1, FIX>;
+  if (two) return k_reactor<1, true, 2, FIX>;
+  return reactor_gj(L, layout) ? k_reactor<1, true, 1, FIX> : k_reactor<1, false, 1, FIX>;
+}
+
+static ReactorKernel reactor_fn(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
+  return L.fix ? reactor_kernel<true>(L, layout) : reactor_kernel<false>(L, layout);
 }
 
 static int slots_of(const ImageLayout& L, int layout) {
   size_t sm = reactor_smem(L, layout);
-  const void* fn = reactor_fn(L, layout);
+  const void* fn = (const void*)reactor_fn(L, layout);
   if (set_smem(fn, sm) != cudaSuccess) return 0;
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, reactor_threads(layout), sm);
@@ -694,7 +716,8 @@ cudaError_t launch_reactor(const uint8_t* img, const ImageLayout& L, int64_t n, 
   if (spl_of(L) < 1 || spl_of(L) > 2) return cudaErrorInvalidValue;
   NvtxRange nvtx("reactor.advance");
   size_t sm = reactor_smem(L, layout);
-  const void* fn = reactor_fn(L, layout);
+  const ReactorKernel kern = reactor_fn(L, layout);
+  const void* fn = (const void*)kern;
   cudaError_t e = set_smem(fn, sm);
   if (e != cudaSuccess) return e;
   const int threads = reactor_threads(layout), wpb = threads / 32;
@@ -713,21 +736,7 @@ cudaError_t launch_reactor(const uint8_t* img, const ImageLayout& L, int64_t n, 
   if (e != cudaSuccess) return e;
   const int64_t sd = reactor_slot_doubles_of(L, layout);
   unsigned long long* wc = reinterpret_cast<unsigned long long*>(work_counter);
-  if (layout == REACTOR_LAYOUT_GLOBAL2B && spl_of(L) > 1)
-    k_reactor<2, true, 2><<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc,
-                                                                          jsave, sd, n_dev);
-  else if (layout == REACTOR_LAYOUT_GLOBAL2B)
-    k_reactor<1, true, 2><<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc,
-                                                                          jsave, sd, n_dev);
-  else if (spl_of(L) > 1)
-    k_reactor<2, true><<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc,
-                                                                       jsave, sd, n_dev);
-  else if (reactor_gj(L, layout))
-    k_reactor<1, true><<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc,
-                                                                       jsave, sd, n_dev);
-  else
-    k_reactor<1, false><<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc,
-                                                                        jsave, sd, n_dev);
+  kern<<<(unsigned)blocks, threads, sm, st>>>(img, L, n, T, p, Y, dt, o, status, nsteps, wc, jsave, sd, n_dev);
   count_launch();
   return cudaGetLastError();
 }
@@ -791,7 +800,7 @@ cudaError_t launch_reactor_noalloc_prepare(const ImageLayout& L) {
   if (e != cudaSuccess) return e;
   e = ensure_bdf_table();
   if (e != cudaSuccess) return e;
-  return set_smem(reactor_fn(L), reactor_smem(L));
+  return set_smem((const void*)reactor_fn(L), reactor_smem(L));
 }
 
 cudaError_t launch_reactor_noalloc(const uint8_t* img, const ImageLayout& L, int64_t n, double* T, const double* p,
