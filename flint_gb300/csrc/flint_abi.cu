@@ -71,6 +71,62 @@ struct flint_mech_s {
 
 namespace flint {
 
+// The constant tables of the exponentials and logarithms, formed once per
+// process in long double (at least 64 significant bits on either host).
+struct MathTables {
+  double exp2[256];                 // 2^(j/256), for fexp
+  double log[3 * 129];              // flog: c_j = 1/(1 + j/128) rounded to double, -ln c_j as hi + lo
+  uint64_t exp2_fix[FIX_EXP2];      // flint_fix.cuh
+  uint64_t log2_fix[2 * FIX_LOG2];
+  MathTables() {
+    for (int j = 0; j < 256; ++j) exp2[j] = (double)exp2l((long double)j / 256.0L);
+    for (int j = 0; j <= 128; ++j) {
+      const double c = (double)(1.0L / (1.0L + (long double)j / 128.0L));
+      const long double l = -logl((long double)c);
+      log[3 * j] = c;
+      log[3 * j + 1] = (double)l;
+      log[3 * j + 2] = (double)(l - (long double)log[3 * j + 1]);
+    }
+    for (int j = 0; j < FIX_EXP2; ++j)   // + half a unit of the double's last place
+      exp2_fix[j] = (uint64_t)llrintl(ldexpl(exp2l((long double)j / FIX_EXP2), 62)) + 512;
+    for (int j = 0; j < FIX_LOG2; ++j) {
+      const uint64_t c = (uint64_t)ldexpl(1.0L / (1.0L + (long double)j / FIX_LOG2), 63) + 1;
+      log2_fix[2 * j] = c;
+      log2_fix[2 * j + 1] = (uint64_t)llrintl(ldexpl(-log2l(ldexpl((long double)c, -63)), 62));
+    }
+  }
+};
+
+static const MathTables& math_tables() {
+  static const MathTables t;
+  return t;
+}
+
+// Class of an elementary reaction for the thread-per-cell kernel: 0 reversible
+// and 1 irreversible with one or two factors on each side, integer coefficients
+// equal to the orders, A > 0 and no species on both sides; 2 anything else.
+static int plain_class(const flint_mech_desc* d, int r) {
+  if (d->rtype[r] != 0 || !(d->arrh[3 * r] > 0.0)) return 2;
+  int nl = 0, np = 0;
+  for (int s = 0; s < 3; ++s) {
+    const int i = d->rsp[3 * r + s], j = d->psp[3 * r + s];
+    if (i >= 0) {
+      const double nu = d->rnu[3 * r + s];
+      if (nu != d->rord[3 * r + s] || !(nu == 1.0 || nu == 2.0)) return 2;
+      nl += (int)nu;
+    }
+    if (j >= 0) {
+      const double nu = d->pnu[3 * r + s];
+      if (!(nu == 1.0 || nu == 2.0)) return 2;
+      np += (int)nu;
+    }
+    for (int u = 0; u < 3; ++u)
+      if (i >= 0 && i == d->psp[3 * r + u]) return 2;
+  }
+  if (nl > 2 || np > 2) return 2;
+  return d->reversible[r] ? 0 : 1;
+}
+
 // Append the fixed-point image (ImageLayout::fix and the f_ offsets) when the
 // mechanism fits it: NASA-7 thermo, reactions whose rate is a product of at most
 // three concentrations a side (with the reverse Gibbs sum over the same
@@ -88,6 +144,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
     if (!(fabsl(x) < limit)) { ok = false; return 0; }
     return (int64_t)llrintl(ldexpl(x, bits));
   };
+  // a factor of mulhi_u: signed, with its sign bit flipped
+  auto flip = [](int64_t x) { return (int64_t)((uint64_t)x ^ 0x8000000000000000ull); };
   // ---- species polynomials; t = T / 2^11 below tmid, T / 2^13 above
   std::vector<int64_t> G(14 * S, 0), H(12 * S, 0), C(10 * S, 0);
   std::vector<double> tmid(S, 0.0);
@@ -102,35 +160,41 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
       const double* a = c + 3 + (wide ? 0 : 7 * rg);
       const ld s = rg == 0 ? 2048.0L : 8192.0L;
       int64_t* g = &G[7 * rg * S + k];
-      g[0] = q(LOG2E * ((ld)a[0] * (1.0L - logl(1024.0L)) - (ld)a[6]), 52, 1000.0L) - 1;   // -1: the products below floor
-      g[S] = q(a[0], 54, 500.0L);
+      // log2 T - 7 = L: -a0 ln T log2e = -a0 (L + 7); + 1: half of the floored products' sum
+      g[0] = q(LOG2E * ((ld)a[0] - (ld)a[6]) - 7.0L * (ld)a[0], 52, 1000.0L);
+      g[S] = flip(q(a[0], 55, 250.0L));
       int64_t* h = &H[6 * rg * S + k];
       int64_t* cp = &C[5 * rg * S + k];
       h[0] = q(a[0], 52, 1000.0L);
       cp[0] = h[0];
-      // coefficient of t^j in Q(52 - j) (Q(53 - j) in g, whose polynomial starts
+      // coefficient of t^j in Q(52 - j) (Q(54 - j) in g, whose polynomial starts
       // at t): one more integer bit per order, for the steep quartics; every
       // Horner stage is checked over the range
       ld sk = 1.0L;
       for (int j = 1; j <= 4; ++j) {
         sk *= s;
-        g[(1 + j) * S] = q(LOG2E * a[j] * sk / (j * (j + 1)), 53 - j, ldexpl(1.0L, 9 + j));
-        h[j * S] = q(a[j] * sk / (j + 1), 52 - j, ldexpl(1.0L, 10 + j));
-        cp[j * S] = q(a[j] * sk, 52 - j, ldexpl(1.0L, 10 + j));
+        g[(1 + j) * S] = q(LOG2E * a[j] * sk / (j * (j + 1)), 54 - j, ldexpl(1.0L, 9 + j));
+        h[j * S] = q(a[j] * sk / (j + 1), 52 - j, ldexpl(1.0L, 11 + j));
+        cp[j * S] = q(a[j] * sk, 52 - j, ldexpl(1.0L, 11 + j));
       }
-      g[6 * S] = q(LOG2E * a[5], 45, 260000.0L);
-      h[5 * S] = q(a[5], 45, 260000.0L);
+      g[6 * S] = flip(q(LOG2E * a[5], 46, 130000.0L));
+      h[5 * S] = flip(q(a[5], 46, 130000.0L));
       const double t0 = (rg == 0 ? 128.0 : tmid[k]) / s, t1 = (rg == 0 ? tmid[k] : Thi) / s;
       for (int i = 0; i <= 32; ++i) {   // (in double: a check of magnitudes with 10 % to spare)
         const double t = t0 + (t1 - t0) * i / 32;
         double sg = 0, sh = 0, sc = 0;
         for (int j = 4; j >= 0; --j) {
-          if (j) sg = std::ldexp((double)g[(1 + j) * S], j - 53) + t * sg;
+          if (j) sg = std::ldexp((double)g[(1 + j) * S], j - 54) + t * sg;
           sh = std::ldexp((double)h[j * S], j - 52) + t * sh;
           sc = std::ldexp((double)cp[j * S], j - 52) + t * sc;
-          const double lim = 0.9 * (1 << (10 + j));
-          if (!(std::fabs(sg) < lim && std::fabs(sh) < 2 * lim && std::fabs(sc) < 2 * lim)) ok = false;
+          const double lim = 0.9 * (1 << (11 + j));
+          if (!(std::fabs(sg) < 0.25 * lim && std::fabs(sh) < lim && std::fabs(sc) < lim)) ok = false;
         }
+      }
+      for (int j = 1; j <= 4; ++j) {
+        g[(1 + j) * S] = flip(g[(1 + j) * S]);
+        h[j * S] = flip(h[j * S]);
+        cp[j * S] = flip(cp[j * S]);
       }
     }
   }
@@ -173,17 +237,17 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
          (uint64_t)(A < 0.0 ? 1 : 0) << 43;
     if (t) { w |= (uint64_t)tb << 48; ++tb; }
     ix[rr] = w;
-    // +1.5 units of 2^-52: the mean of the two floored products added to it
-    fa[rr] = q(log2l(fabsl((ld)A)) + 10.0L * (ld)b + ldexpl(1.5L, -52), 52, 2000.0L);
-    fb[rr] = q(b, 55, 250.0L);
-    fe[rr] = q(-LOG2E * (ld)E, 45, 260000.0L);
+    // + 1 unit of 2^-52: about the mean of what the two floored products lose
+    fa[rr] = q(log2l(fabsl((ld)A)) + 7.0L * (ld)b, 52, 2000.0L) + 1;
+    fb[rr] = flip(q(b, 55, 250.0L));
+    fe[rr] = flip(q(-LOG2E * (ld)E, 45, 260000.0L));
     if (t >= 2) {
       const int i = rr - (nr - L.nfall);
       const ld A0r = (ld)d->arrh0[3 * r] / (ld)A, b0r = (ld)d->arrh0[3 * r + 1] - (ld)b, E0r = (ld)d->arrh0[3 * r + 2] - (ld)E;
       if (!(A0r > 0.0L) || A < 0.0) { ok = false; break; }
-      ra[i] = q(log2l(A0r) + 10.0L * b0r + ldexpl(1.5L, -52), 52, 2000.0L);
-      rb[i] = q(b0r, 55, 250.0L);
-      re[i] = q(-LOG2E * E0r, 45, 260000.0L);
+      ra[i] = q(log2l(A0r) + 7.0L * b0r, 52, 2000.0L) + 1;
+      rb[i] = flip(q(b0r, 55, 250.0L));
+      re[i] = flip(q(-LOG2E * E0r, 45, 260000.0L));
       if (t == 3) {
         const double* z = d->troe + 4 * r;
         tr[i] = (double)(1.0L - (ld)z[0]);
@@ -195,13 +259,13 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
       }
     }
   }
-  const ld lC = log2l((ld)d->p_ref / (ld)d->r_thermo) - 10.0L;
+  const ld lC = log2l((ld)d->p_ref / (ld)d->r_thermo) - 7.0L;
   if (!(fabsl(lC) < 1000.0L)) ok = false;
   if (!ok) return;
   // ---- the range of T over which every exponent stays in format (in double:
   // magnitudes against limits 2 % inside the formats')
   double Tlo = 1e30;
-  const double l2e = (double)LOG2E, lC0 = (double)(lC + 10.0L);
+  const double l2e = (double)LOG2E, lC0 = (double)(lC + 7.0L);
   std::vector<double> g(ns), lA(nr), lA0(nr);
   for (int rr = 0; rr < nr; ++rr) {
     lA[rr] = std::log2(std::fabs(d->arrh[3 * order[rr]]));
@@ -246,6 +310,45 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   L.fix_Tlo = std::max(Tlo, 129.0);
   L.fix_Thi = Thi;
   L.fix_lC = (int64_t)llrintl(ldexpl(lC, 52));
+  // ---- thread-per-cell kernel: row offsets of the plain reactions' factors
+  std::vector<uint64_t> cx(P, 0), cy(P, 0);
+  L.fix_plain_rev = L.fix_plain_irr = 0;
+  for (int rr = 0; rr < nr; ++rr) {
+    const int r = order[rr], cls = plain_class(d, r);
+    if (cls > 1) break;
+    ++(cls == 0 ? L.fix_plain_rev : L.fix_plain_irr);
+    int slot[4] = {ns, ns, ns, ns}, a = 0, b = 2;
+    for (int s = 0; s < 3; ++s) {
+      for (int u = 0; d->rsp[3 * r + s] >= 0 && u < (int)d->rnu[3 * r + s]; ++u) slot[a++] = d->rsp[3 * r + s];
+      for (int u = 0; d->psp[3 * r + s] >= 0 && u < (int)d->pnu[3 * r + s]; ++u) slot[b++] = d->psp[3 * r + s];
+    }
+    for (int u = 0; u < 4; ++u) cx[rr] |= (uint64_t)(slot[u] * CELL_ROW) << (16 * u);
+    for (int u = 0; u < 4; u += 2)
+      if (slot[u] == slot[u + 1] && slot[u] != ns) {
+        slot[u + 1] = ns;
+        ix[rr] |= 1ull << (44 + u / 2);
+      }
+    for (int u = 0; u < 4; ++u) cy[rr] |= (uint64_t)(slot[u] * CELL_ROW) << (16 * u);
+  }
+  // ---- net coefficients by reaction, from the species lists
+  std::vector<std::vector<int>> words(nr);
+  std::vector<double> rv;
+  {
+    const int* cs = reinterpret_cast<const int*>(img.data() + L.o_cstart);
+    const int* lr = reinterpret_cast<const int*>(img.data() + L.o_lr);
+    const double* nu = reinterpret_cast<const double*>(img.data() + L.o_lnu);
+    for (int k = 0; k < ns; ++k)
+      for (int e = cs[k]; e < cs[k + 1]; ++e) {
+        int code = nu[e] == 1.0 ? 1 : (nu[e] == -1.0 ? -1 : 0);
+        if (!code) {
+          size_t i = 0;
+          while (i < rv.size() && rv[i] != nu[e]) ++i;
+          if (i == rv.size()) rv.push_back(nu[e]);
+          code = 2 + (int)i;
+        }
+        words[lr[e]].push_back(k | (int)((unsigned)code << 8));
+      }
+  }
   // ---- sections
   int off = 0;
   auto sec = [&](int bytes) { int o = off; off = rup(off + bytes, 16); return o; };
@@ -255,7 +358,10 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   L.f_a = sec(8 * P); L.f_b = sec(8 * P); L.f_e = sec(8 * P); L.f_ix = sec(8 * P);
   L.f_ra = sec(8 * 16); L.f_rb = sec(8 * 16); L.f_re = sec(8 * 16); L.f_tr = sec(8 * 5 * 16);
   L.f_tbd = sec(8 * L.ntb); L.f_tbp = sec(4 * (L.ntb + 1)); L.f_tbs = sec(4 * ntbl); L.f_tbv = sec(8 * ntbl);
+  L.f_cx = sec(8 * P); L.f_cy = sec(8 * P);
+  L.f_rs = sec(4 * (nr + 1)); L.f_rw = sec(4 * nlist); L.f_rv = sec(8 * (int)std::max<size_t>(rv.size(), 1));
   L.f_exp = sec(8 * FIX_EXP2); L.f_log = sec(8 * 2 * FIX_LOG2);
+  L.fix_bytes_cell = off;   // the thread-per-cell kernel needs no species lists
   L.f_cstart = sec(4 * (S + 1)); L.f_lr = sec(4 * nlist); L.f_lnu = sec(8 * nlist);
   L.o_fix = L.bytes;
   L.fix_bytes = off;
@@ -273,14 +379,16 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   put(L.f_tbs, img.data() + L.o_tbs, 4 * ntbl); put(L.f_tbv, img.data() + L.o_tbv, 8 * (size_t)((L.o_cstart - L.o_tbv) / 8));
   put(L.f_cstart, img.data() + L.o_cstart, 4 * (S + 1)); put(L.f_lr, img.data() + L.o_lr, 4 * nlist);
   put(L.f_lnu, img.data() + L.o_lnu, 8 * nlist);
-  int64_t* et = reinterpret_cast<int64_t*>(F + L.f_exp);
-  for (int j = 0; j < FIX_EXP2; ++j) et[j] = (int64_t)llrintl(ldexpl(exp2l((j + 0.5L) / FIX_EXP2), 62));
-  int64_t* lt = reinterpret_cast<int64_t*>(F + L.f_log);
-  for (int j = 0; j < FIX_LOG2; ++j) {
-    const uint64_t c = (uint64_t)ldexpl(1.0L / (1.0L + (j + 0.5L) / FIX_LOG2), 64);
-    lt[2 * j] = (int64_t)c;
-    lt[2 * j + 1] = (int64_t)llrintl(ldexpl(-log2l(ldexpl((ld)c, -64)), 62));
+  put(L.f_cx, cx.data(), 8 * P); put(L.f_cy, cy.data(), 8 * P);
+  int* rs = reinterpret_cast<int*>(F + L.f_rs);
+  int* rw = reinterpret_cast<int*>(F + L.f_rw);
+  for (int rr = 0; rr < nr; ++rr) {
+    rs[rr + 1] = rs[rr] + (int)words[rr].size();
+    std::copy(words[rr].begin(), words[rr].end(), rw + rs[rr]);
   }
+  put(L.f_rv, rv.data(), 8 * rv.size());
+  put(L.f_exp, math_tables().exp2_fix, sizeof math_tables().exp2_fix);
+  put(L.f_log, math_tables().log2_fix, sizeof math_tables().log2_fix);
 }
 
 // Pack a mechanism description into the device image (see ImageLayout).
@@ -293,10 +401,13 @@ static int pack(const flint_mech_desc* d, ImageLayout& L, std::vector<uint8_t>& 
     return fail(FLINT_ERR_ARG, "NULL array in mechanism description");
   for (int k = 0; k < ns; ++k)
     if (!(d->mw[k] > 0.0)) return fail(FLINT_ERR_MECH, "species %d: molar mass %g", k, d->mw[k]);
-  // order reactions by type: elementary, three-body, Lindemann, Troe
-  std::vector<int> order(nr);
-  for (int r = 0; r < nr; ++r) order[r] = r;
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return d->rtype[a] < d->rtype[b]; });
+  // order reactions by type: elementary (by class), three-body, Lindemann, Troe
+  std::vector<int> order(nr), key(nr);
+  for (int r = 0; r < nr; ++r) {
+    order[r] = r;
+    key[r] = 3 * d->rtype[r] + plain_class(d, r);
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return key[a] < key[b]; });
   int ntb = 0;
   for (int r = 0; r < nr; ++r) {
     int t = d->rtype[r];
@@ -452,18 +563,8 @@ static int pack(const flint_mech_desc* d, ImageLayout& L, std::vector<uint8_t>& 
       for (auto& pr : lists[k]) { I(L.o_lr)[e] = pr.first; D(L.o_lnu)[e] = pr.second; ++e; }
   }
   I(L.o_cstart)[S] = e;
-  // 2^(j/256), rounded from extended precision, for the table-driven exp
-  for (int j = 0; j < 256; ++j) D(L.o_exptab)[j] = (double)exp2l((long double)j / 256.0L);
-  // flog's table: c_j = 1/(1 + j/128) rounded to double, -ln c_j as hi + lo
-  // (long double: at least 64 significant bits on either host)
-  for (int j = 0; j <= 128; ++j) {
-    const double c = (double)(1.0L / (1.0L + (long double)j / 128.0L));
-    const long double l = -logl((long double)c);
-    const double hi = (double)l;
-    D(L.o_logtab)[3 * j] = c;
-    D(L.o_logtab)[3 * j + 1] = hi;
-    D(L.o_logtab)[3 * j + 2] = (double)(l - (long double)hi);
-  }
+  memcpy(img.data() + L.o_exptab, math_tables().exp2, sizeof math_tables().exp2);
+  memcpy(img.data() + L.o_logtab, math_tables().log, sizeof math_tables().log);
   pack_fix(d, order, L, img);
   return FLINT_OK;
 }

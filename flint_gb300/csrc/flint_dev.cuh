@@ -73,15 +73,21 @@ struct ImageLayout {
   // at o_fix, 16-byte aligned, fix_bytes long; the f_ offsets are relative to
   // o_fix.  `bytes` above counts the FP64 sections only.
   int fix, o_fix, fix_bytes;
+  int fix_bytes_cell;            // the leading part that the thread-per-cell kernel stages
   int fix_w3;                    // some reaction has a third factor on a side
   double fix_Tlo, fix_Thi;       // cells with T in [fix_Tlo, fix_Thi) take the fixed-point path
-  int64_t fix_lC;                // log2(p_ref / r_thermo) - 10, Q52
+  int64_t fix_lC;                // log2(p_ref / r_thermo) - 7, Q52
   int f_mw, f_invmw, f_tmid;     // [nsp]
   int f_g, f_h, f_c;             // int64 [2][7][nsp], [2][6][nsp], [2][5][nsp]: g/RT (octaves), h/RT, cp/R; low, high range
-  int f_a, f_b, f_e, f_ix;       // int64 [nrpad]: log2|A| + 10 b, b, -E log2e; packed indices (fix_ix_*)
+  int f_a, f_b, f_e, f_ix;       // int64 [nrpad]: log2|A| + 7 b, b, -E log2e; packed indices (fix_ix_*)
   int f_ra, f_rb, f_re;          // int64 [16]: k0/kinf of the falloff reactions
   int f_tr;                      // double [5][16]: 1 - a, a, log2e/T3, log2e/T1, T2 log2e (0: none)
   int f_tbd, f_tbp, f_tbs, f_tbv;   // as the o_ ones
+  int f_cx, f_cy;                // uint64 [nrpad]: four 16-bit row offsets (r0, r1, p0, p1) of the factors and of the
+                                 // (distinct) species produced by the plain reactions, which
+  int fix_plain_rev, fix_plain_irr;   // come first: reversible, then irreversible (plain_class)
+  int f_rs, f_rw, f_rv;          // net coefficients by reaction: int32 [nr+1], int32 words species | code << 8
+                                 // (code +1, -1, or 2 + an index of f_rv), double values
   int f_exp, f_log;              // int64 [256], [128][2]
   int f_cstart, f_lr, f_lnu;     // as the o_ ones
 };
@@ -303,6 +309,9 @@ struct WarpScratch {
 // c, hRT and gRT have two more entries than species slots: the fixed-point path
 // reads index `dummy` (c = 1, g = 0) for a missing reactant or product.
 __host__ __device__ inline int species_stride(int nsp) { return nsp + 2; }
+// Thread-per-cell kernel (flint_cell.cu): a species' row of a warp holds c, g and
+// the production of the warp's 32 cells, each padded to 33 doubles.
+constexpr int CELL_PAD = 33, CELL_ROW = 3 * CELL_PAD;
 // (63 rather than 64 for the larger size: the packed index has 6 bits, and 63 species leave slot 63 free)
 __host__ __device__ inline int fix_dummy(int nsp) { return nsp == 64 ? 63 : nsp; }
 __host__ __device__ inline int scratch_small_doubles(int nsp, int nrpad) {

@@ -11,14 +11,18 @@
 // chain it replaces rounds at every step to 2^-53 of a magnitude of 10-60.
 // The result is therefore closer to the exact value, not further from it.
 //
-// All logarithms are base 2.  Formats (Qn: n fraction bits in a signed 64-bit
-// integer):
-//   exponents (log2 k, g/RT in octaves)   Q52   |x| < 2^11
-//   log2 T - 10                           Q61   T in [129, 8192)
-//   1/T (T > 128)                         Q70
-//   T/2^13 (high range), T/2^11 (low)     Q63
-//   E log2e, a5 (kelvin)                  Q45   |x| < 2^18
-//   temperature exponents b               Q55   |x| < 2^8
+// All logarithms are base 2.  Formats (Qn: n fraction bits in 64 bits):
+//   exponents (log2 k, g/RT in octaves)   Q52 signed   |x| < 2^11
+//   log2 T - 7                            Q61 unsigned, T in [129, 8192)
+//   1/T                                   Q70 unsigned (T > 128)
+//   T/2^13 (high range), T/2^11 (low)     Q63 unsigned
+//   E log2e (kelvin)                      Q45 signed   |x| < 2^18
+//   a5, a5 log2e (kelvin)                 Q46 signed   |x| < 2^17
+//   temperature exponents b, a0           Q55 signed   |x| < 2^8
+// A product is one unsigned 64 x 64 -> high-64 multiplication: a signed factor
+// is stored with its sign bit flipped (x + 2^63), which adds exactly half of the
+// other, non-negative, factor to the product; that half is a property of the
+// cell and is taken off once (a signed product costs twice the instructions).
 // A mechanism uses this path when every coefficient and every exponent over
 // the temperature range fits its format (ImageLayout::fix, decided when the
 // mechanism is packed); a cell outside [fix_Tlo, fix_Thi) takes the FP64 path.
@@ -29,89 +33,93 @@
 namespace flint {
 
 #ifdef __CUDA_ARCH__
-__device__ __forceinline__ int64_t mulhi_s(int64_t a, int64_t b) { return __mul64hi(a, b); }
 __device__ __forceinline__ uint64_t mulhi_u(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
-__device__ __forceinline__ int mulhi_i(int a, int b) { return __mulhi(a, b); }
+__device__ __forceinline__ uint32_t mulhi_32(uint32_t a, uint32_t b) { return __umulhi(a, b); }
 __device__ __forceinline__ int clz64(uint64_t x) { return __clzll((long long)x); }
 __device__ __forceinline__ int64_t d_bits(double x) { return __double_as_longlong(x); }
 __device__ __forceinline__ double bits_d(int64_t x) { return __longlong_as_double(x); }
 #else
-inline int64_t mulhi_s(int64_t a, int64_t b) { return (int64_t)(((__int128)a * b) >> 64); }
 inline uint64_t mulhi_u(uint64_t a, uint64_t b) { return (uint64_t)(((unsigned __int128)a * b) >> 64); }
-inline int mulhi_i(int a, int b) { return (int)(((int64_t)a * b) >> 32); }
+inline uint32_t mulhi_32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
 inline int clz64(uint64_t x) { return x ? __builtin_clzll(x) : 64; }
 inline int64_t d_bits(double x) { int64_t b; __builtin_memcpy(&b, &x, 8); return b; }
 inline double bits_d(int64_t x) { double d; __builtin_memcpy(&d, &x, 8); return d; }
 #endif
 
+// High half of a product without its low x low part: at most 3 too small.
+__host__ __device__ __forceinline__ uint64_t mulhi_a(uint64_t a, uint64_t b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return (uint64_t)ah * bh + (((uint64_t)ah * bl) >> 32) + (((uint64_t)al * bh) >> 32);
+}
+
 constexpr int64_t ONE52 = 1ll << 52;
 constexpr int FIX_EXP2 = 256;    // entries of the exp2 table
 constexpr int FIX_LOG2 = 128;    // rows of the log2 table
 
-// 2^x for x in Q52, by a 256-entry table of 2^((j + 1/2)/256) (Q62) and the
-// Taylor polynomial of 2^(w/256) - 1, w in [-1/2, 1/2), to degree 5 (the first
-// omitted term is below 2^-65): table-driven as P. T. P. Tang, ACM TOMS 15(2),
-// 1989.  The two low-order coefficients are applied with 64-bit products, the
-// others with 32-bit ones whose weight makes them exact enough (below 2^-59).
-// Error below 0.51 ulp of the returned double (tests/test_fix_cpu.py).  Below
-// the normal range returns 0, above it inf.  No FP64 instruction: 3 64-bit and
-// 3 32-bit products, about 22 cycles per SM and warp where the FP64 form took
-// 9 instructions = 150 cycles.
-__host__ __device__ __forceinline__ double exp2_q52(int64_t X, const int64_t* __restrict__ tab) {
-  constexpr int64_t K1 = 799144290325165979ll;     // ln2/256                   Q68
-  constexpr int64_t K2 = 1081884007225522ll;       // (ln2/256)^2 / 2           Q68
-  constexpr int K3 = 1907106652;                   // (ln2/256)^3 / 6           Q59
-  constexpr int K4 = 1290923;                      // (ln2/256)^4 / 24          Q59
-  constexpr int K5 = 699;                          // (ln2/256)^5 / 120         Q59
-  const int n = (int)(X >> 52);
-  const uint64_t F = (uint64_t)X << 12;
-  const int j = (int)(F >> 56);
-  const int64_t w = (int64_t)((F << 8) ^ 0x8000000000000000ull);   // Q64, [-1/2, 1/2)
-  const int w32 = (int)(w >> 32);
-  int t = K4 + mulhi_i(w32, K5);
-  t = K3 + mulhi_i(w32, t);
-  const int64_t u2 = K2 + (((int64_t)w32 * t) >> 23);
-  const int64_t u1 = K1 + mulhi_s(w, u2);
-  const int64_t p = mulhi_s(w, u1);                                 // 2^(w/256) - 1, Q68
-  const int64_t b = tab[j];
-  const int64_t R = b + (mulhi_s(b, p) >> 4);                       // Q62, in [1, 2)
-  const int64_t bits = ((int64_t)(n + 1022) << 52) + ((R + 512) >> 10);
-  const double r = bits_d(bits);
-  return n < -1022 ? 0.0 : (n > 1023 ? bits_d(0x7ff0000000000000ll) : r);
+// 2^x for x in Q52, by a 256-entry table of 2^(j/256) (Q62, with the rounding
+// half of the last double place added) and the Taylor polynomial of 2^(w/256) -
+// 1, w in [0, 1), to degree 5 (the first omitted term is below 2^-60):
+// table-driven as P. T. P. Tang, ACM TOMS 15(2), 1989.  The low-order
+// coefficients are applied with 64-bit products, the others with 32-bit ones
+// whose weight makes them exact enough.  Error below 0.53 ulp of the returned
+// double (tests/test_fix_cpu.py).  Below the normal range returns 0, above it
+// inf.  No FP64 instruction, where the FP64 form took 9 (150 cycles per SM and
+// warp).
+__host__ __device__ __forceinline__ double exp2_q52(int64_t X, const uint64_t* __restrict__ tab) {
+  constexpr uint64_t K1 = 799144290325165979ull;   // ln2/256                   Q68
+  constexpr uint64_t K2 = 1081884007225522ull;     // (ln2/256)^2 / 2           Q68
+  constexpr uint32_t K3 = 3814213304u;             // (ln2/256)^3 / 6           Q60
+  constexpr uint32_t K4 = 2581847u;                // (ln2/256)^4 / 24          Q60
+  constexpr uint32_t K5 = 1398u;                   // (ln2/256)^5 / 120         Q60
+  const int hi = (int)(X >> 32);
+  const int j = (hi >> 12) & 255;
+  const uint64_t w = (uint64_t)X << 20;                             // Q64, [0, 1)
+  const uint32_t w32 = (uint32_t)(w >> 32);
+  uint32_t t = K4 + mulhi_32(w32, K5);
+  t = K3 + mulhi_32(w32, t);
+  const uint64_t u2 = (uint64_t)mulhi_32(w32, t) * 256u + K2;
+  const uint64_t u1 = K1 + mulhi_a(w, u2);
+  const uint64_t p = mulhi_a(w, u1);                                // 2^(w/256) - 1, Q68
+  const uint64_t b = tab[j];
+  const uint64_t R = b + (mulhi_a(b, p) >> 4);                      // Q62, in [1, 2)
+  const int n1 = (hi >> 20) + 1022;                                 // biased exponent - 1
+  const double r = bits_d(((int64_t)n1 << 52) + (int64_t)(R >> 10));
+  return (unsigned)n1 <= 2045u ? r : (n1 < 0 ? 0.0 : bits_d(0x7ff0000000000000ll));
 }
 
-// log2 of the significand of a normal positive double, Q62 in [0, 1) up to its
-// rounding; e receives the exponent.  128 rows (c, -log2 c), c = 1/(row centre)
-// in Q64: r = y c - 1 (|r| < 2^-8) and log2(1 + r) by its Taylor polynomial to
-// r^7 (first omitted term below 2^-66), after P. T. P. Tang, ACM TOMS 16(4),
-// 1990.  Error below 2^-58.
-__host__ __device__ __forceinline__ int64_t log2_q62(double x, const int64_t* __restrict__ tab, int* e) {
-  constexpr int64_t A0 = 3326628274461080623ll;    // log2e                     Q61
-  constexpr int64_t A1 = -12994641697113596ll;     // -log2e/2 / 2^7            Q61
-  constexpr int64_t A2 = 67680425505800ll;         // log2e/3 / 2^14            Q61
-  constexpr int A3 = -774541002;                   // -log2e/4 / 2^21           Q52
-  constexpr int A4 = 4840881;                      // log2e/5 / 2^28            Q52
-  constexpr int A5 = -31516;                       // -log2e/6 / 2^35           Q52
-  constexpr int A6 = 211;                          // log2e/7 / 2^42            Q52
+// log2 of the significand of a normal positive double, Q62 in [0, 1); e receives
+// the exponent.  128 rows (c, -log2 c), c just above 1/(1 + j/128) in Q63: r =
+// y c - 1 in [0, 2^-7) and log2(1 + r) by its Taylor polynomial to r^8 (first
+// omitted term below 2^-65), after P. T. P. Tang, ACM TOMS 16(4), 1990.  Error
+// below 2^-59.
+__host__ __device__ __forceinline__ int64_t log2_q62(double x, const uint64_t* __restrict__ tab, int* e) {
+  constexpr uint64_t A0 = 6653256548922161246ull;  // log2e                     Q62
+  constexpr uint64_t A1 = 25989283394227192ull;    // log2e/2 / 2^7             Q62
+  constexpr uint64_t A2 = 135360851011600ull;      // log2e/3 / 2^14            Q62
+  constexpr uint32_t A3 = 3098164009u;             // log2e/4 / 2^21            Q54
+  constexpr uint32_t A4 = 19363525u;               // log2e/5 / 2^28            Q54
+  constexpr uint32_t A5 = 126065u;                 // log2e/6 / 2^35            Q54
+  constexpr uint32_t A6 = 844u;                    // log2e/7 / 2^42            Q54
+  constexpr uint32_t A7 = 6u;                      // log2e/8 / 2^49            Q54
   const int64_t b = d_bits(x);
   *e = (int)(b >> 52) - 1023;
   const uint64_t mant = (uint64_t)b & 0xfffffffffffffull;
   const int j = (int)(mant >> 45);
   const uint64_t Y = (mant << 11) | 0x8000000000000000ull;          // Q63
-  const uint64_t C = (uint64_t)tab[2 * j];
-  const int64_t rs = (int64_t)(mulhi_u(Y, C) - 0x8000000000000000ull) << 7;   // r 2^7, Q63
-  const int s = (int)(rs >> 32);
-  int t = A5 + (mulhi_i(s, A6) << 1);
-  t = A4 + (mulhi_i(s, t) << 1);
-  t = A3 + (mulhi_i(s, t) << 1);
-  int64_t u = A2 + (((int64_t)s * t) >> 22);
-  u = A1 + (mulhi_s(rs, u) << 1);
-  u = A0 + (mulhi_s(rs, u) << 1);
-  return tab[2 * j + 1] + (mulhi_s(rs, u) >> 5);
+  const uint64_t s = (mulhi_u(Y, tab[2 * j]) - 0x4000000000000000ull) << 9;   // r 2^7, Q64
+  const uint32_t s32 = (uint32_t)(s >> 32);
+  uint32_t t = A6 - mulhi_32(s32, A7);
+  t = A5 - mulhi_32(s32, t);
+  t = A4 - mulhi_32(s32, t);
+  t = A3 - mulhi_32(s32, t);
+  uint64_t u = A2 - (uint64_t)mulhi_32(s32, t) * 256u;
+  u = A1 - mulhi_a(s, u);
+  u = A0 - mulhi_a(s, u);
+  return (int64_t)(tab[2 * j + 1] + (mulhi_a(s, u) >> 7));
 }
 
 // log2 x in Q52 (x a normal positive double).
-__host__ __device__ __forceinline__ int64_t log2_q52(double x, const int64_t* __restrict__ tab) {
+__host__ __device__ __forceinline__ int64_t log2_q52(double x, const uint64_t* __restrict__ tab) {
   int e;
   const int64_t f = log2_q62(x, tab, &e);
   return ((int64_t)e << 52) + ((f + 512) >> 10);
@@ -139,21 +147,22 @@ __host__ __device__ __forceinline__ int64_t d2fix52(double x) {
 
 // The powers of T that the polynomials and Arrhenius exponents take.
 struct FixT {
-  int64_t L;     // log2 T - 10, Q61
-  int64_t v;     // 1/T, Q70
-  int64_t t13;   // T / 2^13, Q63
-  int64_t t11;   // T / 2^11, Q63 (meaningful for T < 2048)
+  uint64_t L;     // log2 T - 7, Q61
+  uint64_t v;     // 1/T, Q70
+  uint64_t t13;   // T / 2^13, Q63
+  uint64_t t11;   // T / 2^11, Q63 (meaningful for T < 2048)
+  int64_t ka;     // what the flipped signs of b and E add to an Arrhenius exponent
 };
 
-__host__ __device__ __forceinline__ FixT fix_T(double T, const int64_t* __restrict__ ltab) {
+__host__ __device__ __forceinline__ FixT fix_T(double T, const uint64_t* __restrict__ ltab) {
   FixT f;
   int e;
   const int64_t lg = log2_q62(T, ltab, &e);
-  f.L = ((int64_t)(e - 10) << 61) + ((lg + 1) >> 1);
+  f.L = ((uint64_t)(e - 7) << 61) + ((uint64_t)(lg + 1) >> 1);
   const int64_t b = d_bits(T);
   const uint64_t Y = (((uint64_t)b & 0xfffffffffffffull) << 11) | 0x8000000000000000ull;
-  f.t13 = (int64_t)(Y >> (13 - e));
-  f.t11 = (int64_t)(e < 11 ? Y >> (11 - e) : Y >> 1);
+  f.t13 = Y >> (13 - e);
+  f.t11 = e < 11 ? Y >> (11 - e) : Y >> 1;
   // 1/y of the significand y: a single-precision seed r (24 bits) and one
   // third-order (Chebyshev) step r (1 + d + d^2), d = 1 - y r, |d| < 2^-21; d is
   // exact (y and r have 53 and 24 bits, and only the low 64 bits of y r matter)
@@ -172,10 +181,45 @@ __host__ __device__ __forceinline__ FixT fix_T(double T, const int64_t* __restri
   const uint32_t r24 = ((rb & 0x7fffffu) | 0x800000u) << ((int)(rb >> 23) - 126);
   const int64_t d = -(int64_t)((Y >> 3) * r24);                              // Q84
   const int d32 = (int)(d >> 32);                                            // Q52
-  const int64_t c = (d >> 3) + (((int64_t)d32 * d32) >> 23);                 // Q81
-  const int64_t r0 = (int64_t)r24 << 38;                                     // Q62
-  f.v = (e <= 8 ? r0 << (8 - e) : r0 >> (e - 8)) + (mulhi_s(r0, c) >> (e + 9));   // Q79 -> Q70
+  const uint64_t c = (uint64_t)((d >> 3) + (((int64_t)d32 * d32) >> 23)) ^ 0x8000000000000000ull;   // Q81, sign flipped
+  const uint64_t r0 = (uint64_t)r24 << 38;                                   // Q62
+  const int64_t m = (int64_t)(mulhi_u(r0, c) - (r0 >> 1));                   // Q79
+  f.v = (e <= 8 ? r0 << (8 - e) : r0 >> (e - 8)) + (uint64_t)(m >> (e + 9));
+  f.ka = -(int64_t)(f.L >> 1) - (int64_t)f.v;
   return f;
+}
+
+// log2 A + b log2 T - E log2e/T: a = log2 A + 7 b (Q52); b (Q55) and -E log2e
+// (Q45) with their signs flipped.
+__host__ __device__ __forceinline__ int64_t fix_arrhenius(int64_t a, uint64_t b, uint64_t e, const FixT& f) {
+  return a + f.ka + (int64_t)mulhi_u(b, f.L) + (int64_t)(mulhi_u(e, f.v) << 1);
+}
+
+// c1 + t (c2 + t (...)), sign flipped (+ 2^63): coefficients (stride S, signs
+// flipped) in Qn, Q(n - 1), ... by order, t in Q63.
+template <int N>
+__host__ __device__ __forceinline__ uint64_t fix_horner(const uint64_t* __restrict__ c, int S, uint64_t t) {
+  uint64_t a = c[(N - 1) * S];
+#pragma unroll
+  for (int j = N - 2; j >= 0; --j) a = c[j * S] + (mulhi_u(a, t) << 2) - (t << 1);
+  return a;
+}
+
+// Polynomial of order 4, result in Q52: c[0] plain (Q52), c[1..4] as in
+// fix_horner with n = 51.
+__host__ __device__ __forceinline__ int64_t fix_poly5(const uint64_t* __restrict__ c, int S, uint64_t t) {
+  return (int64_t)(c[0] + (mulhi_u(fix_horner<4>(c + S, S, t), t) << 2) - (t << 1));
+}
+
+// g/RT in octaves (Q52): c = constant, a0 (Q55), c1..c4 (Q53...), a5 log2e (Q46).
+__host__ __device__ __forceinline__ int64_t fix_gibbs(const uint64_t* __restrict__ c, int S, uint64_t t, const FixT& f) {
+  return (int64_t)(c[0] + ((f.L >> 1) + (t >> 1) - (f.v >> 1)) + mulhi_u(c[6 * S], f.v) - mulhi_u(c[S], f.L) -
+                   mulhi_u(fix_horner<4>(c + 2 * S, S, t), t));
+}
+
+// h/RT (Q52): the polynomial and a5/T.
+__host__ __device__ __forceinline__ int64_t fix_enthalpy(const uint64_t* __restrict__ c, int S, uint64_t t, const FixT& f) {
+  return fix_poly5(c, S, t) + (int64_t)(mulhi_u(c[5 * S], f.v) - (f.v >> 1));
 }
 
 // 1/x in FP64: the SM's reciprocal approximation (about 2^-20) and one

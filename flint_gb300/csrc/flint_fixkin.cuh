@@ -13,9 +13,12 @@ namespace flint {
 
 // Index word of a reaction: bits 0-17 three reactant factors, 18-35 three
 // product factors (6 bits each, `dummy` where absent), 36-39 dn + 8, 40-41
-// type, 42 reversible, 43 A < 0, 48-55 third-body row.
+// type, 42 reversible, 43 A < 0, 44 and 45 both reactant and both product factors
+// of a plain reaction are one species, 48-55 third-body row.
 __device__ __forceinline__ int fix_type(uint64_t w) { return (int)(w >> 40) & 3; }
 __device__ __forceinline__ bool fix_rev(uint64_t w) { return (w >> 42) & 1; }
+__device__ __forceinline__ bool fix_twice_r(uint64_t w) { return (w >> 44) & 1; }
+__device__ __forceinline__ bool fix_twice_p(uint64_t w) { return (w >> 45) & 1; }
 __device__ __forceinline__ int fix_tbrow(uint64_t w) { return (int)(w >> 48) & 0xff; }
 __device__ __forceinline__ int fix_idx(uint64_t w, int slot) { return (int)(w >> (6 * slot)) & 63; }
 __device__ __forceinline__ int fix_dn(uint64_t w) { return ((int)(w >> 36) & 15) - 8; }
@@ -25,19 +28,22 @@ struct FixView {
   double inv_r_eos, r_eos, r_thermo, Tlo, Thi;
   int64_t lC;
   const double *mw, *invmw, *tr, *tbd, *tbv, *lnu;
-  const int64_t *tmid, *g, *h, *c, *a, *b, *e, *ra, *rb, *re, *et, *lt;
-  const uint64_t* ix;
-  const int *tbp, *tbs, *cstart, *lr;
+  const int64_t *tmid, *a, *ra;
+  const uint64_t *g, *h, *c, *b, *e, *rb, *re, *et, *lt, *ix, *cx, *cy;
+  const int *tbp, *tbs, *cstart, *lr, *rs, *rw;
+  const double* rv;
   __device__ __forceinline__ void bind(const ImageLayout& L, const uint8_t* base) {
     ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; nfall = L.nfall; dummy = fix_dummy(L.nsp); w3 = L.fix_w3;
     inv_r_eos = L.inv_r_eos; r_eos = L.r_eos; r_thermo = L.r_thermo; Tlo = L.fix_Tlo; Thi = L.fix_Thi; lC = L.fix_lC;
     auto D = [&](int o) { return (const double*)(base + o); };
     auto I = [&](int o) { return (const int64_t*)(base + o); };
+    auto U = [&](int o) { return (const uint64_t*)(base + o); };
     mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv); lnu = D(L.f_lnu);
-    tmid = I(L.f_tmid); g = I(L.f_g); h = I(L.f_h); c = I(L.f_c); a = I(L.f_a); b = I(L.f_b); e = I(L.f_e);
-    ra = I(L.f_ra); rb = I(L.f_rb); re = I(L.f_re); et = I(L.f_exp); lt = I(L.f_log);
-    ix = (const uint64_t*)(base + L.f_ix);
+    tmid = I(L.f_tmid); a = I(L.f_a); ra = I(L.f_ra);
+    g = U(L.f_g); h = U(L.f_h); c = U(L.f_c); b = U(L.f_b); e = U(L.f_e);
+    rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); cx = U(L.f_cx); cy = U(L.f_cy);
     tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
+    rs = (const int*)(base + L.f_rs); rw = (const int*)(base + L.f_rw); rv = D(L.f_rv);
     cstart = (const int*)(base + L.f_cstart); lr = (const int*)(base + L.f_lr);
   }
   __device__ __forceinline__ bool covers(double T) const { return T >= Tlo && T < Thi; }
@@ -65,16 +71,6 @@ __device__ __forceinline__ double warp_isum(double v) {
   return fix2d(S, 1080 - (int)emax);
 }
 
-// Polynomial c0 + t (c1 + t (...)) in t (Q63); coefficients (stride S) in Q52,
-// Q51, Q50, ... by order (see pack_fix), the result in Q52.
-template <int N>
-__device__ __forceinline__ int64_t fix_poly(const int64_t* __restrict__ c, int S, int64_t t) {
-  int64_t a = c[(N - 1) * S];
-#pragma unroll
-  for (int j = N - 2; j >= 0; --j) a = c[j * S] + (mulhi_s(a, t) << 2);
-  return a;
-}
-
 __device__ __forceinline__ double fix_tb_conc(const FixView& m, int t, double ctot, const double* c) {
   double M = m.tbd[t] * ctot;
   for (int e = m.tbp[t]; e < m.tbp[t + 1]; ++e) M = fma(m.tbv[e], c[m.tbs[e]], M);
@@ -89,6 +85,21 @@ constexpr int64_t TROE_C75 = 11220475597714730ll;       // 0.75 log2(10)  Q52
 constexpr int64_t TROE_M67 = 6179659264692699791ll;     // 0.67  Q63
 constexpr int64_t TROE_M127 = 5856841243402782638ll;    // 1.27  Q62
 constexpr int64_t TROE_M14 = 1291272085159668613ll;     // 0.14  Q63
+
+// x, or 1e-300 where x is smaller (compared as bit patterns: no FP64 slot).
+__device__ __forceinline__ double floor_tiny(double x) {
+  return __double_as_longlong(x) > 0x01a56e1fc2f8f359ll ? x : 1e-300;
+}
+
+__device__ __forceinline__ int64_t mulhi_s(int64_t a, int64_t b) { return __mul64hi(a, b); }
+
+__device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_t* lt, const uint64_t* et) {
+  const int64_t lg = log2_q52(floor_tiny(Fc), lt);
+  const int64_t xx = log2_q52(floor_tiny(Pr), lt) - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
+  const int64_t den = TROE_C75 - (mulhi_s(lg, TROE_M127) << 2) - (mulhi_s(xx, TROE_M14) << 1);
+  const double dx = fix2d(xx, 52), dd = fix2d(den, 52), d2 = dd * dd;
+  return exp2_q52(d2fix52(fix2d(lg, 52) * (d2 * recip(fma(dx, dx, d2)))), et);
+}
 
 // One cell (see warp_kinetics for the meaning of pr, cv and s.Jr).  RHS: form
 // out.f and out.fT; want_h: form out.cp_mass and out.h_mass.  img: the global
@@ -123,14 +134,11 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       ck = rho * yw[j];
       my_c[j] = ck;
       const bool lo = __double_as_longlong(T) <= m.tmid[k];
-      const int64_t t = lo ? f.t11 : f.t13;
-      const int64_t* c = m.g + (lo ? 0 : 7 * nsp) + k;
-      gk = c[0] - (mulhi_s(c[nsp], f.L) << 1) - (mulhi_s(fix_poly<4>(c + 2 * nsp, nsp, t), t) << 1) +
-           (mulhi_s(c[6 * nsp], f.v) << 1);
+      const uint64_t t = lo ? f.t11 : f.t13;
+      gk = fix_gibbs(m.g + (lo ? 0 : 7 * nsp) + k, nsp, t, f);
       if (thermo) {
-        const int64_t* h = m.h + (lo ? 0 : 6 * nsp) + k;
-        my_hRT[j] = fix2d(fix_poly<5>(h, nsp, t) + (mulhi_s(h[5 * nsp], f.v) << 1), 52);
-        my_cpR[j] = fix2d(fix_poly<5>(m.c + (lo ? 0 : 5 * nsp) + k, nsp, t), 52);
+        my_hRT[j] = fix2d(fix_enthalpy(m.h + (lo ? 0 : 6 * nsp) + k, nsp, t, f), 52);
+        my_cpR[j] = fix2d(fix_poly5(m.c + (lo ? 0 : 5 * nsp) + k, nsp, t), 52);
       }
     }
     if (k < nsp) {
@@ -155,14 +163,13 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   const int NF = m.nfall, f0 = m.nr - NF;
   double* fo = JAC ? s.Jr : s.fo;
   if (NF > 0) {
-    const double Tinv = JAC ? invT : fix2d(f.v, 70);
+    const double Tinv = JAC ? invT : fix2d((int64_t)f.v, 70);
     for (int jb = lane; jb < 5 * NF; jb += WARP) {
       const int i = jb / 5, kind = jb - 5 * i, r = f0 + i;
       int64_t x;
       double keep = 1.0;
       if (kind < 2) {
-        const int64_t a = kind == 0 ? m.a[r] : m.ra[i], b = kind == 0 ? m.b[r] : m.rb[i], e = kind == 0 ? m.e[r] : m.re[i];
-        x = a + mulhi_s(b, f.L) + (mulhi_s(e, f.v) << 1);
+        x = fix_arrhenius(kind == 0 ? m.a[r] : m.ra[i], kind == 0 ? m.b[r] : m.rb[i], kind == 0 ? m.e[r] : m.re[i], f);
       } else {
         const double z = m.tr[16 * kind + i];      // log2e/T3, log2e/T1, T2 log2e
         x = -d2fix52(z * (kind == 4 ? Tinv : T));
@@ -184,7 +191,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
     }
     const double Pr_src = __shfl_sync(FULL, Pr, lane >= NF && lane < 2 * NF ? lane - NF : 0);
     double lg_in = lane < NF ? Fc : (lane < 2 * NF ? Pr_src : 1.0);
-    lg_in = lg_in > 1e-300 ? lg_in : 1e-300;
+    lg_in = floor_tiny(lg_in);
     // octaves; Pr = inf or NaN gives a finite garbage exponent, and the NaN of
     // Pr / (1 + Pr) below makes the rate NaN as before
     const int64_t lg = log2_q52(lg_in, m.lt);
@@ -239,10 +246,10 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       const bool rev = fix_rev(w);
       const int r0 = fix_idx(w, 0), r1 = fix_idx(w, 1), p0 = fix_idx(w, 3), p1 = fix_idx(w, 4);
       const double c0 = s.c[r0], c1 = s.c[r1], d0 = s.c[p0], d1 = s.c[p1];
-      int64_t a = m.a[r] + mulhi_s(m.b[r], f.L) + (mulhi_s(m.e[r], f.v) << 1);
+      int64_t a = fix_arrhenius(m.a[r], m.b[r], m.e[r], f);
       a = type >= 2 ? 0 : a;
       // 1/Kc = 2^(dG - dn log2(p_ref/RT)), kr = kf / Kc
-      int64_t ar = a + G[p0] + G[p1] - G[r0] - G[r1] - (int64_t)fix_dn(w) * (m.lC - (f.L >> 9));
+      int64_t ar = a + G[p0] + G[p1] - G[r0] - G[r1] - (int64_t)fix_dn(w) * (m.lC - (int64_t)(f.L >> 9));
       double c2 = 1.0, d2 = 1.0;
       if (m.w3) {
         const int r2 = fix_idx(w, 2), p2 = fix_idx(w, 5);

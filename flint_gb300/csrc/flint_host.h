@@ -59,6 +59,12 @@ inline cudaError_t set_smem(const void* fn, size_t bytes) {
 cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
                         const double* p, const double* Y, double* wdot, double* cp, double* h, cudaStream_t st,
                         int threads = 0);
+// Thread-per-cell source terms (flint_cell.cu): whether they serve a batch, and
+// the launch (rhs: out is the right-hand side, (n, ns + 1)).
+bool use_cell_kernel(const ImageLayout& L, int64_t n);
+cudaError_t launch_wdot_cell(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
+                             const double* p, const double* Y, double* out, double* cp, double* h, bool rhs, int cv,
+                             cudaStream_t st);
 int warp_block_candidates(int* out);
 bool use_small_kernel(const ImageLayout& L);   // wdot of <= 8 species: thread per cell
 cudaError_t launch_species_thermo(const uint8_t* img, const ImageLayout& L, int64_t n, const double* T, double* cp,

@@ -477,6 +477,7 @@ cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int
     count_launch();
     return cudaGetLastError();
   }
+  if (use_cell_kernel(L, n)) return launch_wdot_cell(img, L, n, layout, T, p, Y, wdot, cp, h, false, 0, st);
   return launch_warp<false, false>(img, L, n, layout, T, p, Y, wdot, cp, h, nullptr, nullptr, nullptr, st, 0, threads);
 }
 
@@ -525,6 +526,7 @@ cudaError_t launch_wdot_jac(const uint8_t* img, const ImageLayout& L, int64_t n,
 cudaError_t launch_rhs(const uint8_t* img, const ImageLayout& L, int64_t n, const double* T, const double* p,
                        const double* Y, double* f, cudaStream_t st, int cv) {
   if (n <= 0) return cudaSuccess;
+  if (use_cell_kernel(L, n)) return launch_wdot_cell(img, L, n, 0, T, p, Y, f, nullptr, nullptr, true, cv, st);
   return launch_warp<false, true>(img, L, n, 0, T, p, Y, nullptr, nullptr, nullptr, nullptr, f, nullptr, st, cv);
 }
 

@@ -9,12 +9,11 @@ using namespace flint;
 
 int main() {
   typedef long double ld;
-  std::vector<int64_t> et(FIX_EXP2), lt(2 * FIX_LOG2);
-  for (int j = 0; j < FIX_EXP2; ++j) et[j] = (int64_t)llrintl(ldexpl(exp2l((j + 0.5L) / FIX_EXP2), 62));
+  std::vector<uint64_t> et(FIX_EXP2), lt(2 * FIX_LOG2);
+  for (int j = 0; j < FIX_EXP2; ++j) et[j] = (uint64_t)llrintl(ldexpl(exp2l((ld)j / FIX_EXP2), 62)) + 512;
   for (int j = 0; j < FIX_LOG2; ++j) {
-    const uint64_t c = (uint64_t)ldexpl(1.0L / (1.0L + (j + 0.5L) / FIX_LOG2), 64);
-    lt[2 * j] = (int64_t)c;
-    lt[2 * j + 1] = (int64_t)llrintl(ldexpl(-log2l(ldexpl((ld)c, -64)), 62));
+    lt[2 * j] = (uint64_t)ldexpl(1.0L / (1.0L + (ld)j / FIX_LOG2), 63) + 1;
+    lt[2 * j + 1] = (uint64_t)llrintl(ldexpl(-log2l(ldexpl((ld)lt[2 * j], -63)), 62));
   }
   std::mt19937_64 g(7);
   std::uniform_real_distribution<double> U(0.0, 1.0);
@@ -38,7 +37,7 @@ int main() {
     if (i % 5 == 1) T = std::exp2(8 + i % 5);
     if (i % 5 == 2) T = std::nextafter(std::exp2(8 + i % 6), 0.0);
     const FixT t = fix_T(T, lt.data());
-    L = fmaxl(L, fabsl(ldexpl((ld)t.L, -61) - (log2l((ld)T) - 10)));
+    L = fmaxl(L, fabsl(ldexpl((ld)t.L, -61) - (log2l((ld)T) - 7)));
     v = fmaxl(v, fabsl(ldexpl((ld)t.v, -70) - 1.0L / (ld)T));
     exact &= (ld)t.t13 == ldexpl((ld)T, 50) && (T >= 2048 || (ld)t.t11 == ldexpl((ld)T, 52));
     // conversions

@@ -96,3 +96,55 @@ def test_unnormalised_mass_fractions(scale):
     w1 = chem.wdot(Tt, pt, Yt * scale)[0]
     _, ws_o, _, _ = Oracle(mech).wdot_batch(T, p, Y)
     assert (np.abs((w1 - w0).cpu().numpy()) / (ws_o.reshape(128, -1) + 1e-300)).max() < 1e-13
+
+
+@pytest.mark.parametrize("name", ["c2", "c5", "tsr_rich_31", "pelucchi", "coria"])
+@pytest.mark.parametrize("n", [15199, 15200, 15233])
+def test_thread_per_cell(name, n):
+    """Batches large enough for the thread-per-cell kernel, a ragged last warp and
+    cells outside the fixed-point range among them, in both storage orders and as
+    right-hand sides; constant volume against the warp kernel (a small batch)."""
+    mech = load(name)
+    rng = np.random.default_rng(n)
+    T = rng.uniform(300.0, 4500.0, n)
+    T[::37] = 8500.0
+    T[n - 1] = 9000.0
+    p = rng.uniform(1.0, 40.0, n) * 101325.0
+    Y = rng.dirichlet(np.full(mech.ns, 0.3), size=n)
+    chem, orc = Chemistry(mech), Oracle(mech)
+    w_o, ws_o, cp_o, h_o = orc.wdot_batch(T, p, Y)
+    w_o, ws_o = w_o.reshape(n, -1), ws_o.reshape(n, -1)
+    Tt, pt, Yt, Ys = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (T, p, Y, Y.T))
+    cp, h = torch.empty_like(Tt), torch.empty_like(Tt)
+    w = chem.wdot(Tt, pt, Yt, cp=cp, h=h)[0].cpu().numpy()
+    ws = chem.wdot(Tt, pt, Ys, layout=SPECIES_MAJOR)[0].cpu().numpy().T
+    f = chem.rhs(Tt, pt, Yt)
+    W = np.array([s.mw for s in mech.species])
+    rho = p / (mech.r_eos * T * (Y / W).sum(1))
+    rt = torch.from_numpy(rho).cuda()
+    fv = chem.rhs_constv(Tt, rt, Yt)
+    few = slice(n - 500, n)
+    args = [a[few].contiguous() for a in (Tt, pt, rt, Yt)]
+    f0, fv0 = chem.rhs(args[0], args[1], args[3]), chem.rhs_constv(args[0], args[2], args[3])
+    torch.cuda.synchronize()
+    assert (np.abs(w - w_o) / (ws_o + 1e-300)).max() < 1e-12
+    assert (np.abs(ws - w_o) / (ws_o + 1e-300)).max() < 1e-12
+    # cp and h on the scale of their absolute terms (a polynomial beyond its range
+    # may pass through zero)
+    tmid = np.array([s.tmid for s in mech.species])
+    a = np.where((T[:, None] <= tmid)[:, :, None], np.array([s.low for s in mech.species]),
+                 np.array([s.high for s in mech.species]))
+    powers = T[:, None, None] ** np.arange(5)
+    cps = mech.r_thermo * (Y / W * (np.abs(a[:, :, :5]) * powers).sum(2)).sum(1)
+    hs = T * cps + mech.r_thermo * (Y / W * np.abs(a[:, :, 5])).sum(1)
+    assert np.max(np.abs(cp.cpu().numpy() - cp_o) / cps) < 1e-13
+    assert np.max(np.abs(h.cpu().numpy() - h_o) / hs) < 1e-13
+    scale = ws_o / rho[:, None]
+    f, fv = f.cpu().numpy(), fv.cpu().numpy()
+    assert (np.abs(f[:, :-1] - w_o / rho[:, None]) / (scale + 1e-300)).max() < 1e-12
+    # dT/dt: a sum over the species of h_k w_k, on the scale of its absolute terms
+    # (|h_k/RT| < 400, cp/R > 2 per mole)
+    tscale = T * 400.0 * (ws_o / W).sum(1) / (2.0 * rho * (Y / W).sum(1))
+    for a, b in ((f, f0.cpu().numpy()), (fv, fv0.cpu().numpy())):
+        assert (np.abs(a[few, :-1] - b[:, :-1]) / (scale[few] + 1e-300)).max() < 1e-12
+        assert (np.abs(a[few, -1] - b[:, -1]) / tscale[few]).max() < 1e-12
