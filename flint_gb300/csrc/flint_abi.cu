@@ -349,6 +349,35 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
         words[lr[e]].push_back(k | (int)((unsigned)code << 8));
       }
   }
+  // ---- species sums: the lists of all species end to end, cut into 32 equal
+  // parts, one per lane; a piece is a lane's run of entries of one species
+  std::vector<uint32_t> seg;
+  std::vector<double> segv{0.0, 1.0};   // index 0: filling entries
+  std::vector<int> piece(S + 1, 0);
+  {
+    const int* cs = reinterpret_cast<const int*>(img.data() + L.o_cstart);
+    const int* lr = reinterpret_cast<const int*>(img.data() + L.o_lr);
+    const double* nu = reinterpret_cast<const double*>(img.data() + L.o_lnu);
+    const int total = cs[ns], len = std::max(1, (total + 31) / 32);
+    seg.assign((size_t)32 * len, 0);
+    int np = 0;
+    for (int k = 0; k < S; ++k) {
+      piece[k] = np;
+      for (int e = cs[k]; k < ns && e < cs[k + 1]; ++e) {
+        size_t i = 0;
+        while (i < segv.size() && segv[i] != std::fabs(nu[e])) ++i;
+        if (i == segv.size()) segv.push_back(std::fabs(nu[e]));
+        const bool last = e + 1 == cs[k + 1] || (e + 1) % len == 0;
+        if (segv.size() > 127 || lr[e] > 0xffff || np > 127) { L.fix = 0; return; }
+        seg[(size_t)(e % len) * 32 + e / len] = (uint32_t)lr[e] | (nu[e] < 0.0 ? 1u << 16 : 0u) | (uint32_t)i << 17 |
+                                                 (uint32_t)np << 24 | (last ? 1u << 31 : 0u);
+        np += last;
+      }
+    }
+    piece[S] = np;
+    L.seg_len = len;
+  }
+  L.fix_ntb = tb;
   // ---- sections
   int off = 0;
   auto sec = [&](int bytes) { int o = off; off = rup(off + bytes, 16); return o; };
@@ -362,6 +391,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   L.f_rs = sec(4 * (nr + 1)); L.f_rw = sec(4 * nlist); L.f_rv = sec(8 * (int)std::max<size_t>(rv.size(), 1));
   L.f_exp = sec(8 * FIX_EXP2); L.f_log = sec(8 * 2 * FIX_LOG2);
   L.fix_bytes_cell = off;   // the thread-per-cell kernel needs no species lists
+  L.f_seg = sec(4 * (int)seg.size()); L.f_segv = sec(8 * (int)segv.size()); L.f_piece = sec(4 * (S + 1));
+  L.fix_bytes_rate = off;   // kernels without a Jacobian need no species lists
   L.f_cstart = sec(4 * (S + 1)); L.f_lr = sec(4 * nlist); L.f_lnu = sec(8 * nlist);
   L.o_fix = L.bytes;
   L.fix_bytes = off;
@@ -379,6 +410,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   put(L.f_tbs, img.data() + L.o_tbs, 4 * ntbl); put(L.f_tbv, img.data() + L.o_tbv, 8 * (size_t)((L.o_cstart - L.o_tbv) / 8));
   put(L.f_cstart, img.data() + L.o_cstart, 4 * (S + 1)); put(L.f_lr, img.data() + L.o_lr, 4 * nlist);
   put(L.f_lnu, img.data() + L.o_lnu, 8 * nlist);
+  put(L.f_seg, seg.data(), 4 * seg.size()); put(L.f_segv, segv.data(), 8 * segv.size());
+  put(L.f_piece, piece.data(), 4 * (S + 1));
   put(L.f_cx, cx.data(), 8 * P); put(L.f_cy, cy.data(), 8 * P);
   int* rs = reinterpret_cast<int*>(F + L.f_rs);
   int* rw = reinterpret_cast<int*>(F + L.f_rw);

@@ -73,7 +73,8 @@ struct ImageLayout {
   // at o_fix, 16-byte aligned, fix_bytes long; the f_ offsets are relative to
   // o_fix.  `bytes` above counts the FP64 sections only.
   int fix, o_fix, fix_bytes;
-  int fix_bytes_cell;            // the leading part that the thread-per-cell kernel stages
+  int fix_bytes_cell, fix_bytes_rate;   // the leading parts that the thread-per-cell kernel and the warp kernels
+                                        // without a Jacobian stage
   int fix_w3;                    // some reaction has a third factor on a side
   double fix_Tlo, fix_Thi;       // cells with T in [fix_Tlo, fix_Thi) take the fixed-point path
   int64_t fix_lC;                // log2(p_ref / r_thermo) - 7, Q52
@@ -89,7 +90,12 @@ struct ImageLayout {
   int f_rs, f_rw, f_rv;          // net coefficients by reaction: int32 [nr+1], int32 words species | code << 8
                                  // (code +1, -1, or 2 + an index of f_rv), double values
   int f_exp, f_log;              // int64 [256], [128][2]
-  int f_cstart, f_lr, f_lnu;     // as the o_ ones
+  int f_cstart, f_lr, f_lnu;     // as the o_ ones (the Jacobian's species rows)
+  // species sums, the entries of all species dealt out evenly over the lanes:
+  // uint32 [seg_len][32] words (reaction | sign << 16 | value << 17 | piece << 24 |
+  // last-of-piece << 31), values, and int32 [nsp+1] first piece of each species
+  int f_seg, f_segv, f_piece, seg_len;
+  int fix_ntb;                   // third-body and falloff reactions (the last ones)
 };
 
 struct MechView {

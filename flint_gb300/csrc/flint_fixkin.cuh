@@ -24,16 +24,18 @@ __device__ __forceinline__ int fix_idx(uint64_t w, int slot) { return (int)(w >>
 __device__ __forceinline__ int fix_dn(uint64_t w) { return ((int)(w >> 36) & 15) - 8; }
 
 struct FixView {
-  int ns, nr, nrpad, nsp, nfall, dummy, w3;
+  int ns, nr, nrpad, nsp, nfall, dummy, w3, ntb, seg_len;
   double inv_r_eos, r_eos, r_thermo, Tlo, Thi;
   int64_t lC;
   const double *mw, *invmw, *tr, *tbd, *tbv, *lnu;
   const int64_t *tmid, *a, *ra;
   const uint64_t *g, *h, *c, *b, *e, *rb, *re, *et, *lt, *ix, *cx, *cy;
-  const int *tbp, *tbs, *cstart, *lr, *rs, *rw;
-  const double* rv;
+  const int *tbp, *tbs, *cstart, *lr, *rs, *rw, *piece;
+  const double *rv, *segv;
+  const uint32_t* seg;
   __device__ __forceinline__ void bind(const ImageLayout& L, const uint8_t* base) {
     ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; nfall = L.nfall; dummy = fix_dummy(L.nsp); w3 = L.fix_w3;
+    ntb = L.fix_ntb; seg_len = L.seg_len;
     inv_r_eos = L.inv_r_eos; r_eos = L.r_eos; r_thermo = L.r_thermo; Tlo = L.fix_Tlo; Thi = L.fix_Thi; lC = L.fix_lC;
     auto D = [&](int o) { return (const double*)(base + o); };
     auto I = [&](int o) { return (const int64_t*)(base + o); };
@@ -44,6 +46,7 @@ struct FixView {
     rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); cx = U(L.f_cx); cy = U(L.f_cy);
     tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
     rs = (const int*)(base + L.f_rs); rw = (const int*)(base + L.f_rw); rv = D(L.f_rv);
+    seg = (const uint32_t*)(base + L.f_seg); segv = D(L.f_segv); piece = (const int*)(base + L.f_piece);
     cstart = (const int*)(base + L.f_cstart); lr = (const int*)(base + L.f_lr);
   }
   __device__ __forceinline__ bool covers(double T) const { return T >= Tlo && T < Thi; }
@@ -101,13 +104,32 @@ __device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_
   return exp2_q52(d2fix52(fix2d(lg, 52) * (d2 * recip(fma(dx, dx, d2)))), et);
 }
 
+// What a cell's fixed pressure (cv: density) contributes: the reactor forms it
+// once per cell.
+struct FixPress {
+  double pr;      // p, or rho (cv)
+  double a;       // p / r_eos
+  double b;       // r_eos / p, or 1 / rho (cv); for the right-hand side and the Jacobian
+  bool cv;
+  template <bool INV>
+  __device__ __forceinline__ static FixPress of(const FixView& m, double pr, bool cv) {
+    FixPress q;
+    q.pr = pr;
+    q.a = pr * m.inv_r_eos;
+    q.b = INV ? (cv ? recip(pr) : m.r_eos * recip(pr)) : 0.0;
+    q.cv = cv;
+    return q;
+  }
+};
+
 // One cell (see warp_kinetics for the meaning of pr, cv and s.Jr).  RHS: form
 // out.f and out.fT; want_h: form out.cp_mass and out.h_mass.  img: the global
 // image, for the Jacobian's FP64 coefficients.
 template <bool JAC, int SPL, bool RHS>
 __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
                                              const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
-                                             double pr, CellOutT<SPL>& out, bool cv, bool want_h) {
+                                             const FixPress& pr, CellOutT<SPL>& out, bool want_h) {
+  const bool cv = pr.cv;
   const int ns = m.ns, nsp = m.nsp, nrpad = m.nrpad;
   const bool thermo = JAC || RHS || want_h;
   int64_t* G = reinterpret_cast<int64_t*>(s.gRT);
@@ -120,7 +142,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   const double sumYW = warp_isum(SPL == 1 ? yw[0] : yw[0] + yw[SPL - 1]);
   const FixT f = fix_T(T, m.lt);
   const double X = T * sumYW;
-  const double rho = cv ? pr : pr * m.inv_r_eos * recip(X);
+  const double rho = cv ? pr.pr : pr.a * recip(X);
   const double ctot = rho * sumYW;
   // ---- species k = lane + 32 j
   double my_cpR[SPL], my_hRT[SPL], my_c[SPL];
@@ -162,6 +184,9 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   // together, pass 4 blends.
   const int NF = m.nfall, f0 = m.nr - NF;
   double* fo = JAC ? s.Jr : s.fo;
+  // third-body concentrations, each row once, kept in the rate's place until the
+  // rate itself is known
+  for (int t = lane; t < m.ntb; t += WARP) s.q[m.nr - m.ntb + t] = fix_tb_conc(m, t, ctot, s.c);
   if (NF > 0) {
     const double Tinv = JAC ? invT : fix2d((int64_t)f.v, 70);
     for (int jb = lane; jb < 5 * NF; jb += WARP) {
@@ -186,7 +211,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       troe = fix_type(w) == 3;
       kinf = fo[lane];
       kratio = fo[WARP + lane];
-      Pr = kratio * fix_tb_conc(m, fix_tbrow(w), ctot, s.c);
+      Pr = kratio * s.q[f0 + lane];
       if (troe) Fc = fma(m.tr[lane], fo[2 * WARP + lane], fma(m.tr[16 + lane], fo[3 * WARP + lane], fo[4 * WARP + lane]));
     }
     const double Pr_src = __shfl_sync(FULL, Pr, lane >= NF && lane < 2 * NF ? lane - NF : 0);
@@ -196,22 +221,23 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
     // Pr / (1 + Pr) below makes the rate NaN as before
     const int64_t lg = log2_q52(lg_in, m.lt);
     const int64_t lgP = __shfl_sync(FULL, lg, lane < NF ? lane + NF : 0);
+    double dx = 0.0, dden = 1.0, lgd = 0.0, nnd = 0.0, d2 = 1.0;
+    if (troe) {
+      const int64_t xx = lgP - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
+      const int64_t nn = TROE_C75 - (mulhi_s(lg, TROE_M127) << 2);
+      const int64_t den = nn - (mulhi_s(xx, TROE_M14) << 1);
+      dx = fix2d(xx, 52);
+      dden = fix2d(den, 52);
+      lgd = fix2d(lg, 52);
+      d2 = dden * dden;
+      if (JAC) nnd = fix2d(nn, 52);
+    }
+    // one reciprocal for both: den^2 + x^2 on lane i, 1 + Pr on lane nfall + i
+    const double rc = recip(lane < NF ? fma(dx, dx, d2) : 1.0 + (lane < 2 * NF ? Pr_src : 0.0));
+    const double iopr = __shfl_sync(FULL, rc, lane < NF ? lane + NF : 0);
     if (lane < NF) {
-      double Fb = 1.0, R = 0.0, dx = 0.0, dden = 1.0, Qr = 1.0, lgd = 0.0, nnd = 0.0;
-      if (troe) {
-        const int64_t xx = lgP - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
-        const int64_t nn = TROE_C75 - (mulhi_s(lg, TROE_M127) << 2);
-        const int64_t den = nn - (mulhi_s(xx, TROE_M14) << 1);
-        dx = fix2d(xx, 52);
-        dden = fix2d(den, 52);
-        lgd = fix2d(lg, 52);
-        const double d2 = dden * dden;
-        Qr = recip(fma(dx, dx, d2));
-        R = d2 * Qr;
-        Fb = exp2_q52(d2fix52(lgd * R), m.et);
-        if (JAC) nnd = fix2d(nn, 52);
-      }
-      const double iopr = recip(1.0 + Pr);
+      const double R = d2 * rc;
+      const double Fb = troe ? exp2_q52(d2fix52(lgd * R), m.et) : 1.0;
       fo[5 * WARP + lane] = kinf * (Pr * iopr) * Fb;
       if (JAC) {
         const int r = f0 + lane;
@@ -265,7 +291,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       const double iKc = kr;                      // (falloff reactions: a = 0)
       double Mfac = 1.0;
       if (type == 1) {
-        Mfac = fix_tb_conc(m, fix_tbrow(w), ctot, s.c);
+        Mfac = s.q[r];
       } else if (type >= 2) {
         kf = fo[5 * WARP + r - f0];
         kr *= kf;
@@ -308,7 +334,24 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
     s.q[r] = q;
   }
   __syncwarp();
-  // ---- species: production rates
+  // ---- species: production rates.  The entries of all species are dealt out
+  // evenly over the lanes (19 each at 31 species and 160 reactions, where the
+  // longest species list has 34); a lane writes the sum of each piece of a
+  // species' list and the species' lane adds the pieces.
+  double* part = fo;
+  {
+    double acc = 0.0;
+    for (int e = 0; e < m.seg_len; ++e) {
+      const uint32_t w = m.seg[32 * e + lane];
+      const double q = s.q[w & 0xffffu], v = m.segv[(w >> 17) & 127u];
+      acc = fma(v, __hiloint2double(__double2hiint(q) ^ (int)((w << 15) & 0x80000000u), __double2loint(q)), acc);
+      if ((int)w < 0) {
+        part[(w >> 24) & 127u] = acc;
+        acc = 0.0;
+      }
+    }
+  }
+  __syncwarp();
   const double cvone = cv ? 1.0 : 0.0;
   double wm[SPL];
   double Ql = 0.0, Dl = 0.0, cpl = 0.0, hl = 0.0;
@@ -317,7 +360,9 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
     const int k = lane + 32 * j;
     wm[j] = 0.0;
     if (k < ns) {
-      for (int e = m.cstart[k]; e < m.cstart[k + 1]; ++e) wm[j] = fma(m.lnu[e], s.q[m.lr[e]], wm[j]);
+      const int e0 = m.piece[k], e1 = m.piece[k + 1];
+      if (e0 < e1) wm[j] = part[e0];
+      for (int e = e0 + 1; e < e1; ++e) wm[j] += part[e];
       if (RHS || JAC) {
         // constant volume: u_k/RT = h_k/RT - 1, cv_k/R = cp_k/R - 1
         Ql = fma(cv ? my_hRT[j] - 1.0 : my_hRT[j], wm[j], Ql);
@@ -339,7 +384,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   const double Q = warp_isum(Ql), D = warp_isum(Dl);
   const double invD = recip(D);
   const double fT = -T * Q * invD;
-  const double irho = recip(rho);
+  const double irho = cv ? pr.b : pr.b * X;
   out.fT = fT;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
@@ -350,6 +395,7 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   if (!JAC) return;
 
   // ---- Jacobian in concentration space: row k = species k ------------------
+  __syncwarp();   // the pieces lie in the rows
   const int ld = s.ldj, nslot = m.w3 ? 3 : 2;
   double JT[SPL];
 #pragma unroll
@@ -460,16 +506,16 @@ __device__ __noinline__ void kinetics_general(const uint8_t* __restrict__ img, c
 template <bool JAC, int SPL, bool RHS>
 __device__ __forceinline__ void kinetics_cell(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
                                               const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
-                                              double pr, CellOutT<SPL>& out, bool cv, bool want_h) {
+                                              const FixPress& pr, CellOutT<SPL>& out, bool want_h) {
   if (m.covers(T)) {
-    kinetics_fix<JAC, SPL, RHS>(m, img, L, s, lane, Yk, T, pr, out, cv, want_h);
+    kinetics_fix<JAC, SPL, RHS>(m, img, L, s, lane, Yk, T, pr, out, want_h);
   } else {
     CellOutT<SPL> o;
     double yk[SPL];
 #pragma unroll
     for (int j = 0; j < SPL; ++j) yk[j] = Yk[j];
     WarpScratch sc = s;
-    kinetics_general<JAC, SPL>(img, L, sc, lane, yk, T, pr, o, cv);
+    kinetics_general<JAC, SPL>(img, L, sc, lane, yk, T, pr.pr, o, pr.cv);
     out = o;
   }
 }

@@ -156,7 +156,7 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
             double* __restrict__ ho, double* __restrict__ jac, double* __restrict__ rhs_out,
             double* __restrict__ gscratch, int cv) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int base = FIX ? L.fix_bytes : L.bytes;
+  const int base = FIX ? (JAC ? L.fix_bytes : L.fix_bytes_rate) : L.bytes;
   stage_image(smem, FIX ? img + L.o_fix : img, base);
   MechView m;
   FixView x;
@@ -187,7 +187,7 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
       if (k < ns) Yk[j] = (layout == 1) ? Yg[(int64_t)k * n + cell] : Yg[cell * ns + k];
     }
     CellOutT<SPL> o;
-    if (FIX) kinetics_cell<JAC, SPL, RHS>(x, img, L, s, lane, Yk, T, p, o, cv != 0, cpo != nullptr || ho != nullptr);
+    if (FIX) kinetics_cell<JAC, SPL, RHS>(x, img, L, s, lane, Yk, T, FixPress::of<JAC || RHS>(x, p, cv != 0), o, cpo != nullptr || ho != nullptr);
     else warp_kinetics<JAC, SPL>(m, s, lane, Yk, T, p, o, cv != 0);
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
@@ -395,11 +395,13 @@ size_t small_smem(const ImageLayout& L) { return L.bytes + 3 * SMALL_NSMAX * SMA
 // layout too large for a block of 256 threads (the choice does not depend on
 // the block size a caller tunes, so one kernel serves every block size).
 // The image a block of the warp kernels stages.
-static size_t image_bytes(const ImageLayout& L) { return L.fix ? L.fix_bytes : L.bytes; }
+static size_t image_bytes(const ImageLayout& L, bool jac) {
+  return L.fix ? (jac ? L.fix_bytes : L.fix_bytes_rate) : L.bytes;
+}
 static bool warp_gj(const ImageLayout& L, bool jac) {
   if (L.nsp > 32) return true;
   if (!jac) return false;
-  return image_bytes(L) + (WARP_THREADS / 32) * scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) >
+  return image_bytes(L, true) + (WARP_THREADS / 32) * scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) >
          device_smem_optin();
 }
 
@@ -407,8 +409,8 @@ static int warp_block(int threads) { return threads == 64 || threads == 128 ? th
 
 size_t warp_smem(const ImageLayout& L, bool jac, int threads) {
   const int wpb = warp_block(threads) / 32;
-  if (warp_gj(L, jac)) return image_bytes(L) + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
-  return image_bytes(L) + wpb * scratch_doubles(L.nsp, L.nrpad, jac) * sizeof(double);
+  if (warp_gj(L, jac)) return image_bytes(L, jac) + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
+  return image_bytes(L, jac) + wpb * scratch_doubles(L.nsp, L.nrpad, jac) * sizeof(double);
 }
 
 int warp_block_candidates(int* out) {

@@ -21,7 +21,7 @@
 // order q-1, q, q+1 error estimates; Newton converged in the weighted max norm;
 // after an error-test failure with a stale Jacobian, a fresh one.  A cell whose
 // integration fails is integrated again at order <= 2, then 1.  The Newton matrix I - gamma*J is factored
-// in shared memory by a row-per-lane LU with partial pivoting that records the
+// by an LU with partial pivoting, its updates dealt out by elements, that records the
 // pivot order instead of swapping rows.  Step-size factors eta = (c*dsm)^(-1/(q+1))
 // are heuristics and are evaluated in FP32 (the oracle does the same); every
 // quantity of the solution itself stays FP64.
@@ -38,16 +38,19 @@ namespace flint {
 constexpr int REACTOR_THREADS = 256;
 constexpr int MAX_DEVICES = 64;
 
-// il1[q] = 1 / l_1 and Eq[q] = 1 / ((q + 1) l_1 + 1) of order q: per-order
-// constants of every step, tabulated so that a step carries two fewer FP64
-// divisions (each a dozen FP64-pipe instructions on this GPU).
-struct BdfL { double l[6][6]; double il1[6]; double Eq[6]; };
+// il1[q] = 1 / l_1, Eq[q] = 1 / ((q + 1) l_1 + 1) and the factors of the order
+// decision: per-order constants of every step, tabulated so that a step carries
+// no division by them (each nine FP64-pipe slots on this GPU).
+struct BdfL {
+  double l[6][6], il1[6], Eq[6];
+  double cdn[6], cup[6], cnew[6];   // order q - 1 and q + 1 error factors; l_q / (q + 1) of the new history entry
+};
 
 // l^(q)_j = coefficient of x^j in prod_{i=1..q} (1 + x/i)  (Nordsieck BDF of order q).
 static void bdf_coeffs(BdfL& B) {
   for (int q = 0; q < 6; ++q) {
     for (int j = 0; j < 6; ++j) B.l[q][j] = 0.0;
-    B.il1[q] = 0.0; B.Eq[q] = 0.0;
+    B.il1[q] = 0.0; B.Eq[q] = 0.0; B.cdn[q] = 0.0; B.cup[q] = 0.0; B.cnew[q] = 0.0;
   }
   for (int q = 1; q <= 5; ++q) {
     double* l = B.l[q];
@@ -56,6 +59,14 @@ static void bdf_coeffs(BdfL& B) {
       for (int j = i; j >= 1; --j) l[j] += l[j - 1] / (double)i;
     B.il1[q] = 1.0 / l[1];
     B.Eq[q] = 1.0 / std::fma((double)(q + 1), l[1], 1.0);
+    B.cnew[q] = l[q] / (double)(q + 1);
+  }
+  for (int q = 1; q <= 5; ++q) {
+    double fact = 1.0;
+    for (int i = 2; i <= q; ++i) fact *= i;
+    B.cdn[q] = q > 1 ? fact / ((double)q * B.l[q - 1][1]) : 0.0;
+    const double Kq = 1.0 + 1.0 / ((double)(q + 1) * B.l[q][1]);
+    B.cup[q] = q < 5 ? 1.0 / (Kq * (double)(q + 2) * B.l[q + 1][1]) : 0.0;
   }
 }
 
@@ -76,22 +87,46 @@ constexpr int MSBP = 20;
 constexpr int MSBJ = 50;
 constexpr int JSLOT = 32 * 32;   // doubles per saved-Jacobian slot of up to 31 species
 
+// sqrt(x) of a non-negative x: the SM's reciprocal square root (about 2^-20) and
+// one third-order (Householder) step, 5 FP64 operations where the library's takes
+// about 9 FP64-pipe slots; relative error below 2^-52.  Zero, subnormal, huge,
+// inf and NaN take the library's.
+static __device__ __noinline__ double sqrt_slow(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrt_fast(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  if (h - 0x03000000u >= 0x79000000u) return sqrt_slow(x);
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double t = x * r;
+  const double e = fma(-t, r, 1.0);                     // 1 - x r^2
+  return fma(t * e, fma(0.375, e, 0.5), t);
+}
+
+// a < b, a <= b of doubles that are not negative (NaN: false), as bit patterns:
+// an FP64 compare costs as much as a DADD.
+__device__ __forceinline__ bool lt_pos(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b) && __double_as_longlong(b) <= 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool le_pos(double a, double b) {
+  return __double_as_longlong(a) <= __double_as_longlong(b) && __double_as_longlong(b) <= 0x7ff0000000000000ll;
+}
+
 // Component k = lane + 32 j of the state lives in slot j (SPL slots per lane).
-// inv_nv = 1 / nv, formed once per cell (a division per norm is a dozen
-// FP64-pipe instructions).
+// inv_nv = 1 / nv, formed once per cell.  The norm carries no sign bit (NaN
+// stays NaN).
 template <int SPL>
 __device__ inline double wrms(const double (&v)[SPL], const double (&w)[SPL], int lane, int nv, double inv_nv) {
   double t = 0.0;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const double a = (lane + 32 * j < nv) ? v[j] * w[j] : 0.0;
-    t += a * a;
+    t = fma(a, a, t);
   }
-  return sqrt(warp_sum(t) * inv_nv);
+  return __longlong_as_double(absbits(sqrt_fast(warp_isum(t) * inv_nv)));
 }
 
 // Weighted max norm (the Newton convergence test), the maximum taken on the
-// bit patterns; the butterfly leaves the same value on every lane.  A NaN
+// bit patterns, high words first; the same value on every lane.  A NaN
 // component makes the norm NaN (the iteration then counts as diverged).
 template <int SPL>
 __device__ inline double wmax(const double (&v)[SPL], const double (&w)[SPL], int lane, int nv) {
@@ -99,65 +134,107 @@ __device__ inline double wmax(const double (&v)[SPL], const double (&w)[SPL], in
 #pragma unroll
   for (int j = 0; j < SPL; ++j)
     if (lane + 32 * j < nv) t = max(t, absbits(v[j] * w[j]));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t = max(t, __shfl_xor_sync(FULL, t, o));
-  return __longlong_as_double(t);
+  const unsigned h = (unsigned)(t >> 32), hmax = __reduce_max_sync(FULL, h);
+  const unsigned lmax = __reduce_max_sync(FULL, h == hmax ? (unsigned)t : 0u);
+  return __hiloint2double((int)hmax, (int)lmax);
 }
 
-// LU of the rows (row r = lane + 32 j) held at A[r*ld ...], partial pivoting by
-// the largest |a| (lowest row on ties; compared as bit patterns, see absbits);
-// the pivot order goes to piv[step] and each row remembers its step in mystep
-// (rows are not swapped).  Stored: L's multipliers; U with unit diagonal (each
-// pivot row's entries right of the pivot divided by the pivot, by the lanes in
-// parallel) and in the diagonal's place the pivot's reciprocal.  A solve then
-// scales once per lane and has no per-column multiply or division (an FP64
-// division is a dozen FP64-pipe instructions on this GPU, and a uniform
-// per-column multiply costs a whole warp instruction for one value).
+// LU of the matrix held by columns, A[c*ld + r], partial pivoting by the largest
+// |a| (lowest row on ties; compared as bit patterns, see absbits); the pivot
+// order goes to piv[step] and each row remembers its step in mystep (rows are
+// not swapped).  Stored: L's multipliers; U with unit diagonal (each pivot row's
+// entries right of the pivot divided by the pivot, by the lanes in parallel) and
+// in the diagonal's place the pivot's reciprocal.  A solve then scales once per
+// lane and has no per-column multiply or division.
+//
+// The rank-one update of step k covers the m = nv - 1 - k rows left times as many
+// columns; its m^2 elements are dealt out over the lanes (consecutive lanes take
+// consecutive rows of a column), so the multiply-adds of a 32 x 32 factorization
+// take 341 FP64 warp instructions where a row per lane takes 496 with half of
+// the lanes idle on average, and the elements of a matrix in global memory are
+// read by whole sectors.  col [nv] receives the rows' entries of column k and
+// prow [nv] the scaled pivot row (shared memory), act [nv] the rows left.
 template <int SPL>
-__device__ inline void warp_lu(double* A, int ld, int nv, int lane, int* piv, int (&mystep)[SPL]) {
+__device__ inline void warp_lu(double* A, int ld, int nv, int lane, int* piv, int (&mystep)[SPL], double* col,
+                               double* prow, int* act) {
 #pragma unroll
   for (int j = 0; j < SPL; ++j) mystep[j] = (lane + 32 * j < nv) ? -1 : 1 << 20;
   for (int k = 0; k < nv; ++k) {
+    double* ck = A + k * ld;
+    double a[SPL];
     long long cand = -1;
     int who = lane;
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int r = lane + 32 * j;
+      a[j] = 0.0;
       if (r < nv && mystep[j] < 0) {
-        const long long v = absbits(A[r * ld + k]);
+        a[j] = ck[r];
+        const long long v = absbits(a[j]);
         if (v > cand) { cand = v; who = r; }
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long oc = __shfl_xor_sync(FULL, cand, o);
-      const int ow = __shfl_xor_sync(FULL, who, o);
-      if (oc > cand || (oc == cand && ow < who)) { cand = oc; who = ow; }
-    }
-#pragma unroll
-    for (int j = 0; j < SPL; ++j)
-      if (lane + 32 * j == who) mystep[j] = k;
+    // the largest: by the high words (+ 1, 0 for lanes without a row), by the low
+    // words among those, by the row among those
+    const unsigned h = cand < 0 ? 0u : (unsigned)(cand >> 32) + 1u;
+    const unsigned hmax = __reduce_max_sync(FULL, h);
+    const unsigned l = h == hmax ? (unsigned)cand : 0u;
+    const unsigned lmax = __reduce_max_sync(FULL, l);
+    who = (int)__reduce_min_sync(FULL, h == hmax && l == lmax ? (unsigned)who : 0xffffu);
     if (lane == 0) piv[k] = who;
-    double* prow = A + who * ld;
-    const double inv = 1.0 / prow[k];
-    __syncwarp();
-    // U row of the pivot: entries right of the pivot scaled to a unit diagonal;
-    // the pivot's reciprocal in the diagonal's place
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) {
-      const int c = lane + 32 * j;
-      if (c > k && c < nv) prow[c] *= inv;
-    }
-    if (lane == (who & 31)) prow[k] = inv;
-    __syncwarp();
+    const double pivot = __shfl_sync(FULL, SPL == 1 || who < 32 ? a[0] : a[SPL - 1], who & 31);
+    const double inv = recip(pivot);
+    int left = 0;
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int r = lane + 32 * j;
-      if (r < nv && mystep[j] < 0) {
-        double* row = A + r * ld;
-        const double a = row[k];
-        row[k] = a * inv;
-        for (int c = k + 1; c < nv; ++c) row[c] -= a * prow[c];
+      if (r == who) mystep[j] = k;
+      const bool on = r < nv && mystep[j] < 0;
+      const unsigned bal = __ballot_sync(FULL, on);
+      if (on) {
+        const int rank = left + __popc(bal & ((1u << lane) - 1u));
+        act[rank] = r;
+        col[rank] = a[j];
+      }
+      left += __popc(bal);
+    }
+    // multipliers below the pivot, the pivot row right of it, the reciprocal
+#pragma unroll
+    for (int j = 0; j < SPL; ++j) {
+      const int r = lane + 32 * j, c = r;
+      if (r < nv && mystep[j] < 0) ck[r] = a[j] * inv;
+      if (r == who) ck[r] = inv;
+      if (c > k && c < nv) {
+        const double u = A[c * ld + who] * inv;
+        A[c * ld + who] = u;
+        prow[c] = u;
+      }
+    }
+    __syncwarp();
+    const int m = left, total = m * m;
+    if (m > 0) {
+      const float rm = 1.0f / (float)m;
+      const int dj = (int)(32.5f * rm), di = 32 - dj * m;        // 32 = dj m + di
+      int j = (int)(((float)lane + 0.5f) * rm), i = lane - j * m;   // lane = j m + i
+      int e = lane;
+      auto next = [&]() {
+        i += di; j += dj;
+        if (i >= m) { i -= m; ++j; }
+        e += 32;
+      };
+      for (; e + 32 < total;) {
+        double* p0 = A + (k + 1 + j) * ld + act[i];
+        const double u0 = prow[k + 1 + j], a0 = col[i], v0 = *p0;
+        next();
+        double* p1 = A + (k + 1 + j) * ld + act[i];
+        const double u1 = prow[k + 1 + j], a1 = col[i], v1 = *p1;
+        next();
+        *p0 = fma(-a0, u0, v0);
+        *p1 = fma(-a1, u1, v1);
+      }
+      if (e < total) {
+        double* p0 = A + (k + 1 + j) * ld + act[i];
+        *p0 = fma(-col[i], prow[k + 1 + j], *p0);
       }
     }
     __syncwarp();
@@ -169,6 +246,7 @@ template <int SPL>
 __device__ inline void warp_lu_solve(const double* A, int ld, int nv, int lane, const int* piv,
                                      const int (&mystep)[SPL], double (&b)[SPL]) {
   // forward: y_k = b_{piv[k]}; rows pivoted later subtract L * y_k
+#pragma unroll 4
   for (int k = 0; k < nv; ++k) {
     const int pk = piv[k];
     const double src = (SPL == 1 || (pk >> 5) == 0) ? b[0] : b[SPL - 1];
@@ -176,7 +254,7 @@ __device__ inline void warp_lu_solve(const double* A, int ld, int nv, int lane, 
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int r = lane + 32 * j;
-      if (r < nv && mystep[j] > k) b[j] -= A[r * ld + k] * yk;
+      if (r < nv && mystep[j] > k) b[j] = fma(-A[k * ld + r], yk, b[j]);
     }
   }
   // backward by columns on the unit-diagonal U: each row's y first divided by
@@ -186,8 +264,9 @@ __device__ inline void warp_lu_solve(const double* A, int ld, int nv, int lane, 
   for (int j = 0; j < SPL; ++j) {
     x[j] = 0.0;
     const int r = lane + 32 * j;
-    if (r < nv) b[j] *= A[r * ld + mystep[j]];
+    if (r < nv) b[j] *= A[mystep[j] * ld + r];
   }
+#pragma unroll 4
   for (int c = nv - 1; c >= 0; --c) {
     const int pc = piv[c];
     const double src = (SPL == 1 || (pc >> 5) == 0) ? b[0] : b[SPL - 1];
@@ -195,7 +274,7 @@ __device__ inline void warp_lu_solve(const double* A, int ld, int nv, int lane, 
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int r = lane + 32 * j;
-      if (r < nv && mystep[j] < c) b[j] -= A[r * ld + c] * xc;
+      if (r < nv && mystep[j] < c) b[j] = fma(-A[c * ld + r], xc, b[j]);
       if (r == c) x[j] = xc;
     }
   }
@@ -213,7 +292,7 @@ template <int SPL, bool FIX>
 __device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const FixView& x,
                                                    const uint8_t* __restrict__ img, const ImageLayout& L,
                                                    const WarpScratch& s, int lane, double p, bool cv,
-                                                   double gamma, int eval_J, double ya, double yb, double* Jg,
+                                                   const FixPress& fp, double gamma, int eval_J, double ya, double yb, double* Jg,
                                                    int* pivs) {
   constexpr int JW = 32 * SPL;
   const int ns = L.ns, nv = ns + 1, ld = s.ldj;
@@ -224,7 +303,7 @@ __device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const F
     yk[0] = (lane < ns) ? ya : 0.0;
     if (SPL > 1) yk[SPL - 1] = (lane + 32 < ns) ? yb : 0.0;
     CellOutT<SPL> co;
-    if (FIX) kinetics_cell<true, SPL, false>(x, img, L, s, lane, yk, Tv, p, co, cv, false);
+    if (FIX) kinetics_cell<true, SPL, false>(x, img, L, s, lane, yk, Tv, fp, co, false);
     else warp_kinetics<true, SPL>(m, s, lane, yk, Tv, p, co, cv);
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
@@ -234,27 +313,22 @@ __device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const F
         for (int c = 0; c < nv; ++c) Jg[c * JW + r] = row[c];
       }
     }
-  } else {
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) {
-      const int r = lane + 32 * j;
-      if (r < nv) {
-        double* row = s.Jr + r * ld;
-        for (int c = 0; c < nv; ++c) row[c] = Jg[c * JW + r];
-      }
-    }
+    __syncwarp();   // the rows are read: the columns of M take their place
   }
+  // M = I - gamma J by columns, from the saved copy (each lane reads back what it
+  // wrote)
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const int r = lane + 32 * j;
-    if (r < nv) {
-      double* row = s.Jr + r * ld;
-      for (int c = 0; c < nv; ++c) row[c] = (c == r ? 1.0 : 0.0) - gamma * row[c];
-    }
+    if (r < nv)
+#pragma unroll 4
+      for (int c = 0; c < nv; ++c) s.Jr[c * ld + r] = fma(-gamma, Jg[c * JW + r], c == r ? 1.0 : 0.0);
   }
   __syncwarp();
   int mystep[SPL];
-  warp_lu<SPL>(s.Jr, ld, nv, lane, pivs, mystep);
+  // (c, hRT and gRT hold nothing between evaluations; the second half of pivs is
+  // filled below)
+  warp_lu<SPL>(s.Jr, ld, nv, lane, pivs, mystep, s.c, s.hRT, pivs + 32 * SPL);
 #pragma unroll
   for (int j = 0; j < SPL; ++j) pivs[32 * SPL + lane + 32 * j] = mystep[j];
   __syncwarp();
@@ -362,6 +436,8 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
         if (lane + 32 * j < ns) yw += y[j] * invmw[lane + 32 * j];
       pr = p / (L.r_eos * T0 * warp_sum(yw));
     }
+    FixPress fp{};
+    if (FIX) fp = FixPress::of<true>(x, pr, cv);
     int status = FLINT_CELL_OK, nst = 0;
     if (bad) status = FLINT_CELL_NAN_INPUT;
     else if (T0 < o.tmin || T0 > o.tmax) status = FLINT_CELL_T_OUT_OF_RANGE;
@@ -392,7 +468,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
         double yk[SPL];
 #pragma unroll
         for (int j = 0; j < SPL; ++j) yk[j] = (lane + 32 * j < ns) ? yv[j] : 0.0;
-        if (FIX) kinetics_cell<false, SPL, true>(x, img, L, s, lane, yk, Tv, pr, co, cv, false);
+        if (FIX) kinetics_cell<false, SPL, true>(x, img, L, s, lane, yk, Tv, fp, co, false);
         else warp_kinetics<false, SPL>(m, s, lane, yk, Tv, pr, co, cv);
         __syncwarp();
 #pragma unroll
@@ -402,7 +478,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
       for (int j = 0; j < SPL; ++j) z[0][j] = y[j];
       rhs(y, f);
 #pragma unroll
-      for (int j = 0; j < SPL; ++j) ewt[j] = (lane + 32 * j < nv) ? 1.0 / (o.rtol * fabs(y[j]) + atol) : 0.0;
+      for (int j = 0; j < SPL; ++j) ewt[j] = (lane + 32 * j < nv) ? recip(fma(o.rtol, fabs(y[j]), atol)) : 0.0;
       const double fn = wrms<SPL>(f, ewt, lane, nv, inv_nv);
       double h = (fn * tout > 1.0) ? 1.0 / fn : tout;
 #pragma unroll
@@ -410,15 +486,15 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
       int q = 1;
       double t = 0.0;
       int ialth = 2, have_J = 0, jfresh = 0, nstJ = 0, nstP = 0, have_eprev = 0, last = 0;
-      double gammaJ = 0.0, crate = 1.0, etamax = 1.0e4;
+      double igammaJ = 0.0, crate = 1.0, etamax = 1.0e4;
       int mystep[SPL];
 #pragma unroll
       for (int j = 0; j < SPL; ++j) mystep[j] = 0;
 
-      while (t < tout) {
+      while (lt_pos(t, tout)) {
         if (nst >= o.max_steps) { status = FLINT_CELL_MAX_STEPS; break; }
         last = 0;
-        if (t + h >= tout) {
+        if (!lt_pos(t + h, tout)) {
           const double eta = (tout - t) / h;
           double r = 1.0;
 #pragma unroll
@@ -427,14 +503,14 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
           ialth = q + 1; have_eprev = 0; last = 1;
         }
 #pragma unroll
-        for (int j = 0; j < SPL; ++j) ewt[j] = (lane + 32 * j < nv) ? 1.0 / (o.rtol * fabs(z[0][j]) + atol) : 0.0;
+        for (int j = 0; j < SPL; ++j) ewt[j] = (lane + 32 * j < nv) ? recip(fma(o.rtol, fabs(z[0][j]), atol)) : 0.0;
         int ncf = 0, nef = 0, need_J = 0, accepted = 0;
         double dsm = 0.0;
         // the first Newton iterate of a step is judged with a rate of at least
         // 0.3: a small rate carried over from the last step would accept it unchecked
-        if (crate < 0.3) crate = 0.3;
+        if (lt_pos(crate, 0.3)) crate = 0.3;
         while (!accepted) {
-          if (h < 1e-300 || t + h == t) { status = FLINT_CELL_ERRTEST_FAIL; break; }
+          if (lt_pos(h, 1e-300) || __double_as_longlong(t + h) == __double_as_longlong(t)) { status = FLINT_CELL_ERRTEST_FAIL; break; }
 #pragma unroll
           for (int jj = 0; jj < 6; ++jj)
 #pragma unroll
@@ -447,8 +523,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
               if (k < q && jj >= k && jj <= q - 1)
 #pragma unroll
                 for (int j = 0; j < SPL; ++j) z[jj][j] += z[jj + 1][j];
-          const double l1 = B.l[q][1];
-          const double gamma = h / l1;
+          const double gamma = h * B.il1[q];
           double ypred[SPL];
 #pragma unroll
           for (int j = 0; j < SPL; ++j) ypred[j] = z[0][j];
@@ -457,8 +532,8 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
           double gamrat = 1.0;
           bool refresh = !have_J || need_J || nst >= nstP + MSBP;
           if (!refresh) {
-            gamrat = gamma / gammaJ;
-            refresh = fabs(gamrat - 1.0) > DGMAX;
+            gamrat = gamma * igammaJ;
+            refresh = lt_pos(gamrat, 1.0 - DGMAX) || lt_pos(1.0 + DGMAX, gamrat);
           }
           if (refresh) {
             const int eval_J = (!have_J || need_J || nst >= nstJ + MSBJ) ? 1 : 0;
@@ -466,11 +541,11 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
               ++n_jac;
               have_J = 1; jfresh = 1; nstJ = nst; need_J = 0;
             }
-            refresh_newton_matrix<SPL, FIX>(m, x, img, L, s, lane, pr, cv, gamma, eval_J, ypred[0], ypred[SPL - 1], Jg, pivs);
+            refresh_newton_matrix<SPL, FIX>(m, x, img, L, s, lane, pr, cv, fp, gamma, eval_J, ypred[0], ypred[SPL - 1], Jg, pivs);
 #pragma unroll
             for (int j = 0; j < SPL; ++j) mystep[j] = pivs[32 * SPL + lane + 32 * j];
             ++n_lu;
-            gammaJ = gamma; nstP = nst; crate = 1.0;
+            igammaJ = recip(gamma); nstP = nst; crate = 1.0;
             gamrat = 1.0;
           }
           double yv[SPL];
@@ -480,13 +555,13 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
           double delp = 0.0;
           const double Eq = B.Eq[q];
           const double il1 = B.il1[q];
-          const double sc = gamrat != 1.0 ? 2.0 / (1.0 + gamrat) : 1.0;
+          const double sc = gamrat != 1.0 ? 2.0 * recip(1.0 + gamrat) : 1.0;
           for (int mi = 0; mi < 3; ++mi) {
             ++n_newt;
             rhs(yv, f);
             double bv[SPL];
 #pragma unroll
-            for (int j = 0; j < SPL; ++j) bv[j] = (lane + 32 * j < nv) ? gamma * f[j] - z[1][j] * il1 - e[j] : 0.0;
+            for (int j = 0; j < SPL; ++j) bv[j] = (lane + 32 * j < nv) ? fma(gamma, f[j], fma(-il1, z[1][j], -e[j])) : 0.0;
             warp_lu_solve<SPL>(s.Jr, ld, nv, lane, pivs, mystep, bv);
             if (gamrat != 1.0) {
 #pragma unroll
@@ -495,10 +570,13 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
             const double del = wmax<SPL>(bv, ewt, lane, nv);
 #pragma unroll
             for (int j = 0; j < SPL; ++j) { e[j] += bv[j]; yv[j] = ypred[j] + e[j]; }
-            if (mi > 0) { const double r = del / delp; crate = (0.3 * crate > r) ? 0.3 * crate : r; }
-            const double dcon = del * (crate < 1.0 ? crate : 1.0) * Eq * 10.0;   // test constant 0.1
-            if (dcon <= 1.0) { conv = 1; break; }
-            if (mi > 0 && !(del <= 2.0 * delp)) break;
+            if (mi > 0) {
+              const double r = del * recip(delp), c3 = 0.3 * crate;
+              crate = lt_pos(r, c3) ? c3 : r;
+            }
+            const double dcon = del * (lt_pos(crate, 1.0) ? crate : 1.0) * (Eq * 10.0);   // test constant 0.1
+            if (le_pos(dcon, 1.0)) { conv = 1; break; }
+            if (mi > 0 && !le_pos(del, 2.0 * delp)) break;
             delp = del;
           }
           if (!conv) {
@@ -518,7 +596,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
             continue;
           }
           dsm = Eq * wrms<SPL>(e, ewt, lane, nv, inv_nv);
-          if (!(dsm <= 1.0)) {
+          if (!le_pos(dsm, 1.0)) {
 #pragma unroll
             for (int jj = 0; jj < 6; ++jj)
 #pragma unroll
@@ -531,9 +609,9 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
               eta = 0.1;
               if (q > 1) q = 1;
             } else {
-              eta = 1.0 / ((double)powf((float)(1.2 * dsm), 1.0f / (float)(q + 1)) + 1e-6);
-              if (eta > 0.9) eta = 0.9;
-              if (eta < 0.1) eta = 0.1;
+              eta = recip((double)powf((float)(1.2 * dsm), 1.0f / (float)(q + 1)) + 1e-6);
+              if (lt_pos(0.9, eta)) eta = 0.9;
+              if (lt_pos(eta, 0.1)) eta = 0.1;
             }
             double r = 1.0;
 #pragma unroll
@@ -549,17 +627,14 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
         ++nst;
         jfresh = 0;
 #pragma unroll
-        for (int jj = 0; jj <= 5; ++jj) if (jj <= q) for (int j = 0; j < SPL; ++j) z[jj][j] += B.l[q][jj] * e[j];
-        if (last || t >= tout) { t = tout; break; }
+        for (int jj = 0; jj <= 5; ++jj) if (jj <= q) for (int j = 0; j < SPL; ++j) z[jj][j] = fma(B.l[q][jj], e[j], z[jj][j]);
+        if (last || !lt_pos(t, tout)) { t = tout; break; }
         --ialth;
         double eta = 1.0;
         if (ialth <= 0) {
-          const double l1 = B.l[q][1];
-          const double etaq = 1.0 / ((double)powf((float)(1.2 * dsm), 1.0f / (float)(q + 1)) + 1.2e-6);
+          const double etaq = recip((double)powf((float)(1.2 * dsm), 1.0f / (float)(q + 1)) + 1.2e-6);
           double etadn = 0.0, etaup = 0.0;
           if (q > 1) {
-            double fact = 1.0;
-            for (int i = 2; i <= q; ++i) fact *= i;
             double zq[SPL];
 #pragma unroll
             for (int j = 0; j < SPL; ++j) {
@@ -567,32 +642,31 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
 #pragma unroll
               for (int jj = 2; jj <= 5; ++jj) if (jj == q) zq[j] = z[jj][j];
             }
-            const double ddn = wrms<SPL>(zq, ewt, lane, nv, inv_nv) * fact / ((double)q * B.l[q - 1][1]);
-            etadn = 1.0 / ((double)powf((float)(1.3 * ddn), 1.0f / (float)q) + 1.3e-6);
+            const double ddn = wrms<SPL>(zq, ewt, lane, nv, inv_nv) * B.cdn[q];
+            etadn = recip((double)powf((float)(1.3 * ddn), 1.0f / (float)q) + 1.3e-6);
           }
           if (q < qmax && have_eprev) {
-            const double Kq = 1.0 + 1.0 / ((double)(q + 1) * l1);
             double de[SPL];
 #pragma unroll
             for (int j = 0; j < SPL; ++j) de[j] = e[j] - eprev[j];
-            const double dup = wrms<SPL>(de, ewt, lane, nv, inv_nv) / (Kq * (double)(q + 2) * B.l[q + 1][1]);
-            etaup = 1.0 / ((double)powf((float)(1.4 * dup), 1.0f / (float)(q + 2)) + 1.4e-6);
+            const double dup = wrms<SPL>(de, ewt, lane, nv, inv_nv) * B.cup[q];
+            etaup = recip((double)powf((float)(1.4 * dup), 1.0f / (float)(q + 2)) + 1.4e-6);
           }
           int newq = q;
           eta = etaq;
-          if (etaup > eta && etaup >= etadn) { eta = etaup; newq = q + 1; }
-          else if (etadn > eta) { eta = etadn; newq = q - 1; }
+          if (lt_pos(eta, etaup) && le_pos(etadn, etaup)) { eta = etaup; newq = q + 1; }
+          else if (lt_pos(eta, etadn)) { eta = etadn; newq = q - 1; }
           if (newq == q + 1) {
-            const double fct = B.l[q][q] / (double)(q + 1);
+            const double fct = B.cnew[q];
 #pragma unroll
             for (int jj = 2; jj <= 5; ++jj) if (jj == q + 1) for (int j = 0; j < SPL; ++j) z[jj][j] = e[j] * fct;
           }
-          if (eta < 1.1 && newq == q) {
+          if (lt_pos(eta, 1.1) && newq == q) {
             eta = 1.0;
             ialth = 3;
           } else {
             q = newq;
-            if (eta > etamax) eta = etamax;
+            if (lt_pos(etamax, eta)) eta = etamax;
             ialth = q + 1;
           }
           have_eprev = 0;
