@@ -14,6 +14,7 @@
 #include <cstring>
 #include <string>
 #include <vector>
+#include <unordered_map>
 #include <algorithm>
 
 #include "flint_host.h"
@@ -138,6 +139,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   const ld LOG2E = 1.0L / logl(2.0L);
   const int ns = L.ns, nr = L.nr, S = L.nsp, P = L.nrpad, dummy = fix_dummy(S);
   L.fix = 0;
+  L.dq_rows = 8;
   if (d->nasa9 || nr < 1 || ns > dummy || L.nfall > 16) return;
   bool ok = true;
   auto q = [&](ld x, int bits, ld limit) -> int64_t {   // to fixed point, checked against the format's range
@@ -226,7 +228,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
     if (rs.size() > 3 || ps.size() > 3) ok = false;
     if (!ok) break;
     lists_r[rr] = rs; lists_p[rr] = ps;
-    w3 |= rs.size() > 2 || ps.size() > 2;
+    w3 |= rs.size() > 2 || ps.size() > 2 || d->rsp[3 * r + 2] >= 0 || d->psp[3 * r + 2] >= 0;
     const int dn = d->reversible[r] ? (int)ps.size() - (int)rs.size() : 0;
     uint64_t w = 0;
     for (int s = 0; s < 3; ++s) {
@@ -378,6 +380,76 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
     L.seg_len = len;
   }
   L.fix_ntb = tb;
+  // ---- Jacobian: every entry (row k, column j) of d(production)/dc as a run of
+  // terms coefficient x derivative of a reaction, the runs dealt out over the lanes,
+  // longest first to the lane with the least; column ns holds the third-body terms
+  // common to every column, row ns the derivative by T
+  const int nslot = w3 ? 3 : 2, rows = S + 1;
+  L.dq_rows = 2 * nslot + 2;
+  std::vector<uint32_t> term;
+  std::vector<uint16_t> target;
+  std::vector<double> coef{0.0};
+  std::unordered_map<double, int> index{{0.0, 0}};
+  L.term_len = 0;
+  {
+    typedef std::pair<int, double> Term;   // derivative index, coefficient
+    std::vector<std::vector<Term>> run((size_t)rows * rows);
+    const int* cs = reinterpret_cast<const int*>(img.data() + L.o_cstart);
+    const int* lr = reinterpret_cast<const int*>(img.data() + L.o_lr);
+    const double* nu = reinterpret_cast<const double*>(img.data() + L.o_lnu);
+    const int* tbp = reinterpret_cast<const int*>(img.data() + L.o_tbp);
+    const int* tbs = reinterpret_cast<const int*>(img.data() + L.o_tbs);
+    const double* tbv = reinterpret_cast<const double*>(img.data() + L.o_tbv);
+    const double* tbd = reinterpret_cast<const double*>(img.data() + L.o_tbd);
+    for (int k = 0; k < ns; ++k)
+      for (int e = cs[k]; e < cs[k + 1]; ++e) {
+        const int rr = lr[e];
+        for (int s = 0; s < (int)lists_r[rr].size(); ++s) run[k * rows + lists_r[rr][s]].push_back({s * P + rr, nu[e]});
+        for (int s = 0; s < (int)lists_p[rr].size(); ++s)
+          run[k * rows + lists_p[rr][s]].push_back({(nslot + s) * P + rr, nu[e]});
+        if (d->rtype[order[rr]] != 0) {
+          const int row = (int)(ix[rr] >> 48) & 0xff;
+          run[k * rows + ns].push_back({2 * nslot * P + rr, nu[e] * tbd[row]});
+          for (int u = tbp[row]; u < tbp[row + 1]; ++u)
+            run[k * rows + tbs[u]].push_back({2 * nslot * P + rr, nu[e] * tbv[u]});
+        }
+        run[ns * rows + k].push_back({(2 * nslot + 1) * P + rr, nu[e]});
+      }
+    std::vector<int> byLen;
+    for (int i = 0; i < rows * rows; ++i)
+      if (!run[i].empty()) byLen.push_back(i);
+    std::stable_sort(byLen.begin(), byLen.end(), [&](int a, int b) { return run[a].size() > run[b].size(); });
+    std::vector<std::vector<int>> lane(32);
+    std::vector<int> load(32, 0);
+    for (int i : byLen) {
+      const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+      lane[l].push_back(i);
+      load[l] += (int)run[i].size();
+    }
+    const int len = *std::max_element(load.begin(), load.end());
+    size_t runs = 0;
+    for (auto& v : lane) runs = std::max(runs, v.size());
+    term.assign((size_t)32 * len, 0);
+    target.assign((size_t)32 * runs, 0);
+    bool fits = L.dq_rows * P <= 0xffff && rows * rows <= 0xffff;
+    for (int l = 0; l < 32 && fits; ++l) {
+      int at = 0, ri = 0;
+      for (int i : lane[l]) {
+        for (size_t u = 0; u < run[i].size(); ++u) {
+          const auto known = index.insert({run[i][u].second, (int)coef.size()});
+          if (known.second) coef.push_back(run[i][u].second);
+          const int c = known.first->second;
+          if (c > 0xfff) { fits = false; break; }
+          term[(size_t)at * 32 + l] = (uint32_t)run[i][u].first | (uint32_t)c << 16 |
+                                      (u + 1 == run[i].size() ? 1u << 31 : 0u);
+          ++at;
+        }
+        target[(size_t)ri * 32 + l] = (uint16_t)i;
+        ++ri;
+      }
+    }
+    if (fits) L.term_len = len;
+  }
   // ---- sections
   int off = 0;
   auto sec = [&](int bytes) { int o = off; off = rup(off + bytes, 16); return o; };
@@ -393,7 +465,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   L.fix_bytes_cell = off;   // the thread-per-cell kernel needs no species lists
   L.f_seg = sec(4 * (int)seg.size()); L.f_segv = sec(8 * (int)segv.size()); L.f_piece = sec(4 * (S + 1));
   L.fix_bytes_rate = off;   // kernels without a Jacobian need no species lists
-  L.f_cstart = sec(4 * (S + 1)); L.f_lr = sec(4 * nlist); L.f_lnu = sec(8 * nlist);
+  L.f_term = sec(4 * (int)term.size()); L.f_target = sec(2 * (int)target.size()); L.f_coef = sec(8 * (int)coef.size());
   L.o_fix = L.bytes;
   L.fix_bytes = off;
   img.resize((size_t)L.bytes + off, 0);
@@ -408,8 +480,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   put(L.f_tr, tr.data(), 8 * 5 * 16);
   put(L.f_tbd, img.data() + L.o_tbd, 8 * L.ntb); put(L.f_tbp, img.data() + L.o_tbp, 4 * (L.ntb + 1));
   put(L.f_tbs, img.data() + L.o_tbs, 4 * ntbl); put(L.f_tbv, img.data() + L.o_tbv, 8 * (size_t)((L.o_cstart - L.o_tbv) / 8));
-  put(L.f_cstart, img.data() + L.o_cstart, 4 * (S + 1)); put(L.f_lr, img.data() + L.o_lr, 4 * nlist);
-  put(L.f_lnu, img.data() + L.o_lnu, 8 * nlist);
+  put(L.f_term, term.data(), 4 * term.size()); put(L.f_target, target.data(), 2 * target.size());
+  put(L.f_coef, coef.data(), 8 * coef.size());
   put(L.f_seg, seg.data(), 4 * seg.size()); put(L.f_segv, segv.data(), 8 * segv.size());
   put(L.f_piece, piece.data(), 4 * (S + 1));
   put(L.f_cx, cx.data(), 8 * P); put(L.f_cy, cy.data(), 8 * P);

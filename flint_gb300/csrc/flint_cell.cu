@@ -64,7 +64,7 @@ __device__ __noinline__ void cell_general(const uint8_t* __restrict__ img, const
                                           int cv) {
   const int ns = L.ns, nv = ns + 1;
   const double* mw = reinterpret_cast<const double*>(img + L.o_mw);
-  const WarpScratch s = carve2(scratch, nullptr, L.nsp, L.nrpad);
+  const WarpScratch s = carve2(scratch, nullptr, L);
   double Yk[SPL];
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {

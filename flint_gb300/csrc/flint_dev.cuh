@@ -90,7 +90,11 @@ struct ImageLayout {
   int f_rs, f_rw, f_rv;          // net coefficients by reaction: int32 [nr+1], int32 words species | code << 8
                                  // (code +1, -1, or 2 + an index of f_rv), double values
   int f_exp, f_log;              // int64 [256], [128][2]
-  int f_cstart, f_lr, f_lnu;     // as the o_ ones (the Jacobian's species rows)
+  // Jacobian terms: uint32 [term_len][32] words (derivative | coefficient << 16 |
+  // last-of-run << 31), uint16 [runs][32] targets (row (nsp + 1) + column), values;
+  // term_len = 0: the mechanism's Jacobian takes the FP64 path
+  int f_term, f_target, f_coef, term_len;
+  int dq_rows;                   // rows of derivatives per reaction (WarpScratch::dq)
   // species sums, the entries of all species dealt out evenly over the lanes:
   // uint32 [seg_len][32] words (reaction | sign << 16 | value << 17 | piece << 24 |
   // last-of-piece << 31), values, and int32 [nsp+1] first piece of each species
@@ -111,10 +115,10 @@ struct MechView {
   const int *tbp, *tbs;
   const double* nasa9;   // null: NASA-7 (nasa)
   const double* logtab;
-  int nfall;
+  int nfall, nslot;      // nslot: slots a side that any reaction uses (rows of dq)
 
   __host__ __device__ void bind(const ImageLayout& L, const uint8_t* base) {
-    ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; ntb = L.ntb; nfall = L.nfall;
+    ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; ntb = L.ntb; nfall = L.nfall; nslot = L.dq_rows / 2 - 1;
     exptab = (const double*)(base + L.o_exptab);
     r_eos = L.r_eos; r_thermo = L.r_thermo; lnpref_rth = L.lnpref_rth; inv_r_eos = L.inv_r_eos;
     mw = (const double*)(base + L.o_mw); invmw = (const double*)(base + L.o_invmw);
@@ -301,14 +305,14 @@ struct WarpScratch {
   double* q;      // [nrpad] rates of progress
   double* fo;     // [8][32] falloff pre-pass values (aliases Jr in Jacobian mode)
   // Jacobian mode only
-  double* dq;     // [8][nrpad]: 6 sparse partials (3 reactant, 3 product slots), tb coef, dq/dT
+  double* dq;     // [dq_rows][nrpad]: partials (nslot reactant, nslot product slots), tb coef, dq/dT
   double* Jr;     // [n][ldj] rows (species rows then T row), ldj = nsp+1 (odd stride)
   int ldj;
 };
 
 // Per-warp scratch in two parts.  The small part (shared memory): c, hRT, gRT
 // [nsp each], q [nrpad] and the falloff pre-pass area [8][32].  The Jacobian
-// part: dq [8][nrpad] and the rows Jr [(nsp+1)^2] -- in shared memory for up to
+// part: dq [dq_rows][nrpad] and the rows Jr [(nsp+1)^2] -- in shared memory for up to
 // 31 species, in a per-warp slot of global memory (L2-resident) for 32-63.
 // The falloff pre-pass of a Jacobian evaluation uses Jr (written only after the
 // rates of progress are done).
@@ -323,32 +327,33 @@ __host__ __device__ inline int fix_dummy(int nsp) { return nsp == 64 ? 63 : nsp;
 __host__ __device__ inline int scratch_small_doubles(int nsp, int nrpad) {
   return (3 * species_stride(nsp) + nrpad + 8 * 32 + 1) & ~1;   // keep 16-byte alignment
 }
-__host__ __device__ inline int scratch_jac_doubles(int nsp, int nrpad) {
-  return (8 * nrpad + (nsp + 1) * (nsp + 1) + 1) & ~1;
+__host__ __device__ inline int scratch_jac_doubles(const ImageLayout& L) {
+  return (L.dq_rows * L.nrpad + (L.nsp + 1) * (L.nsp + 1) + 1) & ~1;
 }
 // One block of scratch per warp.  With the Jacobian, the derivative rows dq
 // start where the falloff scratch fo starts: fo is used only by the kernel
 // calls without the Jacobian (in the Jacobian call it lives in Jr), and dq only
-// inside a Jacobian call, so the two may share (8 nrpad >= 256 doubles).
-__host__ __device__ inline int scratch_doubles(int nsp, int nrpad, bool jac) {
-  return jac ? ((3 * species_stride(nsp) + nrpad + 8 * nrpad + (nsp + 1) * (nsp + 1) + 1) & ~1)
-             : scratch_small_doubles(nsp, nrpad);
+// inside a Jacobian call, so the two may share (dq and Jr together hold 256 doubles).
+__host__ __device__ inline int scratch_doubles(const ImageLayout& L, bool jac) {
+  return jac ? ((3 * species_stride(L.nsp) + L.nrpad + scratch_jac_doubles(L) + 1) & ~1)
+             : scratch_small_doubles(L.nsp, L.nrpad);
 }
 
-__device__ inline WarpScratch carve2(double* small, double* jacbuf, int nsp, int nrpad) {
+__device__ inline WarpScratch carve2(double* small, double* jacbuf, const ImageLayout& L) {
+  const int nsp = L.nsp, nrpad = L.nrpad;
   WarpScratch s;
   const int ss = species_stride(nsp);
   s.c = small; s.hRT = small + ss; s.gRT = small + 2 * ss; s.q = small + 3 * ss;
   s.fo = s.q + nrpad;
   s.ldj = nsp + 1;
   s.dq = jacbuf;
-  s.Jr = jacbuf ? jacbuf + 8 * nrpad : nullptr;
+  s.Jr = jacbuf ? jacbuf + L.dq_rows * nrpad : nullptr;
   return s;
 }
 
 // Both parts contiguous in one buffer (shared memory, up to 31 species).
-__device__ inline WarpScratch carve(double* p, int nsp, int nrpad, bool jac) {
-  return carve2(p, jac ? p + 3 * species_stride(nsp) + nrpad : nullptr, nsp, nrpad);
+__device__ inline WarpScratch carve(double* p, const ImageLayout& L, bool jac) {
+  return carve2(p, jac ? p + 3 * species_stride(L.nsp) + L.nrpad : nullptr, L);
 }
 
 // Cell-level results held per lane: lane k (< ns) gets species k, the T-row
@@ -616,7 +621,7 @@ __device__ void warp_kinetics(const MechView& m, const WarpScratch& s, int lane,
           double d = dpf[sl];
 #pragma unroll
           for (int u = 0; u < MAXSIDE; ++u) if (u != sl) d *= pwf[u];
-          s.dq[sl * nrpad + r] = kM * d;
+          if (sl < m.nslot) s.dq[sl * nrpad + r] = kM * d;
           double e = 0.0;
           if (rev) {
             e = dpr[sl];
@@ -624,13 +629,13 @@ __device__ void warp_kinetics(const MechView& m, const WarpScratch& s, int lane,
             for (int u = 0; u < MAXSIDE; ++u) if (u != sl) e *= pwr[u];
             e = -kM * invKc * e;
           }
-          s.dq[(3 + sl) * nrpad + r] = e;
+          if (sl < m.nslot) s.dq[(m.nslot + sl) * nrpad + r] = e;
         }
         double tb = 0.0;
         if (type == 1) tb = keff * (Pf - (rev ? invKc * Pr : 0.0));
         else if (type >= 2) tb = dkdM * (Pf - (rev ? invKc * Pr : 0.0));
-        s.dq[6 * nrpad + r] = tb;
-        s.dq[7 * nrpad + r] = fwd * dlnkeff - rvs * (dlnkeff - dlnKc);
+        s.dq[2 * m.nslot * nrpad + r] = tb;
+        s.dq[(2 * m.nslot + 1) * nrpad + r] = fwd * dlnkeff - rvs * (dlnkeff - dlnKc);
       }
     }
     s.q[r] = q;
@@ -695,16 +700,16 @@ __device__ void warp_kinetics(const MechView& m, const WarpScratch& s, int lane,
           int sp = m.rsp[sl * nrpad + r];
           if (sp >= 0) Jrow[sp] += nu * s.dq[sl * nrpad + r];
           int sq = m.psp[sl * nrpad + r];
-          if (sq >= 0) Jrow[sq] += nu * s.dq[(3 + sl) * nrpad + r];
+          if (sq >= 0) Jrow[sq] += nu * s.dq[(m.nslot + sl) * nrpad + r];
         }
         const uint32_t w = m.code[r];
         if (rx_type(w) != 0) {
-          const double t = nu * s.dq[6 * nrpad + r];
+          const double t = nu * s.dq[2 * m.nslot * nrpad + r];
           const int row = rx_tbrow(w);
           tball = fma(t, m.tbd[row], tball);
           for (int q = m.tbp[row]; q < m.tbp[row + 1]; ++q) Jrow[m.tbs[q]] += t * m.tbv[q];
         }
-        JT[j] += nu * s.dq[7 * nrpad + r];
+        JT[j] += nu * s.dq[(2 * m.nslot + 1) * nrpad + r];
       }
       if (tball != 0.0)
         for (int jj = 0; jj < ns; ++jj) Jrow[jj] += tball;

@@ -27,12 +27,14 @@ struct FixView {
   int ns, nr, nrpad, nsp, nfall, dummy, w3, ntb, seg_len;
   double inv_r_eos, r_eos, r_thermo, Tlo, Thi;
   int64_t lC;
-  const double *mw, *invmw, *tr, *tbd, *tbv, *lnu;
+  const double *mw, *invmw, *tr, *tbd, *tbv;
   const int64_t *tmid, *a, *ra;
   const uint64_t *g, *h, *c, *b, *e, *rb, *re, *et, *lt, *ix, *cx, *cy;
-  const int *tbp, *tbs, *cstart, *lr, *rs, *rw, *piece;
-  const double *rv, *segv;
-  const uint32_t* seg;
+  const int *tbp, *tbs, *rs, *rw, *piece;
+  const double *rv, *segv, *coef;
+  const uint32_t *seg, *term;
+  const uint16_t* target;
+  int term_len;
   __device__ __forceinline__ void bind(const ImageLayout& L, const uint8_t* base) {
     ns = L.ns; nr = L.nr; nrpad = L.nrpad; nsp = L.nsp; nfall = L.nfall; dummy = fix_dummy(L.nsp); w3 = L.fix_w3;
     ntb = L.fix_ntb; seg_len = L.seg_len;
@@ -40,14 +42,18 @@ struct FixView {
     auto D = [&](int o) { return (const double*)(base + o); };
     auto I = [&](int o) { return (const int64_t*)(base + o); };
     auto U = [&](int o) { return (const uint64_t*)(base + o); };
-    mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv); lnu = D(L.f_lnu);
+    mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv);
     tmid = I(L.f_tmid); a = I(L.f_a); ra = I(L.f_ra);
     g = U(L.f_g); h = U(L.f_h); c = U(L.f_c); b = U(L.f_b); e = U(L.f_e);
     rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); cx = U(L.f_cx); cy = U(L.f_cy);
     tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
     rs = (const int*)(base + L.f_rs); rw = (const int*)(base + L.f_rw); rv = D(L.f_rv);
     seg = (const uint32_t*)(base + L.f_seg); segv = D(L.f_segv); piece = (const int*)(base + L.f_piece);
-    cstart = (const int*)(base + L.f_cstart); lr = (const int*)(base + L.f_lr);
+    bind_terms(L, base);
+  }
+  __device__ __forceinline__ void bind_terms(const ImageLayout& L, const uint8_t* base) {
+    term = (const uint32_t*)(base + L.f_term); target = (const uint16_t*)(base + L.f_target);
+    coef = (const double*)(base + L.f_coef); term_len = L.term_len;
   }
   __device__ __forceinline__ bool covers(double T) const { return T >= Tlo && T < Thi; }
 };
@@ -123,12 +129,13 @@ struct FixPress {
 };
 
 // One cell (see warp_kinetics for the meaning of pr, cv and s.Jr).  RHS: form
-// out.f and out.fT; want_h: form out.cp_mass and out.h_mass.  img: the global
-// image, for the Jacobian's FP64 coefficients.
+// out.f and out.fT; want_h: form out.cp_mass and out.h_mass.  JAC: the Jacobian is
+// written to dst by columns of dld doubles; img: the global image, for its FP64
+// coefficients.
 template <bool JAC, int SPL, bool RHS>
 __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
                                              const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
-                                             const FixPress& pr, CellOutT<SPL>& out, bool want_h) {
+                                             const FixPress& pr, CellOutT<SPL>& out, bool want_h, double* dst, int dld) {
   const bool cv = pr.cv;
   const int ns = m.ns, nsp = m.nsp, nrpad = m.nrpad;
   const bool thermo = JAC || RHS || want_h;
@@ -301,33 +308,36 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       const double fwd = kf * Pf;
       q = fma(-kr, Pr, fwd);
       if (JAC) {
+        // derivatives by factor; by the third body; T times the one by T
+        const int ns2 = m.w3 ? 3 : 2;
         const double kfM = type == 1 ? kf * Mfac : kf, krM = type == 1 ? kr * Mfac : kr;
-        s.dq[r] = kfM * c1;
-        s.dq[nrpad + r] = kfM * c0;
-        s.dq[3 * nrpad + r] = -krM * d1;
-        s.dq[4 * nrpad + r] = -krM * d0;
+        const double rvs = krM * Pr;
         if (m.w3) {
-          s.dq[r] *= c2;
-          s.dq[nrpad + r] *= c2;
+          s.dq[r] = kfM * c1 * c2;
+          s.dq[nrpad + r] = kfM * c0 * c2;
           s.dq[2 * nrpad + r] = kfM * (c0 * c1);
-          s.dq[3 * nrpad + r] *= d2;
-          s.dq[4 * nrpad + r] *= d2;
+          s.dq[3 * nrpad + r] = -krM * d1 * d2;
+          s.dq[4 * nrpad + r] = -krM * d0 * d2;
           s.dq[5 * nrpad + r] = -krM * (d0 * d1);
+        } else {
+          s.dq[r] = kfM * c1;
+          s.dq[nrpad + r] = kfM * c0;
+          s.dq[2 * nrpad + r] = -krM * d1;
+          s.dq[3 * nrpad + r] = -krM * d0;
         }
         double dlnk, tb = 0.0;
         if (type >= 2) {
-          dlnk = fo[6 * WARP + r - f0];
-          tb = fo[7 * WARP + r - f0] * fma(-iKc, Pr, Pf);
+          dlnk = fo[6 * WARP + r - f0] * T;
+          tb = fo[7 * WARP + r - f0] * fma(-iKc, Pr, Pf);   // dkeff/dM (Pf - Pr/Kc)
         } else {
-          dlnk = fma(gE[r], invT, gb[r]) * invT;
+          dlnk = fma(gE[r], invT, gb[r]);
           if (type == 1) tb = q;
         }
-        double dH = s.hRT[p0] + s.hRT[p1] - s.hRT[r0] - s.hRT[r1];
+        double dH = s.hRT[p0] + s.hRT[p1] - s.hRT[r0] - s.hRT[r1] - (double)fix_dn(w);
         if (m.w3) dH += s.hRT[fix_idx(w, 5)] - s.hRT[fix_idx(w, 2)];
-        const double dlnKc = rev ? (dH - (double)fix_dn(w)) * invT : 0.0;
+        s.dq[2 * ns2 * nrpad + r] = tb;
         // fwd dlnk - rvs (dlnk - dlnKc) = q dlnk + rvs dlnKc
-        s.dq[6 * nrpad + r] = tb;
-        s.dq[7 * nrpad + r] = Mfac * fma(q, dlnk, kr * Pr * dlnKc);
+        s.dq[(2 * ns2 + 1) * nrpad + r] = fma(type == 1 ? q * Mfac : q, dlnk, rvs * dH);
       }
       if (type == 1) q *= Mfac;
     }
@@ -395,99 +405,104 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   if (!JAC) return;
 
   // ---- Jacobian in concentration space: row k = species k ------------------
+  // Every entry is a run of terms, the runs dealt out evenly over the lanes (88
+  // multiply-adds a lane at 31 species and 160 reactions, where a row per lane
+  // took about 380: the longest species list times four, and third-body rows met
+  // at different places of different lists).  Column ns collects what a third
+  // body adds to every column, row ns T times the derivative by T.
   __syncwarp();   // the pieces lie in the rows
-  const int ld = s.ldj, nslot = m.w3 ? 3 : 2;
-  double JT[SPL];
+  const int ld = s.ldj;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const int k = lane + 32 * j;
-    JT[j] = 0.0;
-    if (k < ns) {
-      double* Jrow = s.Jr + k * ld;
-      for (int jj = 0; jj < ns; ++jj) Jrow[jj] = 0.0;
-      double tball = 0.0;   // third-body terms common to every column
-      for (int e = m.cstart[k]; e < m.cstart[k + 1]; ++e) {
-        const int r = m.lr[e];
-        const double nu = m.lnu[e];
-        const uint64_t w = m.ix[r];
-        for (int sl = 0; sl < nslot; ++sl) {
-          const int sp = fix_idx(w, sl), sq = fix_idx(w, 3 + sl);
-          if (sp != m.dummy) Jrow[sp] = fma(nu, s.dq[sl * nrpad + r], Jrow[sp]);
-          if (sq != m.dummy) Jrow[sq] = fma(nu, s.dq[(3 + sl) * nrpad + r], Jrow[sq]);
-        }
-        if (fix_type(w) != 0) {
-          const double t = nu * s.dq[6 * nrpad + r];
-          const int row = fix_tbrow(w);
-          tball = fma(t, m.tbd[row], tball);
-          for (int q = m.tbp[row]; q < m.tbp[row + 1]; ++q) Jrow[m.tbs[q]] = fma(t, m.tbv[q], Jrow[m.tbs[q]]);
-        }
-        JT[j] = fma(nu, s.dq[7 * nrpad + r], JT[j]);
+    if (k <= ns)
+      for (int jj = 0; jj <= ns; ++jj) s.Jr[k * ld + jj] = 0.0;
+  }
+  __syncwarp();
+  {
+    double acc = 0.0;
+    const uint16_t* target = m.target + lane;
+    for (int e = 0; e < m.term_len; ++e) {
+      const uint32_t w = m.term[32 * e + lane];
+      acc = fma(m.coef[(w >> 16) & 0xfffu], s.dq[w & 0xffffu], acc);
+      if ((int)w < 0) {
+        s.Jr[*target] = acc;
+        target += WARP;
+        acc = 0.0;
       }
-      if (tball != 0.0)
-        for (int jj = 0; jj < ns; ++jj) Jrow[jj] += tball;
     }
   }
   __syncwarp();
   // S_k = sum_j c_j Jc[k][j] (row k); HJ_m = sum_k hRT_k Jc[k][m] (column m)
-  double Sk[SPL], HJ[SPL];
-  double HSl = 0.0, dQTl = 0.0, dDTl = 0.0;
+  double Sk[SPL], HJ[SPL], tball[SPL], JT[SPL];
+  double HSl = 0.0, dQTl = 0.0, dDTl = 0.0, HTl = 0.0;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const int k = lane + 32 * j;
-    Sk[j] = 0.0; HJ[j] = 0.0;
+    Sk[j] = 0.0; HJ[j] = 0.0; tball[j] = 0.0; JT[j] = 0.0;
     if (k < ns) {
       const double* Jrow = s.Jr + k * ld;
-      const double* a = (const double*)(img + L.o_nasa) + (__double_as_longlong(T) <= m.tmid[k] ? 0 : 7 * nsp) + k;
-      const double dcp = a[nsp] + T * (2.0 * a[2 * nsp] + T * (3.0 * a[3 * nsp] + T * 4.0 * a[4 * nsp]));
+      tball[j] = Jrow[ns];
+      JT[j] = s.Jr[ns * ld + k] * invT;
+      const double* a = (const double*)(img + L.o_nasa) + k;
+      const double tm = a[14 * nsp];
+      a += __double_as_longlong(T) <= __double_as_longlong(tm) ? 0 : 7 * nsp;
+      const double dcp = fma(T, fma(T, fma(4.0 * T, a[4 * nsp], 3.0 * a[3 * nsp]), 2.0 * a[2 * nsp]), a[nsp]);
       if (cv) {
         // rho fixed: no dependence of c on T or through rho on Y (Sk = 0)
-        for (int kk = 0; kk < ns; ++kk) HJ[j] += (s.hRT[kk] - 1.0) * s.Jr[kk * ld + k];
+        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk] - 1.0, s.Jr[kk * ld + k], HJ[j]);
+        HTl += (my_hRT[j] - 1.0) * tball[j];
         dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + (my_hRT[j] - 1.0) * JT[j];
         dDTl += my_c[j] * dcp;
       } else {
+        Sk[j] = tball[j] * ctot;
         for (int jj = 0; jj < ns; ++jj) Sk[j] = fma(s.c[jj], Jrow[jj], Sk[j]);
         for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk], s.Jr[kk * ld + k], HJ[j]);
-        HSl += my_hRT[j] * Sk[j];
+        HTl = fma(my_hRT[j], tball[j], HTl);
+        HSl = fma(my_hRT[j], Sk[j], HSl);
         dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + my_hRT[j] * (JT[j] - Sk[j] * invT);
         dDTl += my_c[j] * (dcp - my_cpR[j] * invT);
       }
     }
   }
-  const double HS = warp_isum(HSl);
-  __syncwarp();
+  const double HS = warp_isum(HSl), HT = warp_isum(HTl);
   const double wbar = recip(sumYW);
   const double wr = cv ? 0.0 : wbar * irho;
   const double dQT = warp_isum(dQTl), dDT = warp_isum(dDTl);
   const double QD = Q * invD, TD = T * invD;
   const double JTT = -QD - TD * (dQT - QD * dDT);
-  double JTm[SPL];
+  // the T row by columns, then row by row (lanes = rows) into (Y, T) variables:
+  // W_k (Jc + tball - wr t_k) / W_j, t_k = S_k - w_k
+  double Wk[SPL], off[SPL], last[SPL];
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const int k = lane + 32 * j;
-    JTm[j] = 0.0;
+    Wk[j] = off[j] = last[j] = 0.0;
     if (k < ns) {
       const double rw = rho * m.invmw[k], ww = cv ? 0.0 : wbar * m.invmw[k];
-      const double dQ = rw * HJ[j] - ww * HS;
+      const double dQ = rw * (HJ[j] + HT) - ww * HS;
       const double dD = rw * (my_cpR[j] - cvone) - ww * D;
-      JTm[j] = -TD * (dQ - QD * dD);
-      // species row k in (Y, T) variables
+      s.q[k] = -TD * (dQ - QD * dD);
       const double tk = Sk[j] - wm[j];
-      const double Wk = m.mw[k];
-      const double wt = wr * tk;
-      double* Jrow = s.Jr + k * ld;
-      for (int jj = 0; jj < ns; ++jj) Jrow[jj] = Wk * m.invmw[jj] * (Jrow[jj] - wt);
-      Jrow[ns] = (Wk * irho) * (cv ? JT[j] : JT[j] - tk * invT);
+      Wk[j] = m.mw[k];
+      off[j] = Wk[j] * (tball[j] - wr * tk);
+      last[j] = (Wk[j] * irho) * (cv ? JT[j] : JT[j] - tk * invT);
     }
   }
   __syncwarp();
-  // T row (row ns)
-  double* JrowT = s.Jr + ns * ld;
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
     const int k = lane + 32 * j;
-    if (k < ns) JrowT[k] = JTm[j];
+    if (k <= ns) {
+      const double* Jrow = s.Jr + k * ld;
+#pragma unroll 4
+      for (int jj = 0; jj < ns; ++jj) {
+        const double v = fma(Wk[j], Jrow[jj], off[j]) * m.invmw[jj];
+        dst[(int64_t)jj * dld + k] = k < ns ? v : s.q[jj];
+      }
+      dst[(int64_t)ns * dld + k] = k < ns ? last[j] : JTT;
+    }
   }
-  if (lane == 0) JrowT[ns] = JTT;
   __syncwarp();
 }
 
@@ -502,22 +517,25 @@ __device__ __noinline__ void kinetics_general(const uint8_t* __restrict__ img, c
   warp_kinetics<JAC, SPL>(g, s, lane, Yk, T, pr, out, cv);
 }
 
-// The fixed-point path where the cell's temperature allows it.
+// The fixed-point path where the cell's temperature allows it.  Returns whether
+// the Jacobian was written to dst (else its rows are in s.Jr).
 template <bool JAC, int SPL, bool RHS>
-__device__ __forceinline__ void kinetics_cell(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
+__device__ __forceinline__ bool kinetics_cell(const FixView& m, const uint8_t* __restrict__ img, const ImageLayout& L,
                                               const WarpScratch& s, int lane, const double (&Yk)[SPL], double T,
-                                              const FixPress& pr, CellOutT<SPL>& out, bool want_h) {
-  if (m.covers(T)) {
-    kinetics_fix<JAC, SPL, RHS>(m, img, L, s, lane, Yk, T, pr, out, want_h);
-  } else {
-    CellOutT<SPL> o;
-    double yk[SPL];
-#pragma unroll
-    for (int j = 0; j < SPL; ++j) yk[j] = Yk[j];
-    WarpScratch sc = s;
-    kinetics_general<JAC, SPL>(img, L, sc, lane, yk, T, pr.pr, o, pr.cv);
-    out = o;
+                                              const FixPress& pr, CellOutT<SPL>& out, bool want_h, double* dst = nullptr,
+                                              int dld = 0) {
+  if (m.covers(T) && (!JAC || m.term_len > 0)) {
+    kinetics_fix<JAC, SPL, RHS>(m, img, L, s, lane, Yk, T, pr, out, want_h, dst, dld);
+    return true;
   }
+  CellOutT<SPL> o;
+  double yk[SPL];
+#pragma unroll
+  for (int j = 0; j < SPL; ++j) yk[j] = Yk[j];
+  WarpScratch sc = s;
+  kinetics_general<JAC, SPL>(img, L, sc, lane, yk, T, pr.pr, o, pr.cv);
+  out = o;
+  return false;
 }
 
 }  // namespace flint

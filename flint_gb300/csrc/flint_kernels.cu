@@ -167,13 +167,13 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpScratch s;
   if (!GJ) {
-    const int sd = scratch_doubles(nsp, nrpad, JAC);
-    s = carve(reinterpret_cast<double*>(smem + base) + wid * sd, nsp, nrpad, JAC);
+    const int sd = scratch_doubles(L, JAC);
+    s = carve(reinterpret_cast<double*>(smem + base) + wid * sd, L, JAC);
   } else {
     const int sd = scratch_small_doubles(nsp, nrpad);
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
     s = carve2(reinterpret_cast<double*>(smem + base) + wid * sd,
-               JAC ? gscratch + gw * scratch_jac_doubles(nsp, nrpad) : nullptr, nsp, nrpad);
+               JAC ? gscratch + gw * scratch_jac_doubles(L) : nullptr, L);
   }
   const int ns = L.ns, nv = ns + 1;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -187,8 +187,14 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
       if (k < ns) Yk[j] = (layout == 1) ? Yg[(int64_t)k * n + cell] : Yg[cell * ns + k];
     }
     CellOutT<SPL> o;
-    if (FIX) kinetics_cell<JAC, SPL, RHS>(x, img, L, s, lane, Yk, T, FixPress::of<JAC || RHS>(x, p, cv != 0), o, cpo != nullptr || ho != nullptr);
-    else warp_kinetics<JAC, SPL>(m, s, lane, Yk, T, p, o, cv != 0);
+    // Fortran (nv, nv, N): column c of this cell is contiguous; lanes = rows.
+    double* dst = JAC ? jac + cell * (int64_t)nv * nv : nullptr;
+    bool stored = false;
+    if (FIX)
+      stored = kinetics_cell<JAC, SPL, RHS>(x, img, L, s, lane, Yk, T, FixPress::of<JAC || RHS>(x, p, cv != 0), o,
+                                            cpo != nullptr || ho != nullptr, dst, nv);
+    else
+      warp_kinetics<JAC, SPL>(m, s, lane, Yk, T, p, o, cv != 0);
 #pragma unroll
     for (int j = 0; j < SPL; ++j) {
       const int k = lane + 32 * j;
@@ -203,9 +209,7 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
       if (cpo) cpo[cell] = o.cp_mass;
       if (ho) ho[cell] = o.h_mass;
     }
-    if (JAC && jac) {
-      // Fortran (nv, nv, N): column c of this cell is contiguous; lanes = rows.
-      double* dst = jac + cell * (int64_t)nv * nv;
+    if (JAC && !stored) {
 #pragma unroll
       for (int j = 0; j < SPL; ++j) {
         const int r = lane + 32 * j;
@@ -401,7 +405,7 @@ static size_t image_bytes(const ImageLayout& L, bool jac) {
 static bool warp_gj(const ImageLayout& L, bool jac) {
   if (L.nsp > 32) return true;
   if (!jac) return false;
-  return image_bytes(L, true) + (WARP_THREADS / 32) * scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) >
+  return image_bytes(L, true) + (WARP_THREADS / 32) * scratch_doubles(L, true) * sizeof(double) >
          device_smem_optin();
 }
 
@@ -410,7 +414,7 @@ static int warp_block(int threads) { return threads == 64 || threads == 128 ? th
 size_t warp_smem(const ImageLayout& L, bool jac, int threads) {
   const int wpb = warp_block(threads) / 32;
   if (warp_gj(L, jac)) return image_bytes(L, jac) + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
-  return image_bytes(L, jac) + wpb * scratch_doubles(L.nsp, L.nrpad, jac) * sizeof(double);
+  return image_bytes(L, jac) + wpb * scratch_doubles(L, jac) * sizeof(double);
 }
 
 int warp_block_candidates(int* out) {
@@ -445,7 +449,7 @@ int64_t warp_jac_scratch_doubles(const ImageLayout& L) {
     if (per_sm < 1) per_sm = 1;
     most = std::max(most, (int64_t)per_sm * device_sms() * (cand[c] / 32));
   }
-  return most * scratch_jac_doubles(L.nsp, L.nrpad);
+  return most * scratch_jac_doubles(L);
 }
 
 template <bool JAC, bool RHS>

@@ -303,14 +303,17 @@ __device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const F
     yk[0] = (lane < ns) ? ya : 0.0;
     if (SPL > 1) yk[SPL - 1] = (lane + 32 < ns) ? yb : 0.0;
     CellOutT<SPL> co;
-    if (FIX) kinetics_cell<true, SPL, false>(x, img, L, s, lane, yk, Tv, fp, co, false);
+    bool stored = false;
+    if (FIX) stored = kinetics_cell<true, SPL, false>(x, img, L, s, lane, yk, Tv, fp, co, false, Jg, JW);
     else warp_kinetics<true, SPL>(m, s, lane, yk, Tv, p, co, cv);
+    if (!stored) {
 #pragma unroll
-    for (int j = 0; j < SPL; ++j) {
-      const int r = lane + 32 * j;
-      if (r < nv) {
-        const double* row = s.Jr + r * ld;
-        for (int c = 0; c < nv; ++c) Jg[c * JW + r] = row[c];
+      for (int j = 0; j < SPL; ++j) {
+        const int r = lane + 32 * j;
+        if (r < nv) {
+          const double* row = s.Jr + r * ld;
+          for (int c = 0; c < nv; ++c) Jg[c * JW + r] = row[c];
+        }
       }
     }
     __syncwarp();   // the rows are read: the columns of M take their place
@@ -339,10 +342,10 @@ __device__ __forceinline__ void refresh_newton_matrix(const MechView& m, const F
 static int spl_of(const ImageLayout& L) { return L.nsp / 32; }
 
 // The image a block stages.
-static size_t staged_bytes(const ImageLayout& L) { return L.fix ? L.fix_bytes : L.bytes; }
+static size_t staged_bytes(const ImageLayout& L) { return L.fix ? L.fix_bytes_rate : L.bytes; }
 
 static size_t reactor_smem_spl1(const ImageLayout& L) {
-  return staged_bytes(L) + (REACTOR_THREADS / 32) * (scratch_doubles(L.nsp, L.nrpad, true) * sizeof(double) + 64 * sizeof(int));
+  return staged_bytes(L) + (REACTOR_THREADS / 32) * (scratch_doubles(L, true) * sizeof(double) + 64 * sizeof(int));
 }
 
 // layout: REACTOR_LAYOUT_AUTO picks shared memory whenever the block fits;
@@ -362,7 +365,7 @@ static int reactor_threads(int layout) { return layout == REACTOR_LAYOUT_GLOBAL4
 // Jacobian (32*SPL)^2, and in GJ layout the Jacobian work area too.
 static int64_t reactor_slot_doubles_of(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
   const int spl = spl_of(L);
-  return (int64_t)(32 * spl) * (32 * spl) + (reactor_gj(L, layout) ? scratch_jac_doubles(L.nsp, L.nrpad) : 0);
+  return (int64_t)(32 * spl) * (32 * spl) + (reactor_gj(L, layout) ? scratch_jac_doubles(L) : 0);
 }
 
 template <int SPL, bool GJ, int MINB, bool FIX>
@@ -374,12 +377,16 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
           const unsigned long long* __restrict__ n_dev) {
   extern __shared__ __align__(16) uint8_t smem[];
   if (n_dev) n = min(n, (int64_t)*n_dev);   // cell count produced on the device
-  const int base = FIX ? L.fix_bytes : L.bytes;
+  const int base = FIX ? L.fix_bytes_rate : L.bytes;
   stage_image(smem, FIX ? img + L.o_fix : img, base);
   MechView m;
   FixView x;
-  if (FIX) x.bind(L, smem);
-  else m.bind(L, smem);
+  if (FIX) {
+    x.bind(L, smem);
+    x.bind_terms(L, img + L.o_fix);   // the Jacobian is rare: its term lists stay in global memory
+  } else {
+    m.bind(L, smem);
+  }
   const double* invmw = FIX ? x.invmw : m.invmw;
   const int nsp = L.nsp, nrpad = L.nrpad;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -389,14 +396,14 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
   WarpScratch s;
   int* pivs;
   if (!GJ) {
-    const int sd = scratch_doubles(nsp, nrpad, true);
+    const int sd = scratch_doubles(L, true);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
-    s = carve(wbase, nsp, nrpad, true);
+    s = carve(wbase, L, true);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
   } else {
     const int sd = scratch_small_doubles(nsp, nrpad);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
-    s = carve2(wbase, Jg + JW * JW, nsp, nrpad);
+    s = carve2(wbase, Jg + JW * JW, L);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64 * SPL;
   }
   const int ns = L.ns, nv = ns + 1;
