@@ -103,6 +103,9 @@ static const MathTables& math_tables() {
   return t;
 }
 
+const uint64_t* fix_exp2_table() { return math_tables().exp2_fix; }
+const uint64_t* fix_log2_table() { return math_tables().log2_fix; }
+
 // Class of an elementary reaction for the thread-per-cell kernel: 0 reversible
 // and 1 irreversible with one or two factors on each side, integer coefficients
 // equal to the orders, A > 0 and no species on both sides; 2 anything else.

@@ -222,6 +222,29 @@ __host__ __device__ __forceinline__ int64_t fix_enthalpy(const uint64_t* __restr
   return fix_poly5(c, S, t) + (int64_t)(mulhi_u(c[5 * S], f.v) - (f.v >> 1));
 }
 
+// a / b, correctly rounded, from y = the correctly rounded 1/b: q = a y is within
+// one unit of the quotient, its remainder a - b q is exact, and q + r y rounds to
+// the quotient (P. W. Markstein, IBM J. Res. Dev. 34(1), 1990).  Needs
+// exponents away from the ends; others take the division.
+__host__ __device__ inline double div_by(double a, double b, double y) {
+#ifdef __CUDA_ARCH__
+  const uint32_t ea = (uint32_t)__double2hiint(a) & 0x7ff00000u, eb = (uint32_t)__double2hiint(b) & 0x7ff00000u;
+#else
+  const uint32_t ea = (uint32_t)(d_bits(a) >> 32) & 0x7ff00000u, eb = (uint32_t)(d_bits(b) >> 32) & 0x7ff00000u;
+#endif
+  // exponents between -400 and 400, or a = 0
+  const bool mid = (ea - 0x26f00000u < 0x32000000u || ((uint64_t)d_bits(a) << 1) == 0) && eb - 0x26f00000u < 0x32000000u;
+#ifdef __CUDA_ARCH__
+  if (!mid) return __ddiv_rn(a, b);
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+#else
+  if (!mid) return a / b;
+  const double q = a * y;
+  return __builtin_fma(__builtin_fma(-b, q, a), y, q);
+#endif
+}
+
 // 1/x in FP64: the SM's reciprocal approximation (about 2^-20) and one
 // third-order (Chebyshev) step r (1 + e + e^2), e = 1 - x r; relative error below
 // 2^-52.  Zero, subnormal, huge, inf and NaN take the division.

@@ -102,12 +102,16 @@ __device__ __forceinline__ double floor_tiny(double x) {
 
 __device__ __forceinline__ int64_t mulhi_s(int64_t a, int64_t b) { return __mul64hi(a, b); }
 
-__device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_t* lt, const uint64_t* et) {
-  const int64_t lg = log2_q52(floor_tiny(Fc), lt);
-  const int64_t xx = log2_q52(floor_tiny(Pr), lt) - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
+// The blend from log2 Fc and log2 Pr (Q52).
+__device__ __forceinline__ double troe_blend_raw(int64_t lg, int64_t lgP, const uint64_t* et) {
+  const int64_t xx = lgP - TROE_C40 - (mulhi_s(lg, TROE_M67) << 1);
   const int64_t den = TROE_C75 - (mulhi_s(lg, TROE_M127) << 2) - (mulhi_s(xx, TROE_M14) << 1);
   const double dx = fix2d(xx, 52), dd = fix2d(den, 52), d2 = dd * dd;
   return exp2_q52(d2fix52(fix2d(lg, 52) * (d2 * recip(fma(dx, dx, d2)))), et);
+}
+
+__device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_t* lt, const uint64_t* et) {
+  return troe_blend_raw(log2_q52(floor_tiny(Fc), lt), log2_q52(floor_tiny(Pr), lt), et);
 }
 
 // What a cell's fixed pressure (cv: density) contributes: the reactor forms it

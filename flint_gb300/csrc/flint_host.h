@@ -30,6 +30,9 @@ struct flint_ir_s {
 namespace flint {
 
 void count_launch();
+// The constant tables of flint_fix.cuh (FIX_EXP2 and 2 FIX_LOG2 words).
+const uint64_t* fix_exp2_table();
+const uint64_t* fix_log2_table();
 cudaError_t probe_fp64(double* tflops);
 cudaError_t launch_exp_selftest(const uint8_t* img, const ImageLayout& L, int64_t n, const double* x, double* y,
                                 cudaStream_t st);

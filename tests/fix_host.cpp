@@ -48,6 +48,13 @@ int main() {
     const double y = (U(g) - 0.5) * 4000.0 * std::exp2(-40.0 * U(g));
     d2f = fmaxl(d2f, fabsl(ldexpl((ld)d2fix52(y), -52) - (ld)y));
   }
+  // div_by: the correctly rounded quotient, for divisors like molar masses and any others
+  for (int i = 0; i < 4000000; ++i) {
+    const double b = i % 2 ? 1.0 + 300.0 * U(g) : std::ldexp(1.0 + U(g), (int)(g() % 900) - 450);
+    const double a = (i % 3 ? 1.0 + U(g) : U(g)) * std::ldexp(1.0, (int)(g() % 900) - 450) * (i % 5 ? 1.0 : -1.0);
+    exact &= div_by(a, b, 1.0 / b) == a / b;
+  }
+  exact &= div_by(0.0, 3.0, 1.0 / 3.0) == 0.0 && std::isinf(div_by(INFINITY, 3.0, 1.0 / 3.0)) && std::isnan(div_by(NAN, 3.0, 1.0 / 3.0));
   // ends of the ranges
   exact &= fix2d(0, 52) == 0.0 && d2fix52(0.0) == 0 && d2fix52(1e300) == (2047ll << 52) && d2fix52(-1e300) == -(2047ll << 52);
   exact &= exp2_q52(-(1500ll << 52), et.data()) == 0.0 && std::isinf(exp2_q52(1100ll << 52, et.data()));
