@@ -28,7 +28,6 @@
 #include <string>
 #include <vector>
 #include <algorithm>
-#include <cuda_bf16.h>
 
 #include "flint_host.h"
 #include "flint_mlp.h"
@@ -45,7 +44,6 @@ struct Net {
   int dims[MAXL + 1] = {0};
   int64_t off_w[MAXL] = {0}, off_b[MAXL] = {0}, P = 0;
   float *w = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;
-  __nv_bfloat16* wb = nullptr;
   int64_t step = 0;
   // the fused tcgen05 inference forward (flint_umma.cu): packed BF16 hi/lo
   // weights, refreshed from w whenever w changed
@@ -71,11 +69,12 @@ struct Surrogate {
   int ne;
   // workspaces
   int64_t cap = 0;          // rows of the inference workspaces (A, yhat, yout2, xf)
-  int64_t cap_tr = 0;       // rows of the training-only workspaces (Z, dz0, dz1)
+  int64_t cap_tr = 0;       // rows of the training-only workspaces (Z, which back-propagation turns into the layers'
+                            // gradients, and dz0, the output's)
   int64_t cap_fb = 0;       // cells of the fallback compaction buffers
   float* Z[MAXL] = {nullptr};
   float* A[MAXL] = {nullptr};   // FP32 activations (the forward GEMMs split them into BF16 hi + lo)
-  float *dz0 = nullptr, *dz1 = nullptr, *yhat = nullptr, *xf = nullptr, *yout2 = nullptr;
+  float *dz0 = nullptr, *yhat = nullptr, *xf = nullptr, *yout2 = nullptr;
   double* loss = nullptr;
   // fallback compaction
   int64_t* rej_idx = nullptr;
@@ -431,10 +430,8 @@ static cudaError_t net_forward(Surrogate* s, Net& nt, int64_t n, const float* X,
   for (int l = 0; l < nt.nl && !e; ++l) {
     GemmArgs g{};
     g.M = (int)n; g.N = nt.dims[l + 1]; g.K = nt.dims[l];
-    if (l == 0) { g.A = X; g.a_bf16 = 0; } else { g.A = s->A[l - 1]; g.a_bf16 = 0; }
-    g.sa_m = g.K; g.sa_k = 1;
-    g.B = nt.w + nt.off_w[l]; g.b_bf16 = 0; g.sb_k = 1; g.sb_n = g.K;
-    g.split = 1;
+    g.A = l == 0 ? X : s->A[l - 1]; g.lda = g.K;
+    g.B = nt.w + nt.off_w[l]; g.ldb = g.K;
     g.bias = nt.w + nt.off_b[l];
     if (l < nt.nl - 1) {
       g.epi = EPI_BIAS_GELU;
@@ -444,7 +441,7 @@ static cudaError_t net_forward(Surrogate* s, Net& nt, int64_t n, const float* X,
       g.epi = EPI_BIAS;
       g.C = out; g.ldc = g.N;
     }
-    e = launch_gemm(g, st);
+    e = launch_gemm(GEMM_FORWARD, g, st);
   }
   return e;
 }
@@ -467,13 +464,11 @@ static int alloc_ws(Surrogate* s, int64_t cap, bool train) {
   }
   if (train && cap > s->cap_tr) {
     for (int l = 0; l < MAXL; ++l) { fr(s->Z[l]); s->Z[l] = nullptr; }
-    fr(s->dz0); fr(s->dz1);
-    s->dz0 = s->dz1 = nullptr;
+    fr(s->dz0);
+    s->dz0 = nullptr;
     s->cap_tr = 0;
-    const int W = std::max(s->H, std::max(s->n_in, s->n_out));
     for (int l = 0; l < nh && !e; ++l) e = cudaMalloc(&s->Z[l], cap * s->H * sizeof(float));
-    if (!e) e = cudaMalloc(&s->dz0, cap * W * sizeof(float));
-    if (!e) e = cudaMalloc(&s->dz1, cap * W * sizeof(float));
+    if (!e) e = cudaMalloc(&s->dz0, cap * s->n_out * sizeof(float));
     if (e) return FLINT_ERR_NOMEM;
     s->cap_tr = cap;
   }
@@ -500,7 +495,7 @@ static int alloc_fb(Surrogate* s, int64_t n) {
 }
 
 static void net_free(Net& nt) {
-  cudaFree(nt.w); cudaFree(nt.g); cudaFree(nt.m1); cudaFree(nt.m2); cudaFree(nt.wb);
+  cudaFree(nt.w); cudaFree(nt.g); cudaFree(nt.m1); cudaFree(nt.m2);
   cudaFree(nt.upk); cudaFree(nt.ubias); cudaFree(nt.uoff);
   nt = Net();
 }
@@ -510,7 +505,7 @@ void surrogate_free(Surrogate* s) {
   for (int i = 0; i < 2; ++i) net_free(s->net[i]);
   auto fr = [](void* p) { if (p) cudaFree(p); };
   for (int l = 0; l < MAXL; ++l) { fr(s->Z[l]); fr(s->A[l]); }
-  fr(s->dz0); fr(s->dz1); fr(s->yhat); fr(s->xf); fr(s->yout2); fr(s->rej_idx); fr(s->rej_count);
+  fr(s->dz0); fr(s->yhat); fr(s->xf); fr(s->yout2); fr(s->rej_idx); fr(s->rej_count);
   fr(s->cT); fr(s->cp); fr(s->cY); fr(s->cdt); fr(s->cst); fr(s->cns); fr(s->loss);
   fr(s->xmean); fr(s->xstd); fr(s->ymean); fr(s->ystd); fr(s->G0); fr(s->Bm); fr(s->uerr);
   delete s;
@@ -530,11 +525,9 @@ static int net_init(Net& nt, int nl, const int* dims, const float* w0) {
   if (!e) e = cudaMalloc(&nt.g, off * sizeof(float));
   if (!e) e = cudaMalloc(&nt.m1, off * sizeof(float));
   if (!e) e = cudaMalloc(&nt.m2, off * sizeof(float));
-  if (!e) e = cudaMalloc(&nt.wb, off * sizeof(__nv_bfloat16));
   if (!e) e = cudaMemcpy(nt.w, w0, off * sizeof(float), cudaMemcpyHostToDevice);
   if (!e) e = cudaMemset(nt.m1, 0, off * sizeof(float));
   if (!e) e = cudaMemset(nt.m2, 0, off * sizeof(float));
-  if (!e) e = launch_to_bf16(nt.w, nt.wb, off, nullptr);
   nt.ufits = umma_fits(nl, dims);
   if (!e && nt.ufits) {
     const int64_t bytes = umma_describe(nl, dims, &nt.u);
@@ -642,33 +635,28 @@ int surrogate_train_step(Surrogate* s, int net, int64_t n, const float* X, const
   if (net_forward(s, nt, n, X, s->yhat, true, st)) return FLINT_ERR_CUDA;
   if (cudaMemsetAsync(s->loss, 0, 8, st)) return FLINT_ERR_CUDA;
   const int nl = nt.nl;
-  float* dz = s->dz0;
-  float* dzn = s->dz1;
-  if (launch_mse(s->yhat, Yt, n * s->n_out, 1.0f / (float)(n * s->n_out), dz, s->loss, st)) return FLINT_ERR_CUDA;
-  for (int l = nl - 1; l >= 0; --l) {
-    const int N = nt.dims[l + 1], K = nt.dims[l];
-    GemmArgs g{};
-    g.M = N; g.N = K; g.K = (int)n;
-    g.A = dz; g.a_bf16 = 0; g.sa_m = 1; g.sa_k = N;
-    if (l == 0) { g.B = X; g.b_bf16 = 0; } else { g.B = s->A[l - 1]; g.b_bf16 = 0; }
-    g.sb_k = K; g.sb_n = 1;
-    g.C = nt.g + nt.off_w[l]; g.ldc = K; g.epi = EPI_STORE;
-    if (launch_gemm(g, st)) return FLINT_ERR_CUDA;
-    if (launch_colsum(dz, (int)n, N, N, nt.g + nt.off_b[l], 0, st)) return FLINT_ERR_CUDA;
-    if (l > 0) {
-      GemmArgs h{};
-      h.M = (int)n; h.N = K; h.K = N;
-      h.A = dz; h.a_bf16 = 0; h.sa_m = N; h.sa_k = 1;
-      h.B = nt.wb + nt.off_w[l]; h.b_bf16 = 1; h.sb_k = K; h.sb_n = 1;
-      h.C = dzn; h.ldc = K; h.epi = EPI_GELU_BWD; h.Zprev = s->Z[l - 1]; h.ldz = K;
-      if (launch_gemm(h, st)) return FLINT_ERR_CUDA;
-      std::swap(dz, dzn);
-    }
+  if (launch_mse(s->yhat, Yt, n * s->n_out, 1.0f / (float)(n * s->n_out), s->dz0, s->loss, st)) return FLINT_ERR_CUDA;
+  // the gradient by each layer's pre-activation takes its place
+  auto dz = [&](int l) { return l == nl - 1 ? s->dz0 : s->Z[l]; };
+  for (int l = nl - 1; l > 0; --l) {
+    GemmArgs h{};
+    h.M = (int)n; h.N = nt.dims[l]; h.K = nt.dims[l + 1];
+    h.A = dz(l); h.lda = h.K;
+    h.B = nt.w + nt.off_w[l]; h.ldb = h.N;
+    h.C = s->Z[l - 1]; h.ldc = h.N; h.epi = EPI_GELU_BWD; h.Zprev = s->Z[l - 1]; h.ldz = h.N;
+    if (launch_gemm(GEMM_INPUT, h, st)) return FLINT_ERR_CUDA;
   }
+  static_assert(MAXL <= GRAD_BATCH, "one launch holds every layer");
+  WeightGrad g[MAXL];
+  for (int l = 0; l < nl; ++l)
+    g[l] = WeightGrad{nt.dims[l + 1], nt.dims[l], (int)n, dz(l), l == 0 ? X : s->A[l - 1], nt.g + nt.off_w[l],
+                      nt.g + nt.off_b[l]};
+  if (launch_weight_grads(g, nl, st)) return FLINT_ERR_CUDA;
   nt.step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float bc1 = 1.f - powf(b1, (float)nt.step), bc2 = 1.f - powf(b2, (float)nt.step);
-  if (launch_adam(nt.w, nt.g, nt.m1, nt.m2, nt.wb, nt.P, lr, b1, b2, 1e-8f, bc1, bc2, 0.f, st)) return FLINT_ERR_CUDA;
+  if (launch_adam(nt.w, nt.g, nt.m1, nt.m2, nt.P, lr, b1, b2, 1e-8f, bc1, bc2, 0.f, st))
+    return FLINT_ERR_CUDA;
   nt.udirty = true;
   if (loss_out) {
     if (cudaMemcpyAsync(loss_out, s->loss, 8, cudaMemcpyDeviceToHost, st)) return FLINT_ERR_CUDA;
@@ -691,7 +679,6 @@ int surrogate_state(Surrogate* s, int net, float* host, int64_t* step, int get) 
     e = cudaMemcpy(nt.w, host, P * 4, cudaMemcpyHostToDevice);
     if (!e) e = cudaMemcpy(nt.m1, host + P, P * 4, cudaMemcpyHostToDevice);
     if (!e) e = cudaMemcpy(nt.m2, host + 2 * P, P * 4, cudaMemcpyHostToDevice);
-    if (!e) e = launch_to_bf16(nt.w, nt.wb, P, nullptr);
     if (!e) e = cudaDeviceSynchronize();
     nt.udirty = true;
     if (step) nt.step = *step;
