@@ -134,14 +134,15 @@ static int plain_class(const flint_mech_desc* d, int r) {
 // Append the fixed-point image (ImageLayout::fix and the f_ offsets) when the
 // mechanism fits it: NASA-7 thermo, reactions whose rate is a product of at most
 // three concentrations a side (with the reverse Gibbs sum over the same
-// factors), non-zero A, and every coefficient and exponent within its format
+// factors; irreversible reactions of up to 16 species may have any orders, which
+// only the small-mechanism kernel takes: sfix without fix), non-zero A, and every coefficient and exponent within its format
 // from fix_Tlo <= 600 K up to fix_Thi >= 3000 K.  Coefficients are formed in long double.
 static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, ImageLayout& L,
                      std::vector<uint8_t>& img) {
   typedef long double ld;
   const ld LOG2E = 1.0L / logl(2.0L);
   const int ns = L.ns, nr = L.nr, S = L.nsp, P = L.nrpad, dummy = fix_dummy(S);
-  L.fix = 0;
+  L.fix = L.sfix = 0;
   L.dq_rows = 8;
   if (d->nasa9 || nr < 1 || ns > dummy || L.nfall > 16) return;
   bool ok = true;
@@ -208,6 +209,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   std::vector<uint64_t> ix(P, 0);
   std::vector<double> tr(5 * 16, 0.0);
   std::vector<std::vector<int>> lists_r(nr), lists_p(nr);
+  std::vector<uint64_t> ordq(3 * P, 0);   // orders of the reactions in power form, Q60
+  bool powers = false, any_rev = false;
   bool w3 = false;
   int tb = 0;
   for (int rr = 0; rr < nr && ok; ++rr) {
@@ -219,7 +222,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
       const int i = d->rsp[3 * r + s], j = d->psp[3 * r + s];
       if (i >= 0) {
         const double o = d->rord[3 * r + s], nu = d->rnu[3 * r + s];
-        if (!(o == 0.0 || o == 1.0 || o == 2.0 || o == 3.0) || (d->reversible[r] && o != nu)) { ok = false; break; }
+        if (d->reversible[r] && (o != nu || !(o == 0.0 || o == 1.0 || o == 2.0 || o == 3.0))) { ok = false; break; }
         for (int u = 0; u < (int)o; ++u) rs.push_back(i);
       }
       if (j >= 0 && d->reversible[r]) {
@@ -227,6 +230,26 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
         if (!(nu == 0.0 || nu == 1.0 || nu == 2.0 || nu == 3.0)) { ok = false; break; }
         for (int u = 0; u < (int)nu; ++u) ps.push_back(j);
       }
+    }
+    any_rev |= d->reversible[r] != 0;
+    // an irreversible reaction with other orders: the factors' logarithms times
+    // their orders (thread-per-cell kernel of small mechanisms only)
+    bool power = false;
+    for (int s = 0; s < 3; ++s) {
+      const double o = d->rsp[3 * r + s] >= 0 ? d->rord[3 * r + s] : 0.0;
+      power |= !(o == 0.0 || o == 1.0 || o == 2.0 || o == 3.0);
+      if (!(o < 16.0)) ok = false;
+    }
+    if (!d->reversible[r] && (power || rs.size() > 3)) {
+      rs.clear();
+      for (int s = 0; s < 3; ++s)
+        if (d->rsp[3 * r + s] >= 0 && d->rord[3 * r + s] != 0.0) {
+          ordq[(int)rs.size() * P + rr] = (uint64_t)llrintl(ldexpl((ld)d->rord[3 * r + s], 60));
+          rs.push_back(d->rsp[3 * r + s]);
+        }
+      powers = power = true;
+    } else {
+      power = false;
     }
     if (rs.size() > 3 || ps.size() > 3) ok = false;
     if (!ok) break;
@@ -239,7 +262,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
       w |= (uint64_t)(s < (int)ps.size() ? ps[s] : dummy) << (18 + 6 * s);
     }
     w |= (uint64_t)(dn + 8) << 36 | (uint64_t)t << 40 | (uint64_t)(d->reversible[r] ? 1 : 0) << 42 |
-         (uint64_t)(A < 0.0 ? 1 : 0) << 43;
+         (uint64_t)(A < 0.0 ? 1 : 0) << 43 | (uint64_t)(power ? 1 : 0) << 46;
     if (t) { w |= (uint64_t)tb << 48; ++tb; }
     ix[rr] = w;
     // + 1 unit of 2^-52: about the mean of what the two floored products lose
@@ -310,7 +333,10 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
     Tlo = T;
   }
   if (!(Tlo <= 600.0 && Thi >= 3000.0)) return;
-  L.fix = 1;
+  L.fix = powers ? 0 : 1;
+  L.sfix = ns <= 16 ? 1 : 0;
+  if (!L.fix && !L.sfix) return;
+  L.fix_rev = any_rev ? 1 : 0;
   L.fix_w3 = w3 ? 1 : 0;
   L.fix_Tlo = std::max(Tlo, 129.0);
   L.fix_Thi = Thi;
@@ -373,7 +399,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
         while (i < segv.size() && segv[i] != std::fabs(nu[e])) ++i;
         if (i == segv.size()) segv.push_back(std::fabs(nu[e]));
         const bool last = e + 1 == cs[k + 1] || (e + 1) % len == 0;
-        if (segv.size() > 127 || lr[e] > 0xffff || np > 127) { L.fix = 0; return; }
+        if (segv.size() > 127 || lr[e] > 0xffff || np > 127) { L.fix = L.sfix = 0; return; }
         seg[(size_t)(e % len) * 32 + e / len] = (uint32_t)lr[e] | (nu[e] < 0.0 ? 1u << 16 : 0u) | (uint32_t)i << 17 |
                                                  (uint32_t)np << 24 | (last ? 1u << 31 : 0u);
         np += last;
@@ -388,7 +414,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   // longest first to the lane with the least; column ns holds the third-body terms
   // common to every column, row ns the derivative by T
   const int nslot = w3 ? 3 : 2, rows = S + 1;
-  L.dq_rows = 2 * nslot + 2;
+  L.dq_rows = powers ? 8 : 2 * nslot + 2;
   std::vector<uint32_t> term;
   std::vector<uint16_t> target;
   std::vector<double> coef{0.0};
@@ -404,7 +430,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
     const int* tbs = reinterpret_cast<const int*>(img.data() + L.o_tbs);
     const double* tbv = reinterpret_cast<const double*>(img.data() + L.o_tbv);
     const double* tbd = reinterpret_cast<const double*>(img.data() + L.o_tbd);
-    for (int k = 0; k < ns; ++k)
+    for (int k = 0; k < ns && !powers; ++k)
       for (int e = cs[k]; e < cs[k + 1]; ++e) {
         const int rr = lr[e];
         for (int s = 0; s < (int)lists_r[rr].size(); ++s) run[k * rows + lists_r[rr][s]].push_back({s * P + rr, nu[e]});
@@ -463,6 +489,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   L.f_ra = sec(8 * 16); L.f_rb = sec(8 * 16); L.f_re = sec(8 * 16); L.f_tr = sec(8 * 5 * 16);
   L.f_tbd = sec(8 * L.ntb); L.f_tbp = sec(4 * (L.ntb + 1)); L.f_tbs = sec(4 * ntbl); L.f_tbv = sec(8 * ntbl);
   L.f_cx = sec(8 * P); L.f_cy = sec(8 * P);
+  L.f_ord = sec(8 * 3 * P);
   L.f_rs = sec(4 * (nr + 1)); L.f_rw = sec(4 * nlist); L.f_rv = sec(8 * (int)std::max<size_t>(rv.size(), 1));
   L.f_exp = sec(8 * FIX_EXP2); L.f_log = sec(8 * 2 * FIX_LOG2);
   L.fix_bytes_cell = off;   // the thread-per-cell kernel needs no species lists
@@ -487,6 +514,7 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   put(L.f_coef, coef.data(), 8 * coef.size());
   put(L.f_seg, seg.data(), 4 * seg.size()); put(L.f_segv, segv.data(), 8 * segv.size());
   put(L.f_piece, piece.data(), 4 * (S + 1));
+  put(L.f_ord, ordq.data(), 8 * 3 * P);
   put(L.f_cx, cx.data(), 8 * P); put(L.f_cy, cy.data(), 8 * P);
   int* rs = reinterpret_cast<int*>(F + L.f_rs);
   int* rw = reinterpret_cast<int*>(F + L.f_rw);

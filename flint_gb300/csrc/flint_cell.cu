@@ -38,22 +38,6 @@ __device__ __forceinline__ double opaque(double x) {
   return x;
 }
 
-// Effective rate coefficient of a falloff reaction (i-th, reaction word w) from
-// its high-pressure limit's exponent xinf (Q52).
-__device__ __forceinline__ double cell_falloff(const FixView& m, int i, int type, int64_t xinf, double M, const FixT& f,
-                                               double T, double Tinv) {
-  const double kinf = exp2_q52(xinf, m.et);
-  const double kratio = exp2_q52(fix_arrhenius(m.ra[i], m.rb[i], m.re[i], f), m.et);
-  const double Pr = kratio * M;
-  const double k = kinf * (Pr * recip(1.0 + Pr));
-  if (type != 3) return k;
-  const double z2 = m.tr[64 + i];
-  double Fc = z2 != 0.0 ? exp2_q52(-d2fix52(z2 * Tinv), m.et) : 0.0;
-  Fc = fma(m.tr[16 + i], exp2_q52(-d2fix52(m.tr[48 + i] * T), m.et), Fc);
-  Fc = fma(m.tr[i], exp2_q52(-d2fix52(m.tr[32 + i] * T), m.et), Fc);
-  return k * troe_blend(Fc, Pr, m.lt, m.et);
-}
-
 // One cell of the batch on the FP64 path, by the whole warp; scratch: the warp's
 // columns.
 template <bool RHS, int SPL>

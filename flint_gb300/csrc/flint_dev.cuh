@@ -75,6 +75,9 @@ struct ImageLayout {
   int fix, o_fix, fix_bytes;
   int fix_bytes_cell, fix_bytes_rate;   // the leading parts that the thread-per-cell kernel and the warp kernels
                                         // without a Jacobian stage
+  int sfix;                      // the small-mechanism kernel (<= 16 species) may use the image
+  int fix_rev;                   // some reaction is reversible
+  int f_ord;                     // uint64 [3][nrpad]: orders (Q60) of the reactions in power form
   int fix_w3;                    // some reaction has a third factor on a side
   double fix_Tlo, fix_Thi;       // cells with T in [fix_Tlo, fix_Thi) take the fixed-point path
   int64_t fix_lC;                // log2(p_ref / r_thermo) - 7, Q52

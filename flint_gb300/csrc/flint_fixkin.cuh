@@ -14,9 +14,11 @@ namespace flint {
 // Index word of a reaction: bits 0-17 three reactant factors, 18-35 three
 // product factors (6 bits each, `dummy` where absent), 36-39 dn + 8, 40-41
 // type, 42 reversible, 43 A < 0, 44 and 45 both reactant and both product factors
-// of a plain reaction are one species, 48-55 third-body row.
+// of a plain reaction are one species, 46 power form (the factors' orders are
+// f_ord), 48-55 third-body row.
 __device__ __forceinline__ int fix_type(uint64_t w) { return (int)(w >> 40) & 3; }
 __device__ __forceinline__ bool fix_rev(uint64_t w) { return (w >> 42) & 1; }
+__device__ __forceinline__ bool fix_power(uint64_t w) { return (w >> 46) & 1; }
 __device__ __forceinline__ bool fix_twice_r(uint64_t w) { return (w >> 44) & 1; }
 __device__ __forceinline__ bool fix_twice_p(uint64_t w) { return (w >> 45) & 1; }
 __device__ __forceinline__ int fix_tbrow(uint64_t w) { return (int)(w >> 48) & 0xff; }
@@ -29,7 +31,7 @@ struct FixView {
   int64_t lC;
   const double *mw, *invmw, *tr, *tbd, *tbv;
   const int64_t *tmid, *a, *ra;
-  const uint64_t *g, *h, *c, *b, *e, *rb, *re, *et, *lt, *ix, *cx, *cy;
+  const uint64_t *g, *h, *c, *b, *e, *rb, *re, *et, *lt, *ix, *cx, *cy, *ord;
   const int *tbp, *tbs, *rs, *rw, *piece;
   const double *rv, *segv, *coef;
   const uint32_t *seg, *term;
@@ -45,7 +47,7 @@ struct FixView {
     mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv);
     tmid = I(L.f_tmid); a = I(L.f_a); ra = I(L.f_ra);
     g = U(L.f_g); h = U(L.f_h); c = U(L.f_c); b = U(L.f_b); e = U(L.f_e);
-    rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); cx = U(L.f_cx); cy = U(L.f_cy);
+    rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); ord = U(L.f_ord); cx = U(L.f_cx); cy = U(L.f_cy);
     tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
     rs = (const int*)(base + L.f_rs); rw = (const int*)(base + L.f_rw); rv = D(L.f_rv);
     seg = (const uint32_t*)(base + L.f_seg); segv = D(L.f_segv); piece = (const int*)(base + L.f_piece);
@@ -112,6 +114,22 @@ __device__ __forceinline__ double troe_blend_raw(int64_t lg, int64_t lgP, const 
 
 __device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_t* lt, const uint64_t* et) {
   return troe_blend_raw(log2_q52(floor_tiny(Fc), lt), log2_q52(floor_tiny(Pr), lt), et);
+}
+
+// Effective rate coefficient of a falloff reaction (i-th, reaction word w) from
+// its high-pressure limit's exponent xinf (Q52).
+__device__ __forceinline__ double cell_falloff(const FixView& m, int i, int type, int64_t xinf, double M, const FixT& f,
+                                               double T, double Tinv) {
+  const double kinf = exp2_q52(xinf, m.et);
+  const double kratio = exp2_q52(fix_arrhenius(m.ra[i], m.rb[i], m.re[i], f), m.et);
+  const double Pr = kratio * M;
+  const double k = kinf * (Pr * recip(1.0 + Pr));
+  if (type != 3) return k;
+  const double z2 = m.tr[64 + i];
+  double Fc = z2 != 0.0 ? exp2_q52(-d2fix52(z2 * Tinv), m.et) : 0.0;
+  Fc = fma(m.tr[16 + i], exp2_q52(-d2fix52(m.tr[48 + i] * T), m.et), Fc);
+  Fc = fma(m.tr[i], exp2_q52(-d2fix52(m.tr[32 + i] * T), m.et), Fc);
+  return k * troe_blend(Fc, Pr, m.lt, m.et);
 }
 
 // What a cell's fixed pressure (cv: density) contributes: the reactor forms it

@@ -25,6 +25,114 @@ constexpr int SMALL_THREADS = 128;
 constexpr int WARP_THREADS = 256;
 
 // ---------------------------------------------------------------- small
+// One cell of a small mechanism on the FP64 path, by one thread.  cs, gs, ws:
+// the thread's columns of shared memory (stride S).
+__device__ inline void small_cell(const MechView& m, int64_t i, int64_t n, int layout, const double* __restrict__ Tg,
+                                  const double* __restrict__ pg, const double* __restrict__ Yg,
+                                  double* __restrict__ wdot, double* __restrict__ cpo, double* __restrict__ ho,
+                                  int roi_mode, double* roi_io, double* cs, double* gs, double* ws, int S) {
+  const int ns = m.ns, P = m.nrpad;
+#define CS(k) cs[(k) * S]
+#define GS(k) gs[(k) * S]
+#define WS(k) ws[(k) * S]
+  const double T = Tg[i];
+  const double lnT = flog(T, m.logtab), invT = 1.0 / T;
+  double rho;
+  double cpm = 0.0, hm = 0.0, ctot = 0.0;
+  if (roi_mode) {
+    // chemistry_source(roi, T, omegadot): c = max(roi,0)/W (WD.f90:18-21)
+    rho = 0.0;
+    for (int k = 0; k < ns; ++k) {
+      double r = roi_io[i * ns + k];
+      r = r > 0.0 ? r : 0.0;
+      roi_io[i * ns + k] = r;
+      CS(k) = r * m.invmw[k];
+      ctot += CS(k);
+    }
+  } else {
+    double sumYW = 0.0;
+    for (int k = 0; k < ns; ++k) {
+      double y = (layout == 1) ? Yg[(int64_t)k * n + i] : Yg[i * ns + k];
+      CS(k) = y;
+      sumYW += y * m.invmw[k];
+    }
+    rho = pg[i] / (m.r_eos * T * sumYW);
+    for (int k = 0; k < ns; ++k) {
+      double y = CS(k);
+      SpThermo th = nasa7(m, k, T, lnT, invT);
+      cpm += y * th.cpR * m.invmw[k];
+      hm += y * th.hRT * m.invmw[k];
+      CS(k) = rho * y * m.invmw[k];
+      ctot += CS(k);
+      GS(k) = th.hRT - th.sR;
+    }
+  }
+  if (roi_mode) {
+    for (int k = 0; k < ns; ++k) {
+      SpThermo th = nasa7(m, k, T, lnT, invT);
+      GS(k) = th.hRT - th.sR;
+    }
+  }
+  for (int k = 0; k < ns; ++k) WS(k) = 0.0;
+  const double lnC0 = m.lnpref_rth - lnT;
+  for (int r = 0; r < m.nr; ++r) {
+    const uint32_t w = m.code[r];
+    const int type = rx_type(w);
+    double kf = m.A[r] * fexp(m.b[r] * lnT - m.E[r] * invT, m.exptab);
+    double Pf = 1.0, d;
+#pragma unroll
+    for (int sl = 0; sl < MAXSIDE; ++sl) {
+      int sp = m.rsp[sl * P + r];
+      if (sp >= 0) Pf *= powc(CS(sp), rx_ordcode(w, sl), m.rord[sl * P + r], &d, m.exptab, m.logtab);
+    }
+    double rvsf = 0.0;
+    if (rx_rev(w)) {
+      double dG = 0.0, Pr = 1.0;
+#pragma unroll
+      for (int sl = 0; sl < MAXSIDE; ++sl) {
+        int sp = m.psp[sl * P + r];
+        if (sp >= 0) {
+          double nu = m.pnu[sl * P + r];
+          dG += nu * GS(sp);
+          Pr *= powc(CS(sp), (m.pcode[r] >> (4 * sl)) & 0xf, nu, &d, m.exptab, m.logtab);
+        }
+        int sq = m.rsp[sl * P + r];
+        if (sq >= 0) dG -= m.rnu[sl * P + r] * GS(sq);
+      }
+      rvsf = fexp(dG - m.dnu[r] * lnC0, m.exptab) * Pr;
+    }
+    double keff = kf, Mfac = 1.0;
+    if (type != 0) {
+      const int row = rx_tbrow(w);
+      double M = m.tbd[row] * ctot;
+      for (int e = m.tbp[row]; e < m.tbp[row + 1]; ++e) M = fma(m.tbv[e], CS(m.tbs[e]), M);
+      if (type == 1) Mfac = M;
+      else keff = falloff_eval(m, r, type, kf, 0.0, M, T, lnT, invT).keff;
+    }
+    const double q = Mfac * keff * (Pf - rvsf);
+#pragma unroll
+    for (int sl = 0; sl < MAXSIDE; ++sl) {
+      int sp = m.rsp[sl * P + r];
+      if (sp >= 0) WS(sp) -= m.rnu[sl * P + r] * q;
+      int sq = m.psp[sl * P + r];
+      if (sq >= 0) WS(sq) += m.pnu[sl * P + r] * q;
+    }
+  }
+  if (wdot) {
+    for (int k = 0; k < ns; ++k) {
+      double v = m.mw[k] * WS(k);
+      if (roi_mode || layout == 0) wdot[i * ns + k] = v;
+      else wdot[(int64_t)k * n + i] = v;
+    }
+  }
+  (void)rho;
+  if (cpo) cpo[i] = cpm * m.r_thermo;
+  if (ho) ho[i] = hm * m.r_thermo * T;
+#undef CS
+#undef GS
+#undef WS
+}
+
 __global__ void __launch_bounds__(SMALL_THREADS)
 k_wdot_small(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, int layout,
              const double* __restrict__ Tg, const double* __restrict__ pg,
@@ -34,112 +142,173 @@ k_wdot_small(const uint8_t* __restrict__ img, ImageLayout L, int64_t n, int layo
   stage_image(smem, img, L.bytes);
   MechView m;
   m.bind(L, smem);
-  const int ns = m.ns, P = m.nrpad;
-  double* cs = reinterpret_cast<double*>(smem + L.bytes);      // [NSMAX][threads]
-  double* gs = cs + SMALL_NSMAX * SMALL_THREADS;
-  double* ws = gs + SMALL_NSMAX * SMALL_THREADS;
-  const int t = threadIdx.x;
-#define CS(k) cs[(k) * SMALL_THREADS + t]
-#define GS(k) gs[(k) * SMALL_THREADS + t]
-#define WS(k) ws[(k) * SMALL_THREADS + t]
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + t; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  double* cs = reinterpret_cast<double*>(smem + L.bytes) + threadIdx.x;      // [NSMAX][threads]
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    small_cell(m, i, n, layout, Tg, pg, Yg, wdot, cpo, ho, roi_mode, roi_io, cs, cs + SMALL_NSMAX * SMALL_THREADS,
+               cs + 2 * SMALL_NSMAX * SMALL_THREADS, SMALL_THREADS);
+}
+
+__device__ __noinline__ void small_cell_general(const uint8_t* __restrict__ img, const ImageLayout& L, int64_t i,
+                                                int64_t n, int layout, const double* __restrict__ Tg,
+                                                const double* __restrict__ pg, const double* __restrict__ Yg,
+                                                double* __restrict__ wdot, double* __restrict__ cpo,
+                                                double* __restrict__ ho, int roi_mode, double* roi_io, double* cs, int S) {
+  MechView m;
+  m.bind(L, img);
+  small_cell(m, i, n, layout, Tg, pg, Yg, wdot, cpo, ho, roi_mode, roi_io, cs, cs + L.ns * S, cs + 2 * L.ns * S, S);
+}
+
+// The same on the fixed-point image (flint_fix.cuh).  A rate with other than
+// integer orders is one exponential of log2 k + sum of order x log2 c, so the
+// 2-step CH4/air source term leaves about 60 operations of a thread on the FP64
+// pipe (concentrations, sums, cp and h) where it took about 300, half of them
+// logarithms and exponentials.  The mechanism's few words are read through the
+// read-only cache: staging them cost a block more than they are worth.  A thread
+// whose temperature or concentrations leave the formats (2^-64 <= c < 2^63 for a
+// factor in power form, or c = 0) takes the FP64 path.
+__global__ void __launch_bounds__(SMALL_THREADS)
+k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, int layout,
+                 const double* __restrict__ Tg, const double* __restrict__ pg, const double* __restrict__ Yg,
+                 double* __restrict__ wdot, double* __restrict__ cpo, double* __restrict__ ho, int roi_mode,
+                 double* roi_io) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  FixView m;
+  m.bind(L, img + L.o_fix);
+  const int ns = m.ns, nsp = m.nsp, S = blockDim.x, P = m.nrpad, f0 = m.nr - m.nfall;
+  double* cs = reinterpret_cast<double*>(smem) + threadIdx.x;      // c, G, w, log2 c: [ns][threads] each
+  int64_t* gs = reinterpret_cast<int64_t*>(cs + ns * S);
+  double* ws = cs + 2 * ns * S;
+  uint64_t* ls = reinterpret_cast<uint64_t*>(cs + 3 * ns * S);
+  const bool thermo = cpo || ho;
+  for (int64_t i = (int64_t)blockIdx.x * S + threadIdx.x; i < n; i += (int64_t)gridDim.x * S) {
     const double T = Tg[i];
-    const double lnT = flog(T, m.logtab), invT = 1.0 / T;
-    double rho;
+    bool in = m.covers(T);
+    const FixT f = fix_T(in ? T : 1000.0, m.lt);
     double cpm = 0.0, hm = 0.0, ctot = 0.0;
     if (roi_mode) {
       // chemistry_source(roi, T, omegadot): c = max(roi,0)/W (WD.f90:18-21)
-      rho = 0.0;
       for (int k = 0; k < ns; ++k) {
         double r = roi_io[i * ns + k];
         r = r > 0.0 ? r : 0.0;
         roi_io[i * ns + k] = r;
-        CS(k) = r * m.invmw[k];
-        ctot += CS(k);
+        cs[k * S] = r * m.invmw[k];
       }
     } else {
       double sumYW = 0.0;
       for (int k = 0; k < ns; ++k) {
-        double y = (layout == 1) ? Yg[(int64_t)k * n + i] : Yg[i * ns + k];
-        CS(k) = y;
-        sumYW += y * m.invmw[k];
+        const double yw = (layout == 1 ? Yg[(int64_t)k * n + i] : Yg[i * ns + k]) * m.invmw[k];
+        cs[k * S] = yw;
+        sumYW += yw;
       }
-      rho = pg[i] / (m.r_eos * T * sumYW);
+      const double rho = pg[i] * m.inv_r_eos * recip(T * sumYW);
       for (int k = 0; k < ns; ++k) {
-        double y = CS(k);
-        SpThermo th = nasa7(m, k, T, lnT, invT);
-        cpm += y * th.cpR * m.invmw[k];
-        hm += y * th.hRT * m.invmw[k];
-        CS(k) = rho * y * m.invmw[k];
-        ctot += CS(k);
-        GS(k) = th.hRT - th.sR;
-      }
-    }
-    if (roi_mode) {
-      for (int k = 0; k < ns; ++k) {
-        SpThermo th = nasa7(m, k, T, lnT, invT);
-        GS(k) = th.hRT - th.sR;
-      }
-    }
-    for (int k = 0; k < ns; ++k) WS(k) = 0.0;
-    const double lnC0 = m.lnpref_rth - lnT;
-    for (int r = 0; r < m.nr; ++r) {
-      const uint32_t w = m.code[r];
-      const int type = rx_type(w);
-      double kf = m.A[r] * fexp(m.b[r] * lnT - m.E[r] * invT, m.exptab);
-      double Pf = 1.0, d;
-#pragma unroll
-      for (int sl = 0; sl < MAXSIDE; ++sl) {
-        int sp = m.rsp[sl * P + r];
-        if (sp >= 0) Pf *= powc(CS(sp), rx_ordcode(w, sl), m.rord[sl * P + r], &d, m.exptab, m.logtab);
-      }
-      double rvsf = 0.0;
-      if (rx_rev(w)) {
-        double dG = 0.0, Pr = 1.0;
-#pragma unroll
-        for (int sl = 0; sl < MAXSIDE; ++sl) {
-          int sp = m.psp[sl * P + r];
-          if (sp >= 0) {
-            double nu = m.pnu[sl * P + r];
-            dG += nu * GS(sp);
-            Pr *= powc(CS(sp), (m.pcode[r] >> (4 * sl)) & 0xf, nu, &d, m.exptab, m.logtab);
-          }
-          int sq = m.rsp[sl * P + r];
-          if (sq >= 0) dG -= m.rnu[sl * P + r] * GS(sq);
+        const double yw = cs[k * S];
+        if (thermo) {
+          const bool lo = __double_as_longlong(T) <= m.tmid[k];
+          const uint64_t t = lo ? f.t11 : f.t13;
+          cpm = fma(yw, fix2d(fix_poly5(m.c + (lo ? 0 : 5 * nsp) + k, nsp, t), 52), cpm);
+          hm = fma(yw, fix2d(fix_enthalpy(m.h + (lo ? 0 : 6 * nsp) + k, nsp, t, f), 52), hm);
         }
-        rvsf = fexp(dG - m.dnu[r] * lnC0, m.exptab) * Pr;
-      }
-      double keff = kf, Mfac = 1.0;
-      if (type != 0) {
-        const int row = rx_tbrow(w);
-        double M = m.tbd[row] * ctot;
-        for (int e = m.tbp[row]; e < m.tbp[row + 1]; ++e) M = fma(m.tbv[e], CS(m.tbs[e]), M);
-        if (type == 1) Mfac = M;
-        else keff = falloff_eval(m, r, type, kf, 0.0, M, T, lnT, invT).keff;
-      }
-      const double q = Mfac * keff * (Pf - rvsf);
-#pragma unroll
-      for (int sl = 0; sl < MAXSIDE; ++sl) {
-        int sp = m.rsp[sl * P + r];
-        if (sp >= 0) WS(sp) -= m.rnu[sl * P + r] * q;
-        int sq = m.psp[sl * P + r];
-        if (sq >= 0) WS(sq) += m.pnu[sl * P + r] * q;
+        cs[k * S] = rho * yw;
       }
     }
-    if (wdot) {
+    if (m.ntb)
+      for (int k = 0; k < ns; ++k) ctot += cs[k * S];
+    if (L.fix_rev)
       for (int k = 0; k < ns; ++k) {
-        double v = m.mw[k] * WS(k);
+        const bool lo = __double_as_longlong(T) <= m.tmid[k];
+        gs[k * S] = fix_gibbs(m.g + (lo ? 0 : 7 * nsp) + k, nsp, lo ? f.t11 : f.t13, f);
+      }
+    for (int k = 0; k < ns; ++k) {
+      ws[k * S] = 0.0;
+      ls[k * S] = 0;       // log2 c not formed yet
+    }
+    const int64_t lC0 = m.lC - (int64_t)(f.L >> 9);
+    for (int r = 0; r < m.nr; ++r) {
+      const uint64_t w = m.ix[r];
+      const int type = fix_type(w);
+      int64_t a = fix_arrhenius(m.a[r], m.b[r], m.e[r], f);
+      double Pf = 1.0;
+      bool none = false;
+      if (fix_power(w)) {
+#pragma unroll
+        for (int sl = 0; sl < 3; ++sl) {
+          const int s = fix_idx(w, sl);
+          if (s >= ns) continue;
+          uint64_t l = ls[s * S];
+          if (l == 0) {
+            // log2 c in Q57, sign flipped
+            const double c = cs[s * S];
+            const unsigned e = (unsigned)(__double2hiint(c) >> 20);     // sign and exponent
+            if (e - 960u < 126u) {
+              int ex;
+              const int64_t fr = log2_q62(c, m.lt, &ex);
+              l = ((((uint64_t)(int64_t)ex) << 57) + (uint64_t)(fr >> 5)) ^ 0x8000000000000000ull;
+            } else if ((__double_as_longlong(c) << 1) == 0) {
+              l = 1;     // c = 0
+            } else {
+              in = false;
+              l = 1;
+            }
+            ls[s * S] = l;
+          }
+          const uint64_t o = m.ord[sl * P + r];
+          if (l == 1) none = true;
+          else a += (int64_t)(mulhi_u(o, l) - (o >> 1)) >> 1;      // Q60 x Q57 -> Q53 -> Q52
+        }
+      } else {
+#pragma unroll
+        for (int sl = 0; sl < 3; ++sl) {
+          const int s = fix_idx(w, sl);
+          if (s < ns) Pf *= cs[s * S];
+        }
+      }
+      double M = 1.0;
+      if (type != 0) {
+        const int row = fix_tbrow(w);
+        M = m.tbd[row] * ctot;
+        for (int e = m.tbp[row]; e < m.tbp[row + 1]; ++e) M = fma(m.tbv[e], cs[m.tbs[e] * S], M);
+      }
+      double kf;
+      if (type < 2) kf = none ? 0.0 : exp2_q52(a, m.et);
+      else kf = cell_falloff(m, r - f0, type, a, M, f, T, fix2d((int64_t)f.v, 70));
+      const int sgn = ((int)(w >> 43) & 1) << 31;
+      kf = __hiloint2double(__double2hiint(kf) ^ sgn, __double2loint(kf));
+      double q = kf * Pf;
+      if (fix_rev(w)) {
+        int64_t ar = (type < 2 ? a : 0) - (int64_t)fix_dn(w) * lC0;
+        double Pr = 1.0;
+#pragma unroll
+        for (int sl = 0; sl < 3; ++sl) {
+          const int s = fix_idx(w, sl), p = fix_idx(w, 3 + sl);
+          if (s < ns) ar -= gs[s * S];
+          if (p < ns) { ar += gs[p * S]; Pr *= cs[p * S]; }
+        }
+        double kr = exp2_q52(ar, m.et);
+        if (type < 2) kr = __hiloint2double(__double2hiint(kr) ^ sgn, __double2loint(kr));
+        else kr *= kf;
+        q = fma(-kr, Pr, q);
+      }
+      if (type == 1) q *= M;
+      for (int e = m.rs[r]; e < m.rs[r + 1]; ++e) {
+        const int word = m.rw[e], code = word >> 8;
+        double* wk = ws + (word & 0xff) * S;
+        *wk = fma(code == 1 ? 1.0 : (code == -1 ? -1.0 : m.rv[code - 2]), q, *wk);
+      }
+    }
+    if (!in) {
+      small_cell_general(img, L, i, n, layout, Tg, pg, Yg, wdot, cpo, ho, roi_mode, roi_io, cs, S);
+      continue;
+    }
+    if (wdot)
+      for (int k = 0; k < ns; ++k) {
+        const double v = m.mw[k] * ws[k * S];
         if (roi_mode || layout == 0) wdot[i * ns + k] = v;
         else wdot[(int64_t)k * n + i] = v;
       }
-    }
-    (void)rho;
     if (cpo) cpo[i] = cpm * m.r_thermo;
     if (ho) ho[i] = hm * m.r_thermo * T;
   }
-#undef CS
-#undef GS
-#undef WS
 }
 
 // ---------------------------------------------------------------- warp
@@ -469,20 +638,36 @@ static cudaError_t launch_warp(const uint8_t* img, const ImageLayout& L, int64_t
   return cudaGetLastError();
 }
 
+// Thread per cell, small mechanisms.  Fixed point: blocks small enough that a
+// small batch reaches every SM.
+static cudaError_t launch_small(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
+                                const double* p, const double* Y, double* wdot, double* cp, double* h, int roi_mode,
+                                double* roi, cudaStream_t st) {
+  if (L.sfix) {
+    const int64_t per_sm = (n + device_sms() - 1) / device_sms();
+    const int bt = per_sm <= 32 ? 32 : (per_sm <= 64 ? 64 : SMALL_THREADS);
+    const size_t sm = (size_t)4 * L.ns * bt * sizeof(double);
+    cudaError_t e = set_smem((const void*)k_wdot_small_fix, (size_t)4 * L.ns * SMALL_THREADS * sizeof(double));
+    if (e != cudaSuccess) return e;
+    const int64_t g = grid_for((const void*)k_wdot_small_fix, bt, sm, n);
+    k_wdot_small_fix<<<(unsigned)g, bt, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, roi_mode, roi);
+  } else {
+    const size_t sm = small_smem(L);
+    set_smem((const void*)k_wdot_small, sm);
+    const int64_t g = grid_for((const void*)k_wdot_small, SMALL_THREADS, sm, n);
+    k_wdot_small<<<(unsigned)g, SMALL_THREADS, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, roi_mode, roi);
+  }
+  count_launch();
+  return cudaGetLastError();
+}
+
 bool use_small_kernel(const ImageLayout& L) { return L.ns <= SMALL_NSMAX && L.ns <= 8; }
 
 cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
                         const double* p, const double* Y, double* wdot, double* cp, double* h,
                         cudaStream_t st, int threads) {
   if (n <= 0) return cudaSuccess;
-  if (use_small_kernel(L)) {
-    size_t sm = small_smem(L);
-    set_smem((const void*)k_wdot_small, sm);
-    int64_t g = grid_for((const void*)k_wdot_small, SMALL_THREADS, sm, n);
-    k_wdot_small<<<(unsigned)g, SMALL_THREADS, sm, st>>>(img, L, n, layout, T, p, Y, wdot, cp, h, 0, nullptr);
-    count_launch();
-    return cudaGetLastError();
-  }
+  if (use_small_kernel(L)) return launch_small(img, L, n, layout, T, p, Y, wdot, cp, h, 0, nullptr, st);
   if (use_cell_kernel(L, n)) return launch_wdot_cell(img, L, n, layout, T, p, Y, wdot, cp, h, false, 0, st);
   return launch_warp<false, false>(img, L, n, layout, T, p, Y, wdot, cp, h, nullptr, nullptr, nullptr, st, 0, threads);
 }
@@ -512,13 +697,7 @@ cudaError_t launch_species_thermo(const uint8_t* img, const ImageLayout& L, int6
 cudaError_t launch_chemistry_source(const uint8_t* img, const ImageLayout& L, int64_t n, double* roi,
                                     const double* T, double* omegadot, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  size_t sm = small_smem(L);
-  set_smem((const void*)k_wdot_small, sm);
-  int64_t g = grid_for((const void*)k_wdot_small, SMALL_THREADS, sm, n);
-  k_wdot_small<<<(unsigned)g, SMALL_THREADS, sm, st>>>(img, L, n, 0, T, nullptr, nullptr, omegadot, nullptr,
-                                                         nullptr, 1, roi);
-  count_launch();
-  return cudaGetLastError();
+  return launch_small(img, L, n, 0, T, nullptr, nullptr, omegadot, nullptr, nullptr, 1, roi, st);
 }
 
 cudaError_t launch_wdot_jac(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
