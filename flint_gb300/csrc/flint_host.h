@@ -51,12 +51,12 @@ struct NvtxRange {
 // Largest dynamic shared memory a block may opt into on the current device.
 size_t device_smem_optin();
 // Opt a kernel into `bytes` of dynamic shared memory.  A refusal is returned
-// and consumed, so that it does not surface in a later cudaGetLastError.
-inline cudaError_t set_smem(const void* fn, size_t bytes) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) (void)cudaGetLastError();
-  return e;
-}
+// and consumed, so that it does not surface in a later cudaGetLastError.  What a
+// kernel was opted into on a device is remembered: asking the driver each time
+// costs a small launch more than the launch itself.
+cudaError_t set_smem(const void* fn, size_t bytes);
+// Blocks of a kernel that an SM holds (remembered as well), at least 0.
+int resident_blocks(const void* fn, int threads, size_t smem);
 
 // threads: threads per block of the warp kernels (64, 128 or 256; 0 = 256)
 cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,

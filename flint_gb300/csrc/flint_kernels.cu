@@ -14,6 +14,8 @@
 // SMs, so any N (including 0 and ragged tails) is handled without a tail kernel.
 #include <algorithm>
 #include <atomic>
+#include <mutex>
+#include <unordered_map>
 #include "flint_dev.cuh"
 #include "flint_fixkin.cuh"
 #include "flint_host.h"
@@ -553,9 +555,60 @@ size_t device_smem_optin() {
   return (size_t)cached_attr(g_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 48 * 1024);
 }
 
-static int64_t grid_for(const void* fn, int threads, size_t smem, int64_t work_items) {
+namespace {
+struct LaunchKey {
+  const void* fn;
+  size_t smem;
+  int threads, dev;
+  bool operator==(const LaunchKey& o) const {
+    return fn == o.fn && smem == o.smem && threads == o.threads && dev == o.dev;
+  }
+};
+struct LaunchKeyHash {
+  size_t operator()(const LaunchKey& k) const {
+    size_t h = reinterpret_cast<size_t>(k.fn);
+    h = h * 0x9E3779B97F4A7C15ull + k.smem;
+    return (h * 0x9E3779B97F4A7C15ull + (size_t)k.threads) * 0x9E3779B97F4A7C15ull + (size_t)k.dev;
+  }
+};
+// one entry per kernel, launch shape and device: a few dozen in all
+std::mutex g_launch_mu;
+std::unordered_map<LaunchKey, int, LaunchKeyHash> g_resident;
+std::unordered_map<LaunchKey, size_t, LaunchKeyHash> g_opted;   // threads = 0, smem = 0 in the key
+}  // namespace
+
+cudaError_t set_smem(const void* fn, size_t bytes) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const LaunchKey key{fn, 0, 0, dev};
+  std::lock_guard<std::mutex> lk(g_launch_mu);
+  auto it = g_opted.find(key);
+  if (it != g_opted.end() && it->second >= bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  else g_opted[key] = bytes;
+  return e;
+}
+
+int resident_blocks(const void* fn, int threads, size_t smem) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  const LaunchKey key{fn, smem, threads, dev};
+  std::lock_guard<std::mutex> lk(g_launch_mu);
+  auto it = g_resident.find(key);
+  if (it != g_resident.end()) return it->second;
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  if (per_sm > 0) g_resident[key] = per_sm;
+  return per_sm;
+}
+
+static int64_t grid_for(const void* fn, int threads, size_t smem, int64_t work_items) {
+  int per_sm = resident_blocks(fn, threads, smem);
   if (per_sm < 1) per_sm = 1;
   int64_t full = (int64_t)device_sms() * per_sm;
   int64_t need = (work_items + threads - 1) / threads;
@@ -613,8 +666,7 @@ int64_t warp_jac_scratch_doubles(const ImageLayout& L) {
   for (int c = 0; c < nc; ++c) {
     const size_t sm = warp_smem(L, true, cand[c]);
     if (set_smem(fn, sm) != cudaSuccess) return 0;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, cand[c], sm);
+    int per_sm = resident_blocks(fn, cand[c], sm);
     if (per_sm < 1) per_sm = 1;
     most = std::max(most, (int64_t)per_sm * device_sms() * (cand[c] / 32));
   }

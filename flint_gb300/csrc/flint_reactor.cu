@@ -743,8 +743,7 @@ static int slots_of(const ImageLayout& L, int layout) {
   size_t sm = reactor_smem(L, layout);
   const void* fn = (const void*)reactor_fn(L, layout);
   if (set_smem(fn, sm) != cudaSuccess) return 0;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, reactor_threads(layout), sm);
+  int per_sm = resident_blocks(fn, reactor_threads(layout), sm);
   return per_sm * device_sms() * (reactor_threads(layout) / 32);
 }
 
@@ -802,8 +801,7 @@ cudaError_t launch_reactor(const uint8_t* img, const ImageLayout& L, int64_t n, 
   cudaError_t e = set_smem(fn, sm);
   if (e != cudaSuccess) return e;
   const int threads = reactor_threads(layout), wpb = threads / 32;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sm);
+  int per_sm = resident_blocks(fn, threads, sm);
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   int64_t warps_needed = n;
   int64_t blocks = (warps_needed + wpb - 1) / wpb;

@@ -633,8 +633,7 @@ cudaError_t launch_general(const uint8_t* img, const TableLayout& L, const doubl
   const void* fn = rhs ? (const void*)k_general_warp<1> : (const void*)k_general_warp<0>;
   cudaError_t e = set_smem(fn, sm);
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TABLE_THREADS, sm);
+  int per_sm = resident_blocks(fn, TABLE_THREADS, sm);
   if (per_sm < 1) per_sm = 1;
   int64_t blocks = (n + TABLE_THREADS / 32 - 1) / (TABLE_THREADS / 32);
   int64_t full = (int64_t)device_sms() * per_sm;

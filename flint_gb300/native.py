@@ -151,6 +151,19 @@ def lib():
     return L
 
 
+_raw_stream = None
+
+
+def current_stream():
+    """The current torch stream as a pointer (torch's Stream object costs a small
+    call more than the call's own launch)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        _raw_stream = (torch._C._cuda_getCurrentRawStream, torch.cuda.current_device)
+    return C.c_void_p(_raw_stream[0](_raw_stream[1]()))
+
+
 def check(rc, what=""):
     if rc != FLINT_OK:
         msg = lib().flint_last_error().decode(errors="replace")

@@ -94,9 +94,7 @@ def _ptr(t):
     return C.c_void_p(t.data_ptr())
 
 
-def _stream():
-    import torch
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+_stream = native.current_stream
 
 
 # ------------------------------------------------------------------ data

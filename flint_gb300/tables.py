@@ -523,7 +523,7 @@ class Tables:
         import torch
         if omegadot is None:
             omegadot = torch.empty_like(roi)
-        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        s = native.current_stream()
         native.check(self.L.flint_chemistry_source_batch(self.h, T.shape[0], C.c_void_p(roi.data_ptr()),
                                                          C.c_void_p(T.data_ptr()), C.c_void_p(omegadot.data_ptr()),
                                                          s), "flint_chemistry_source_batch")
@@ -534,7 +534,7 @@ class Tables:
         import torch
         if F is None:
             F = torch.empty_like(Z)
-        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        s = native.current_stream()
         native.check(self.L.flint_rhs_native_batch(self.h, Z.shape[0], C.c_void_p(Z.data_ptr()),
                                                    C.c_void_p(F.data_ptr()), s), "flint_rhs_native_batch")
         return F
@@ -546,7 +546,7 @@ class Tables:
             mu = torch.empty_like(T)
         if lam is None:
             lam = torch.empty_like(T)
-        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        s = native.current_stream()
         native.check(self.L.flint_transport_batch(self.h, rhoi.shape[0], C.c_void_p(rhoi.data_ptr()),
                                                   C.c_void_p(T.data_ptr()), C.c_void_p(mu.data_ptr()),
                                                   C.c_void_p(lam.data_ptr()), s), "flint_transport_batch")
@@ -561,7 +561,7 @@ class Tables:
             prim = torch.empty_like(cons)
         if T_out is None:
             T_out = torch.empty_like(T)
-        s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        s = native.current_stream()
         native.check(self.L.flint_cons2prim_batch(self.h, cons.shape[0], ndim, C.c_void_p(cons.data_ptr()),
                                                   C.c_void_p(T.data_ptr()), C.c_void_p(prim.data_ptr()),
                                                   C.c_void_p(T_out.data_ptr()), s), "flint_cons2prim_batch")
