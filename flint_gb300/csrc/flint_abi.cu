@@ -57,6 +57,7 @@ struct flint_mech_s {
   // saved-Jacobian scratch of the reactor, one slot per resident warp
   double* djsave = nullptr;
   int jslots = 0;
+  int* jorder = nullptr;   // the reactor's order of cells (ORDER_CELLS), behind the slots
   int rx_layout = 0;       // reactor layout chosen by flint_reactor_autotune (0: by size)
   int tuned_n = 0;         // layouts the last flint_reactor_autotune timed, and their times
   int tuned_layout[8] = {0};
@@ -1023,7 +1024,7 @@ int flint_reactor_advance(flint_mech_t h, int64_t n, double* T, const double* p,
   rc = ensure_jsave(h);
   if (rc) return rc;
   cudaError_t e = launch_reactor(h->dimg, h->L, n, T, p, Y, dt, o, status, nsteps, h->dcounter, h->djsave,
-                                 h->jslots, (cudaStream_t)stream, nullptr, h->rx_layout);
+                                 h->jslots, (cudaStream_t)stream, nullptr, h->rx_layout, h->jorder);
   return e == cudaSuccess ? FLINT_OK : cuda_fail(e, "flint_reactor_advance");
 }
 
@@ -1062,7 +1063,7 @@ int flint_reactor_autotune(flint_mech_t h, int64_t n, const double* T, const dou
         if (!e) e = cudaMemcpyAsync(Yc, Y, n * ns * sizeof(double), cudaMemcpyDeviceToDevice, st);
         if (!e) e = cudaEventRecord(e0, st);
         if (!e) e = launch_reactor(h->dimg, h->L, n, Tc, p, Yc, dt, o, sc, nsc, h->dcounter, h->djsave, h->jslots,
-                                   st, nullptr, cand[c]);
+                                   st, nullptr, cand[c], h->jorder);
         if (!e) e = cudaEventRecord(e1, st);
         if (!e) e = cudaEventSynchronize(e1);
       }
@@ -1200,9 +1201,11 @@ static int ensure_jsave(flint_mech_t h) {
   if (h->djsave) return FLINT_OK;
   int slots = reactor_slots(h->L);
   if (slots < 1) return fail(FLINT_ERR_MECH, "reactor kernel does not fit this mechanism (shared memory)");
-  cudaError_t ea = cudaMalloc(&h->djsave, (size_t)slots * reactor_slot_bytes(h->L));
+  const size_t slot_bytes = (size_t)slots * reactor_slot_bytes(h->L);
+  cudaError_t ea = cudaMalloc(&h->djsave, slot_bytes + ORDER_CELLS * sizeof(int));
   if (ea != cudaSuccess) { h->djsave = nullptr; return fail(FLINT_ERR_NOMEM, "reactor scratch: %s", cudaGetErrorString(ea)); }
   h->jslots = slots;
+  h->jorder = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(h->djsave) + slot_bytes);
   return FLINT_OK;
 }
 
@@ -1277,7 +1280,7 @@ int flint_surrogate_advance(flint_surrogate_t s, int64_t n, double* T, const dou
   rc = ensure_jsave(s->mech);
   if (rc) return rc;
   rc = surrogate_advance(s->s, n, T, p, Y, dt, o, gate, status, nsteps, s->mech->djsave, s->mech->jslots,
-                         nullptr, counts != nullptr, (cudaStream_t)stream, s->mech->rx_layout);
+                         nullptr, counts != nullptr, (cudaStream_t)stream, s->mech->rx_layout, s->mech->jorder);
   if (rc) return fail(rc, "flint_surrogate_advance failed: %s", cudaGetErrorString(cudaGetLastError()));
   if (counts) surrogate_counts(s->s, &counts[0], &counts[1]);
   return FLINT_OK;

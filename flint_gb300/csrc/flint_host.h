@@ -94,7 +94,10 @@ cudaError_t launch_reactor(const uint8_t* img, const ImageLayout& L, int64_t n, 
                            double* Y, const double* dt, const flint_reactor_opts& o, int* status, int* nsteps,
                            unsigned int* work_counter, double* jsave, int slots, cudaStream_t st,
                            const unsigned long long* n_dev = nullptr,   // optional device-side cell count <= n
-                           int layout = REACTOR_LAYOUT_AUTO);
+                           int layout = REACTOR_LAYOUT_AUTO,
+                           int* order = nullptr);   // scratch for ORDER_CELLS cells' order; null: as they lie
+// Cells up to which the reactor takes them up longest first.
+constexpr int ORDER_CELLS = 65536;
 
 size_t reactor_noalloc_bytes();
 int reactor_noalloc_slots();
@@ -120,7 +123,7 @@ int surrogate_state(Surrogate* s, int net, float* host, int64_t* step, int get);
 int surrogate_advance(Surrogate* s, int64_t n, double* T, const double* p, double* Y, const double* dt,
                       const flint_reactor_opts& o, const flint_surrogate_gate* gate, int* status, int* nsteps,
                       double* jsave, int jslots, double* metrics, bool want_counts, cudaStream_t st,
-                      int reactor_layout = REACTOR_LAYOUT_AUTO);
+                      int reactor_layout = REACTOR_LAYOUT_AUTO, int* order = nullptr);
 void surrogate_counts(Surrogate* s, int64_t* acc, int64_t* rej);
 int surrogate_set_forward(Surrogate* s, int mode);
 int surrogate_forward_kind(Surrogate* s);
