@@ -485,18 +485,19 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   auto sec = [&](int bytes) { int o = off; off = rup(off + bytes, 16); return o; };
   const int ntbl = (L.o_tbv - L.o_tbs) / 4, nlist = std::max(L.nlist, 1);
   L.f_mw = sec(8 * S); L.f_invmw = sec(8 * S); L.f_tmid = sec(8 * S);
-  L.f_g = sec(8 * 14 * S); L.f_h = sec(8 * 12 * S); L.f_c = sec(8 * 10 * S);
   L.f_a = sec(8 * P); L.f_b = sec(8 * P); L.f_e = sec(8 * P); L.f_ix = sec(8 * P);
   L.f_ra = sec(8 * 16); L.f_rb = sec(8 * 16); L.f_re = sec(8 * 16); L.f_tr = sec(8 * 5 * 16);
   L.f_tbd = sec(8 * L.ntb); L.f_tbp = sec(4 * (L.ntb + 1)); L.f_tbs = sec(4 * ntbl); L.f_tbv = sec(8 * ntbl);
   L.f_cx = sec(8 * P); L.f_cy = sec(8 * P);
-  L.f_ord = sec(8 * 3 * P);
   L.f_rs = sec(4 * (nr + 1)); L.f_rw = sec(4 * nlist); L.f_rv = sec(8 * (int)std::max<size_t>(rv.size(), 1));
   L.f_exp = sec(8 * FIX_EXP2); L.f_log = sec(8 * 2 * FIX_LOG2);
-  L.fix_bytes_cell = off;   // the thread-per-cell kernel needs no species lists
+  L.fix_bytes_cell = off;
+  L.f_g = sec(8 * 14 * S); L.f_h = sec(8 * 12 * S); L.f_c = sec(8 * 10 * S);
+  L.fix_bytes_thermo = off;
   L.f_seg = sec(4 * (int)seg.size()); L.f_segv = sec(8 * (int)segv.size()); L.f_piece = sec(4 * (S + 1));
   L.fix_bytes_rate = off;   // kernels without a Jacobian need no species lists
   L.f_term = sec(4 * (int)term.size()); L.f_target = sec(2 * (int)target.size()); L.f_coef = sec(8 * (int)coef.size());
+  L.f_ord = sec(8 * 3 * P);
   L.o_fix = L.bytes;
   L.fix_bytes = off;
   img.resize((size_t)L.bytes + off, 0);

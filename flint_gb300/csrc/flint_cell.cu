@@ -78,14 +78,15 @@ template <bool RHS, bool THERMO>
 __global__ void __launch_bounds__(32 * CELL_MAX_WARPS)
 k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, int layout,
             const double* __restrict__ Tg, const double* __restrict__ pg, const double* __restrict__ Yg,
-            double* __restrict__ out, double* __restrict__ cpo, double* __restrict__ ho, int cv) {
+            double* __restrict__ out, double* __restrict__ cpo, double* __restrict__ ho, int cv, int staged) {
   extern __shared__ __align__(16) uint8_t smem[];
-  stage_image(smem, img + L.o_fix, L.fix_bytes_cell);
+  stage_image(smem, img + L.o_fix, staged);
   FixView m;
   m.bind(L, smem);
+  if (staged < L.fix_bytes_thermo) m.bind_thermo(L, img + L.o_fix);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int ns = m.ns, nsp = m.nsp, nr = m.nr, f0 = nr - m.nfall, nv = ns + 1;
-  double* base = reinterpret_cast<double*>(smem + L.fix_bytes_cell) + wid * cell_warp_doubles(ns);
+  double* base = reinterpret_cast<double*>(smem + staged) + wid * cell_warp_doubles(ns);
   double* c = base + lane;                 // row k: c[k * CELL_ROW], G and w one and two paddings on
   int64_t* G = reinterpret_cast<int64_t*>(c + CELL_PAD);
   double* w = c + 2 * CELL_PAD;
@@ -278,24 +279,27 @@ k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
 }
 
 // Warps per block: what fits a block's shared memory, at most 8.
-static int cell_warps(const ImageLayout& L) {
+static int cell_warps(const ImageLayout& L, int staged) {
   const size_t room = device_smem_optin(), per = cell_warp_doubles(L.ns) * sizeof(double);
-  if (room < L.fix_bytes_cell + per) return 0;
-  return (int)std::min<size_t>(CELL_MAX_WARPS, (room - L.fix_bytes_cell) / per);
+  if (room < staged + per) return 0;
+  return (int)std::min<size_t>(CELL_MAX_WARPS, (room - staged) / per);
 }
 
 // When the thread-per-cell kernel is the faster one.  A warp's pass over the
-// reactions takes the same time for one cell as for 32 (31 species, 160
-// reactions: 120 us with one warp per scheduler, 145 us with two), so the GPU
-// has to be given enough cells: it passes the warp-per-cell kernel at about 100
-// per SM (16,000 cells: 121 against 134 us; 12,000: 121 against 99 us; 197
-// reactions: 148 against 180 and 131 us), and at 1 M cells it takes 4.57 ms
-// against 8.0.  With 4 resident warps (54 species) there is too little to hide
-// latencies behind: 100,003 cells take 1.37 ms against 1.28, so six or more are
-// asked for.
+// reactions takes about the same time for one cell as for 32 (31 species, 160
+// reactions: 121 us with four warps on an SM, 145 with eight), so each round of
+// warps has to bring enough cells: as many as the warp-per-cell kernel does in that
+// time, about 145 per SM (measured, thread against warp: 20,000 cells 136 against
+// 125 us, 24,000 136 against 146, 32,000 145 against 193; 197 reactions: 20,000 167
+// against 152, 24,000 167 against 177).  At 1 M cells it takes 4.5 ms against 6.1.
+// With 4 resident warps (54 species) there is too little to hide latencies
+// behind (100,003 cells: 1.37 ms against 1.28 with the warp kernel of that time), so
+// six or more are asked for.
 bool use_cell_kernel(const ImageLayout& L, int64_t n) {
-  return L.fix && n >= 100 * (int64_t)device_sms() && cell_warps(L) >= 6 &&
-         scratch_small_doubles(L.nsp, L.nrpad) <= cell_warp_doubles(L.ns);
+  const int64_t sms = device_sms(), w = cell_warps(L, L.fix_bytes_cell);
+  if (!L.fix || w < 6 || scratch_small_doubles(L.nsp, L.nrpad) > cell_warp_doubles(L.ns)) return false;
+  const int64_t rounds = (n + 32 * w * sms - 1) / (32 * w * sms);
+  return n >= 145 * sms * rounds;
 }
 
 cudaError_t launch_wdot_cell(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
@@ -303,13 +307,18 @@ cudaError_t launch_wdot_cell(const uint8_t* img, const ImageLayout& L, int64_t n
                              cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int64_t tasks = (n + 31) / 32, sms = device_sms();
-  const int w = (int)std::min<int64_t>(cell_warps(L), (tasks + sms - 1) / sms);
-  const size_t sm = L.fix_bytes_cell + (size_t)w * cell_warp_doubles(L.ns) * sizeof(double);
+  // the thermo polynomials are read once per cell, at the same place on every
+  // lane: they stay in global memory where staging them would cost a warp (1 M
+  // cells of 31 species: 4.57 ms staged, 4.76 not, both with 8 warps; 4.9 staged with 7)
+  const int wmax = cell_warps(L, L.fix_bytes_cell);
+  const int staged = cell_warps(L, L.fix_bytes_thermo) == wmax ? L.fix_bytes_thermo : L.fix_bytes_cell;
+  const int w = (int)std::min<int64_t>(wmax, (tasks + sms - 1) / sms);
+  const size_t sm = staged + (size_t)w * cell_warp_doubles(L.ns) * sizeof(double);
   auto* fn = rhs ? k_wdot_cell<true, false> : (cp || h ? k_wdot_cell<false, true> : k_wdot_cell<false, false>);
   cudaError_t e = set_smem((const void*)fn, sm);
   if (e != cudaSuccess) return e;
   const int64_t blocks = std::min<int64_t>(sms, (tasks + w - 1) / w);
-  fn<<<(unsigned)blocks, 32 * w, sm, st>>>(img, L, n, layout, T, p, Y, out, cp, h, cv);
+  fn<<<(unsigned)blocks, 32 * w, sm, st>>>(img, L, n, layout, T, p, Y, out, cp, h, cv, staged);
   count_launch();
   return cudaGetLastError();
 }

@@ -73,8 +73,9 @@ struct ImageLayout {
   // at o_fix, 16-byte aligned, fix_bytes long; the f_ offsets are relative to
   // o_fix.  `bytes` above counts the FP64 sections only.
   int fix, o_fix, fix_bytes;
-  int fix_bytes_cell, fix_bytes_rate;   // the leading parts that the thread-per-cell kernel and the warp kernels
-                                        // without a Jacobian stage
+  // the leading parts that the thread-per-cell kernel stages, without and with the
+  // thermo polynomials, and the warp kernels without a Jacobian
+  int fix_bytes_cell, fix_bytes_thermo, fix_bytes_rate;
   int sfix;                      // the small-mechanism kernel (<= 16 species) may use the image
   int fix_rev;                   // some reaction is reversible
   int f_ord;                     // uint64 [3][nrpad]: orders (Q60) of the reactions in power form

@@ -46,12 +46,16 @@ struct FixView {
     auto U = [&](int o) { return (const uint64_t*)(base + o); };
     mw = D(L.f_mw); invmw = D(L.f_invmw); tr = D(L.f_tr); tbd = D(L.f_tbd); tbv = D(L.f_tbv);
     tmid = I(L.f_tmid); a = I(L.f_a); ra = I(L.f_ra);
-    g = U(L.f_g); h = U(L.f_h); c = U(L.f_c); b = U(L.f_b); e = U(L.f_e);
+    b = U(L.f_b); e = U(L.f_e);
+    bind_thermo(L, base);
     rb = U(L.f_rb); re = U(L.f_re); et = U(L.f_exp); lt = U(L.f_log); ix = U(L.f_ix); ord = U(L.f_ord); cx = U(L.f_cx); cy = U(L.f_cy);
     tbp = (const int*)(base + L.f_tbp); tbs = (const int*)(base + L.f_tbs);
     rs = (const int*)(base + L.f_rs); rw = (const int*)(base + L.f_rw); rv = D(L.f_rv);
     seg = (const uint32_t*)(base + L.f_seg); segv = D(L.f_segv); piece = (const int*)(base + L.f_piece);
     bind_terms(L, base);
+  }
+  __device__ __forceinline__ void bind_thermo(const ImageLayout& L, const uint8_t* base) {
+    g = (const uint64_t*)(base + L.f_g); h = (const uint64_t*)(base + L.f_h); c = (const uint64_t*)(base + L.f_c);
   }
   __device__ __forceinline__ void bind_terms(const ImageLayout& L, const uint8_t* base) {
     term = (const uint32_t*)(base + L.f_term); target = (const uint16_t*)(base + L.f_target);

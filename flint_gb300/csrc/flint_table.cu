@@ -424,8 +424,11 @@ k_general_warp(const uint8_t* __restrict__ img, TableLayout L, const double* __r
 // The table rows differ from lane to lane; two reactions' entries are one 16-byte
 // load, fetched a pair ahead.
 constexpr int TC_MAX_WARPS = 12;
-// From how many cells per SM on it is the faster kernel (see launch_general).
-constexpr int64_t TC_CELLS_PER_SM = 16;
+// From how many cells per SM on it is the faster kernel.  A warp's pass takes 306 us
+// (31 species, 160 reactions) or 385 us (197) however few its cells; the
+// warp-per-cell kernel takes 73 and 140 us per 1,000 cells and passes that at 4,200
+// and 2,750 cells.
+constexpr int64_t TC_CELLS_PER_SM = 24;
 
 __device__ __forceinline__ double tc_ipow(double x, int n) {
   if (n == 1) return x;

@@ -99,7 +99,7 @@ def test_unnormalised_mass_fractions(scale):
 
 
 @pytest.mark.parametrize("name", ["c2", "c5", "tsr_rich_31", "pelucchi", "coria"])
-@pytest.mark.parametrize("n", [15199, 15200, 15233])
+@pytest.mark.parametrize("n", [22039, 22040, 22073])
 def test_thread_per_cell(name, n):
     """Batches large enough for the thread-per-cell kernel, a ragged last warp and
     cells outside the fixed-point range among them, in both storage orders and as

@@ -44,7 +44,7 @@ def small_batches(f, *arrays, size=1000):
 
 
 @pytest.mark.parametrize("name", ["c2_no_falloff", "c2", "pelucchi", "tsr_rich_31"])
-@pytest.mark.parametrize("n", [2431, 2432, 2433, 5003])
+@pytest.mark.parametrize("n", [3647, 3648, 3649, 5003])
 def test_general_loop(name, n):
     m = mechanism(name)
     gpu = tables.Tables(tables.generate(m, 1, 3000))
@@ -69,7 +69,7 @@ def test_general_loop(name, n):
 def test_odd_concentrations(value):
     m = mechanism("c2_no_falloff")
     gpu = tables.Tables(tables.generate(m, 1, 3000))
-    T, roi = states(m, 2600, 5)
+    T, roi = states(m, 3700, 5)
     for i in range(m.ns):
         roi[7 * i, i] = value
     w = gpu.chemistry_source(roi, T)
