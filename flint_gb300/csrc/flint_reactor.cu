@@ -352,6 +352,23 @@ static size_t reactor_smem_spl1(const ImageLayout& L) {
 // REACTOR_LAYOUT_SHARED / _GLOBAL force one (the autotuner times both).
 // REACTOR_LAYOUT_GLOBAL2B: global slots, two blocks of 8 warps per SM (16
 // resident warps) from a build capped at 128 registers per thread.
+// REACTOR_LAYOUT_WIDE is not a caller's choice: the shared-memory layout takes this
+// form for many cells (launch_reactor).  The derivatives that a Jacobian goes through
+// move to the warp's global slot (a Jacobian comes once in 24 right-hand sides); 7 KB
+// less of shared memory per warp leave room for 12 warps on an SM instead of 8, at 168
+// registers a thread.
+// REACTOR_LAYOUT_NARROW, of the allocation-free entry, is SHARED without that form: its
+// slots hold the saved Jacobian alone.
+constexpr int REACTOR_LAYOUT_WIDE = 100, REACTOR_LAYOUT_NARROW = 101;
+constexpr int WIDE_THREADS = 384;
+
+static size_t wide_warp_doubles(const ImageLayout& L) {
+  return scratch_small_doubles(L.nsp, L.nrpad) + (((L.nsp + 1) * (L.nsp + 1) + 1) & ~1);
+}
+static size_t wide_smem(const ImageLayout& L) {
+  return staged_bytes(L) + (WIDE_THREADS / 32) * (wide_warp_doubles(L) * sizeof(double) + 64 * sizeof(int));
+}
+
 static bool reactor_gj(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
   if (spl_of(L) > 1 || reactor_smem_spl1(L) > device_smem_optin()) return true;
   return layout == REACTOR_LAYOUT_GLOBAL || layout == REACTOR_LAYOUT_GLOBAL4 || layout == REACTOR_LAYOUT_GLOBAL2B;
@@ -359,13 +376,18 @@ static bool reactor_gj(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
 
 // Threads per block: 8 warps, or 4 in the GLOBAL4 layout (half the resident
 // warps, twice the L1 per warp for the global Newton matrices).
-static int reactor_threads(int layout) { return layout == REACTOR_LAYOUT_GLOBAL4 ? 128 : REACTOR_THREADS; }
+// WIDE has 12.
+static int reactor_threads(int layout) {
+  return layout == REACTOR_LAYOUT_GLOBAL4 ? 128 : layout == REACTOR_LAYOUT_WIDE ? WIDE_THREADS : REACTOR_THREADS;
+}
 
 // Doubles per resident-warp slot of the reactor's global scratch: the saved
-// Jacobian (32*SPL)^2, and in GJ layout the Jacobian work area too.
+// Jacobian (32*SPL)^2, in GJ layout the Jacobian work area too, in WIDE its derivatives.
 static int64_t reactor_slot_doubles_of(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
   const int spl = spl_of(L);
-  return (int64_t)(32 * spl) * (32 * spl) + (reactor_gj(L, layout) ? scratch_jac_doubles(L) : 0);
+  const int64_t saved = (int64_t)(32 * spl) * (32 * spl);
+  if (layout == REACTOR_LAYOUT_WIDE) return saved + ((L.dq_rows * L.nrpad + 1) & ~1);
+  return saved + (reactor_gj(L, layout) ? scratch_jac_doubles(L) : 0);
 }
 
 // Order in which the cells are taken up, the likely longest first, so that the
@@ -421,8 +443,8 @@ k_order(int64_t n, const double* __restrict__ T, const double* __restrict__ dt, 
   for (int i = t; i < (int)n; i += blockDim.x) order[atomicAdd(&count[cls(i)], 1)] = i;
 }
 
-template <int SPL, bool GJ, int MINB, bool FIX>
-__global__ void __launch_bounds__(REACTOR_THREADS, MINB)
+template <int SPL, bool GJ, int MINB, bool FIX, bool WIDE = false>
+__global__ void __launch_bounds__(WIDE ? WIDE_THREADS : REACTOR_THREADS, MINB)
 k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, double* __restrict__ Tg,
           const double* __restrict__ pg, double* __restrict__ Yg, const double* __restrict__ dtg,
           flint_reactor_opts o, int* __restrict__ status_g, int* __restrict__ nsteps_g,
@@ -448,7 +470,13 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
   constexpr int JW = 32 * SPL;   // row stride of the saved Jacobian
   WarpScratch s;
   int* pivs;
-  if (!GJ) {
+  if (WIDE) {
+    const int small = scratch_small_doubles(nsp, nrpad), sd = small + (((nsp + 1) * (nsp + 1) + 1) & ~1);
+    double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
+    s = carve2(wbase, Jg + JW * JW, L);
+    s.Jr = wbase + small;
+    pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
+  } else if (!GJ) {
     const int sd = scratch_doubles(L, true);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
     s = carve(wbase, L, true);
@@ -772,6 +800,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
 }
 
 size_t reactor_smem(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
+  if (layout == REACTOR_LAYOUT_WIDE) return wide_smem(L);
   if (!reactor_gj(L, layout)) return reactor_smem_spl1(L);
   return staged_bytes(L) + (reactor_threads(layout) / 32) *
                        (scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double) + 64 * spl_of(L) * sizeof(int));
@@ -784,6 +813,7 @@ typedef void (*ReactorKernel)(const uint8_t*, ImageLayout, int64_t, double*, con
 template <bool FIX>
 static ReactorKernel reactor_kernel(const ImageLayout& L, int layout) {
   const bool two = layout == REACTOR_LAYOUT_GLOBAL2B;
+  if (layout == REACTOR_LAYOUT_WIDE) return k_reactor<1, false, 1, true, true>;
   if (spl_of(L) > 1) return two ? k_reactor<2, true, 2, FIX> : k_reactor<2, true, 1, FIX>;
   if (two) return k_reactor<1, true, 2, FIX>;
   return reactor_gj(L, layout) ? k_reactor<1, true, 1, FIX> : k_reactor<1, false, 1, FIX>;
@@ -799,6 +829,17 @@ static int slots_of(const ImageLayout& L, int layout) {
   if (set_smem(fn, sm) != cudaSuccess) return 0;
   int per_sm = resident_blocks(fn, reactor_threads(layout), sm);
   return per_sm * device_sms() * (reactor_threads(layout) / 32);
+}
+
+// WIDE's rule.  31 species, 8 against 12 warps on an SM: 89.5 / 106 ms at 2,432 cells,
+// 164 / 157 at 4,096, 298 / 287 at 8,192, 592 / 537 at 16,384 (a round of 12 warps takes
+// longer than one of 8, and 168 registers spill a little): from two rounds of 12 warps on
+// every SM.
+// Where the count is only on the device it may be far below n (the cells that a
+// surrogate leaves): 8 warps.
+static bool reactor_wide(const ImageLayout& L, int64_t n, bool n_on_device) {
+  return L.fix && !n_on_device && !reactor_gj(L) && wide_smem(L) <= device_smem_optin() &&
+         n >= 2ll * (WIDE_THREADS / 32) * device_sms();
 }
 
 // Resident-warp slots and bytes per slot that serve every layout.
@@ -848,18 +889,23 @@ cudaError_t launch_reactor(const uint8_t* img, const ImageLayout& L, int64_t n, 
                            const unsigned long long* n_dev, int layout, int* order) {
   if (n <= 0) return cudaSuccess;
   if (spl_of(L) < 1 || spl_of(L) > 2) return cudaErrorInvalidValue;
+  if (layout <= REACTOR_LAYOUT_SHARED && reactor_wide(L, n, n_dev != nullptr)) layout = REACTOR_LAYOUT_WIDE;
   NvtxRange nvtx("reactor.advance");
   size_t sm = reactor_smem(L, layout);
   const ReactorKernel kern = reactor_fn(L, layout);
   const void* fn = (const void*)kern;
   cudaError_t e = set_smem(fn, sm);
   if (e != cudaSuccess) return e;
-  const int threads = reactor_threads(layout), wpb = threads / 32;
-  int per_sm = resident_blocks(fn, threads, sm);
+  const int most = reactor_threads(layout);
+  int per_sm = resident_blocks(fn, most, sm);
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int64_t warps_needed = n;
-  int64_t blocks = (warps_needed + wpb - 1) / wpb;
-  int64_t full = (int64_t)device_sms() * per_sm;
+  const int64_t full = (int64_t)device_sms() * per_sm;
+  // Fewer cells than warps: smaller blocks on more SMs, with the matrices in shared
+  // memory (31 species, 600 cells: 40.3 ms, in blocks of 8 warps 45.5).  Matrices in
+  // global slots keep full blocks (54 species, 600 cells: 260 ms, spread 328).
+  const int wpb = reactor_gj(L, layout) ? most / 32 : (int)std::min<int64_t>(most / 32, (n + full - 1) / full);
+  const int threads = 32 * wpb;
+  int64_t blocks = (n + wpb - 1) / wpb;
   if (blocks > full) blocks = full;
   if (blocks * wpb > slots) blocks = slots / wpb;
   if (blocks < 1) return cudaErrorInvalidValue;
@@ -925,8 +971,8 @@ static cudaError_t noalloc_scratch_address(void** out) {
 }
 
 size_t reactor_noalloc_bytes() { return NOALLOC_BYTES; }
-// Only the shared-memory layout keeps a warp's scratch within one 32 x 32
-// slot; the entry point always runs it (a layout chosen by
+// Only the shared-memory layout with 8 warps keeps a warp's scratch within one 32 x 32
+// slot; the entry point always runs that form (a layout chosen by
 // flint_reactor_autotune applies to flint_reactor_advance only).
 bool reactor_noalloc_fits(const ImageLayout& L) { return reactor_slot_doubles_of(L) <= JSLOT; }
 int reactor_noalloc_slots() { return NOALLOC_SLOTS; }
@@ -941,7 +987,7 @@ cudaError_t launch_reactor_noalloc_prepare(const ImageLayout& L) {
   if (e != cudaSuccess) return e;
   e = ensure_bdf_table();
   if (e != cudaSuccess) return e;
-  return set_smem((const void*)reactor_fn(L), reactor_smem(L));
+  return set_smem((const void*)reactor_fn(L, REACTOR_LAYOUT_NARROW), reactor_smem(L, REACTOR_LAYOUT_NARROW));
 }
 
 cudaError_t launch_reactor_noalloc(const uint8_t* img, const ImageLayout& L, int64_t n, double* T, const double* p,
@@ -955,7 +1001,8 @@ cudaError_t launch_reactor_noalloc(const uint8_t* img, const ImageLayout& L, int
   unsigned int* counters = reinterpret_cast<unsigned int*>(base);
   double* jsave = reinterpret_cast<double*>(static_cast<unsigned char*>(base) + NOALLOC_COUNTER_BYTES);
   // launch_reactor zeroes the counters on `st` and caps the grid to the slots
-  return launch_reactor(img, L, n, T, p, Y, dt, o, status, nsteps, counters, jsave, NOALLOC_SLOTS, st);
+  return launch_reactor(img, L, n, T, p, Y, dt, o, status, nsteps, counters, jsave, NOALLOC_SLOTS, st,
+                        nullptr, REACTOR_LAYOUT_NARROW);
 }
 
 }  // namespace flint
