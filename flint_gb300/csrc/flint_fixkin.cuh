@@ -437,13 +437,14 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   // at different places of different lists).  Column ns collects what a third
   // body adds to every column, row ns T times the derivative by T.
   __syncwarp();   // the pieces lie in the rows
-  const int ld = s.ldj;
-#pragma unroll
-  for (int j = 0; j < SPL; ++j) {
-    const int k = lane + 32 * j;
-    if (k <= ns)
-      for (int jj = 0; jj <= ns; ++jj) s.Jr[k * ld + jj] = 0.0;
-  }
+  // SPL 2: the work area lies in global memory and its entries by columns, so that
+  // lanes (rows) that go along a row read whole sectors (54 species, 320 reactions,
+  // 20,011 cells: 2.30 -> 2.21 ms).  With the derivatives in shared memory instead
+  // the L1 left over is too small for the rows: 2.61.
+  constexpr bool COL = SPL > 1;
+  constexpr int ld = 32 * SPL + 1;
+  constexpr int rs = COL ? 1 : ld, cs = COL ? ld : 1;   // strides of a row and of a column
+  for (int i = lane; i < (ns + 1) * ld; i += WARP) s.Jr[i] = 0.0;
   __syncwarp();
   {
     double acc = 0.0;
@@ -452,7 +453,8 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
       const uint32_t w = m.term[32 * e + lane];
       acc = fma(m.coef[(w >> 16) & 0xfffu], s.dq[w & 0xffffu], acc);
       if ((int)w < 0) {
-        s.Jr[*target] = acc;
+        const int t = *target;   // row * ld + column
+        s.Jr[COL ? t / ld + t % ld * ld : t] = acc;
         target += WARP;
         acc = 0.0;
       }
@@ -467,23 +469,23 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
     const int k = lane + 32 * j;
     Sk[j] = 0.0; HJ[j] = 0.0; tball[j] = 0.0; JT[j] = 0.0;
     if (k < ns) {
-      const double* Jrow = s.Jr + k * ld;
-      tball[j] = Jrow[ns];
-      JT[j] = s.Jr[ns * ld + k] * invT;
+      const double* Jrow = s.Jr + k * rs;
+      tball[j] = Jrow[ns * cs];
+      JT[j] = s.Jr[ns * rs + k * cs] * invT;
       const double* a = (const double*)(img + L.o_nasa) + k;
       const double tm = a[14 * nsp];
       a += __double_as_longlong(T) <= __double_as_longlong(tm) ? 0 : 7 * nsp;
       const double dcp = fma(T, fma(T, fma(4.0 * T, a[4 * nsp], 3.0 * a[3 * nsp]), 2.0 * a[2 * nsp]), a[nsp]);
       if (cv) {
         // rho fixed: no dependence of c on T or through rho on Y (Sk = 0)
-        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk] - 1.0, s.Jr[kk * ld + k], HJ[j]);
+        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk] - 1.0, s.Jr[kk * rs + k * cs], HJ[j]);
         HTl += (my_hRT[j] - 1.0) * tball[j];
         dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + (my_hRT[j] - 1.0) * JT[j];
         dDTl += my_c[j] * dcp;
       } else {
         Sk[j] = tball[j] * ctot;
-        for (int jj = 0; jj < ns; ++jj) Sk[j] = fma(s.c[jj], Jrow[jj], Sk[j]);
-        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk], s.Jr[kk * ld + k], HJ[j]);
+        for (int jj = 0; jj < ns; ++jj) Sk[j] = fma(s.c[jj], Jrow[jj * cs], Sk[j]);
+        for (int kk = 0; kk < ns; ++kk) HJ[j] = fma(s.hRT[kk], s.Jr[kk * rs + k * cs], HJ[j]);
         HTl = fma(my_hRT[j], tball[j], HTl);
         HSl = fma(my_hRT[j], Sk[j], HSl);
         dQTl += (my_cpR[j] - my_hRT[j]) * invT * wm[j] + my_hRT[j] * (JT[j] - Sk[j] * invT);
@@ -520,10 +522,10 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   for (int j = 0; j < SPL; ++j) {
     const int k = lane + 32 * j;
     if (k <= ns) {
-      const double* Jrow = s.Jr + k * ld;
+      const double* Jrow = s.Jr + k * rs;
 #pragma unroll 4
       for (int jj = 0; jj < ns; ++jj) {
-        const double v = fma(Wk[j], Jrow[jj], off[j]) * m.invmw[jj];
+        const double v = fma(Wk[j], Jrow[jj * cs], off[j]) * m.invmw[jj];
         dst[(int64_t)jj * dld + k] = k < ns ? v : s.q[jj];
       }
       dst[(int64_t)ns * dld + k] = k < ns ? last[j] : JTT;
