@@ -43,17 +43,22 @@ from flint_gb300 import dist as fdist  # noqa: E402
 CELLS = 262144
 METRIC = "cell-steps/s on 1 GB300: surrogate+fallback vs plain FP64 at stated T/Y error"
 # FP64 FLOPs per kinetics evaluation (2 x DFMA + DADD + DMUL thread instructions,
-# predicated on) of the warp kernels, per state: k_wdot_warp<0> for one RHS and
-# k_wdot_warp<1> for one Jacobian, from ncu on the c2-wdot / c2-wdotjac and
-# c5-wdot / c5-wdotjac workloads (profiles/fp64_ops_per_state.md).
-KINETICS_FLOPS = {"synthetic-31sp-160r": {"rhs": 18800.0, "jac": 40686.0},
-                  "synthetic-54sp-320r": {"rhs": 31720.0, "jac": 82537.0}}
+# predicated on) of the kernels, per state: k_wdot_warp without and with the
+# Jacobian (a right-hand side and a Jacobian of the reactor) and k_wdot_cell, from
+# ncu on the c2-wdot / c2-wdotjac and c5-wdot / c5-wdotjac workloads
+# (profiles/fp64_ops_per_state.md).  Exponents, exponentials, logarithms and
+# polynomials run on the integer pipes and are not in them.
+KINETICS_FLOPS = {"synthetic-31sp-160r": {"rhs": 3534.0, "jac": 22575.0, "cell": 2638.0},
+                  "synthetic-54sp-320r": {"rhs": 6480.0, "jac": 50216.0}}
+# The generated kernels do all of it in FP64, as the FP64 form of the warp kernels.
+GENERATED_FLOPS = {"synthetic-31sp-160r": {"rhs": 18800.0, "jac": 40686.0},
+                   "synthetic-54sp-320r": {"rhs": 31720.0, "jac": 82537.0}}
 
 
 # DRAM bytes (read + write) per cell of one k_reactor launch, from ncu
-# (profiles/k_reactor_c3_8192cells.md: 2.70 MB for 8,192 cells of the
+# (profiles/k_reactor_c3_8192cells.md: 152 MB for 8,192 cells of the
 # 31-species workload); the traffic field scales it by the launch's cells.
-REACTOR_DRAM_BYTES_PER_CELL = {"synthetic-31sp-160r": 2.699264e6 / 8192}
+REACTOR_DRAM_BYTES_PER_CELL = {"synthetic-31sp-160r": 152.4e6 / 8192}
 
 
 def fp64_ops(ev, ns, mech_name="synthetic-31sp-160r"):
@@ -686,13 +691,15 @@ def run_kernel_workload(args):
     nv = chem.ns + 1
     bytes_per_state = 8 * (2 + 2 * chem.ns) + (8 * nv * nv if jac is not None else 16)
     roof = None
-    kf = KINETICS_FLOPS.get(chem.mech.name)
+    kf = (GENERATED_FLOPS if gen else KINETICS_FLOPS).get(chem.mech.name)
     if kf is not None and tab is None:
-        fl = kf["jac" if jac is not None else "rhs"]
+        cell = jac is None and "cell" in kf and n >= 32768
+        fl = kf["jac" if jac is not None else "cell" if cell else "rhs"]
         peak = chem_peak_fp64()
         roof = {"bound": "fp64", "kernel": (f"ytf_<mech>_{'jac_' if jac is not None else ''}kernel" if gen else
-                                            f"k_wdot_warp<{int(jac is not None)}>"),
-                "flops_note": "the data-driven kernel's FP64 operations per state, for both kernels",
+                                            "k_wdot_cell" if cell else f"k_wdot_warp<{int(jac is not None)}>"),
+                "flops_note": ("the FP64 path's operations per state" if gen else
+                               "FP64 operations per state (exponentials and polynomials are integer work)"),
                 "flops_per_state": fl, "achieved": n * fl / t / 1e12, "peak": peak, "unit": "TFLOP/s",
                 "frac": (n * fl / t / 1e12) / peak if peak else None,
                 "peak_source": "DFMA probe kernel measured in this run",

@@ -6,7 +6,7 @@
 // owns a cell and every lane of an FP64 instruction does needed work: 4 products
 // and 4 multiply-adds per reversible reaction.  31 species, 160 reactions: 53
 // FP64 warp instructions per cell (ncu) where the warp kernel takes 132; 1 M cells
-// with cp and h 4.57 ms against 8.0, 66 % of the FP64 pipe.  Of that the 142
+// with cp and h 4.6 ms against 6.1, 66 % of the FP64 pipe.  Of that the 142
 // plain reactions are 2.2 ms (86 % of the pipe), the 18 third-body and falloff
 // ones 1.1, cp and h 0.4 and loads, concentrations and Gibbs exponents 0.9.
 //
@@ -14,8 +14,9 @@
 // sum of every species of its 32 cells in shared memory, one row per species
 // (CELL_ROW doubles), so that a lane's own values are conflict-free and a
 // row-contiguous transfer to or from global memory (cell-major arrays) is too.
-// 8 warps per SM at 31 species; the reactions' data are broadcast reads.  Two plain reactions are evaluated side by side, for want of warps to
-// hide the integer chains behind.
+// 8 warps per SM at 31 species; the reactions' data are broadcast reads.  Two plain
+// reactions are evaluated side by side, for want of warps to hide the integer chains
+// behind.
 //
 // A cell whose temperature the fixed-point path does not cover is evaluated by
 // its warp afterwards, on the FP64 path, with the warp's columns as scratch.
@@ -289,9 +290,9 @@ static int cell_warps(const ImageLayout& L, int staged) {
 // reactions takes about the same time for one cell as for 32 (31 species, 160
 // reactions: 121 us with four warps on an SM, 145 with eight), so each round of
 // warps has to bring enough cells: as many as the warp-per-cell kernel does in that
-// time, about 145 per SM (measured, thread against warp: 20,000 cells 136 against
+// time, about 145 per SM (thread against warp: 20,000 cells 136 against
 // 125 us, 24,000 136 against 146, 32,000 145 against 193; 197 reactions: 20,000 167
-// against 152, 24,000 167 against 177).  At 1 M cells it takes 4.5 ms against 6.1.
+// against 152, 24,000 167 against 177).  At 1 M cells it takes 4.6 ms against 6.1.
 // With 4 resident warps (54 species) there is too little to hide latencies
 // behind (100,003 cells: 1.37 ms against 1.28 with the warp kernel of that time), so
 // six or more are asked for.

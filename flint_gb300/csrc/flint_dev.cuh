@@ -7,6 +7,9 @@
 // block in shared memory as structure-of-arrays so that the 32 lanes of a
 // round read 32 consecutive words (no bank conflicts).
 //
+// The kinetics here are the FP64 path: of mechanisms and cells that the fixed-point
+// one (flint_fixkin.cuh) does not cover.  The image holds both forms.
+//
 // Math follows FLINT's chemistry path (paths within the FLINT project):
 //   rates of progress, third body, species sums  src/lib/Lib_Chemistry_wdot.f90:96-220
 //   Lindemann / Troe blending, f_F              src/lib/Lib_Chemistry_falloff.f90:12-80

@@ -1,14 +1,17 @@
 // flint_kernels.cu -- batched source-term, Jacobian and thermo kernels.
 //
 //  k_wdot_small   one thread per cell, for small mechanisms (ns <= 16): the
-//                 2-step CH4/air case.  Mechanism staged in shared memory;
-//                 every thread reads the same reaction word at the same time
-//                 (broadcast), per-thread species arrays live in shared memory
-//                 as [species][thread] (conflict-free).
+//                 2-step CH4/air case.  Every thread reads the same reaction
+//                 word at the same time (broadcast), per-thread species arrays
+//                 live in shared memory as [species][thread] (conflict-free).
+//                 k_wdot_small_fix on the fixed-point image, k_wdot_small in
+//                 FP64 for a mechanism without one.
 //  k_wdot_warp    one warp per cell (ns <= 63, species k on lane k % 32): reaction-parallel rates of
 //                 progress, species-parallel sums; optional analytic Jacobian
-//                 written coalesced (lane = row, one column per store).
-//  k_rhs_warp     constant-pressure reactor right-hand side.
+//                 written coalesced (lane = row, one column per store); FIX: on
+//                 the fixed-point image (flint_fixkin.cuh); RHS: the reactor's
+//                 right-hand side.  Source terms of large batches go to
+//                 flint_cell.cu.
 //
 // All kernels are grid-stride loops over cells sized to whole waves of the 152
 // SMs, so any N (including 0 and ragged tails) is handled without a tail kernel.

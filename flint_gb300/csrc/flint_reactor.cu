@@ -6,7 +6,7 @@
 // finite differences.
 //
 // Execution model: one warp integrates one cell; component i of the state
-// x = (Y_0..Y_{ns-1}, T) lives on lane i (ns + 1 <= 32).  The kernel is
+// x = (Y_0..Y_{ns-1}, T) lives on lane i % 32 (ns <= 63).  The kernel is
 // persistent (one wave of blocks) and warps fetch the next cell from a global
 // atomic counter, so cells with very uneven step counts keep every warp busy.
 // Every decision (step size, order, convergence) is made from warp-reduced
