@@ -218,7 +218,8 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
   const int NF = m.nfall, f0 = m.nr - NF;
   double* fo = JAC ? s.Jr : s.fo;
   // third-body concentrations, each row once, kept in the rate's place until the
-  // rate itself is known
+  // rate itself is known; formed on one lane and read on another, so a barrier lies
+  // between: the falloff passes' first one or, without falloff reactions, the else's
   for (int t = lane; t < m.ntb; t += WARP) s.q[m.nr - m.ntb + t] = fix_tb_conc(m, t, ctot, s.c);
   if (NF > 0) {
     const double Tinv = JAC ? invT : fix2d((int64_t)f.v, 70);
@@ -294,6 +295,8 @@ __device__ __forceinline__ void kinetics_fix(const FixView& m, const uint8_t* __
         fo[7 * WARP + lane] = kinf * Fb * iopr * (iopr + Gf) * kratio;
       }
     }
+    __syncwarp();
+  } else {
     __syncwarp();
   }
   // ---- reactions: rates of progress
