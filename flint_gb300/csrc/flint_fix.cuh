@@ -125,13 +125,15 @@ __host__ __device__ __forceinline__ int64_t log2_q52(double x, const uint64_t* _
   return ((int64_t)e << 52) + ((f + 512) >> 10);
 }
 
-// A fixed-point value (q fraction bits) as the nearest double.
+// A fixed-point value (q fraction bits) as the nearest double.  The rounding bit is
+// added after the shift: before it the sum of a value just below a power of two would
+// leave the 64 bits, and its carry is the next exponent.
 __host__ __device__ __forceinline__ double fix2d(int64_t X, int q) {
   const uint64_t sgn = (uint64_t)X & 0x8000000000000000ull;
   uint64_t m = (uint64_t)(X < 0 ? -X : X);
   const int lz = clz64(m);
   m = (lz < 64) ? m << lz : 0;
-  const int64_t bits = ((int64_t)(1023 + 62 - lz - q) << 52) + (int64_t)((m + 1024) >> 11);
+  const int64_t bits = ((int64_t)(1023 + 62 - lz - q) << 52) + (int64_t)((m >> 11) + ((m >> 10) & 1));
   return X == 0 ? 0.0 : bits_d((int64_t)((uint64_t)bits | sgn));
 }
 
