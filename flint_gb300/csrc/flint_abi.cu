@@ -245,7 +245,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
       rs.clear();
       for (int s = 0; s < 3; ++s)
         if (d->rsp[3 * r + s] >= 0 && d->rord[3 * r + s] != 0.0) {
-          ordq[(int)rs.size() * P + rr] = (uint64_t)llrintl(ldexpl((ld)d->rord[3 * r + s], 60));
+          // (below 16 = 2^64 in Q60: beyond the signed range from 8 on)
+          ordq[(int)rs.size() * P + rr] = (uint64_t)(ldexpl((ld)d->rord[3 * r + s], 60) + 0.5L);
           rs.push_back(d->rsp[3 * r + s]);
         }
       powers = power = true;

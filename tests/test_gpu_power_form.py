@@ -1,0 +1,53 @@
+"""Orders in power form (small mechanisms, fixed-point image) against the oracle.
+
+An irreversible reaction whose orders are not 0 to 3 is evaluated as one
+exponential of log2 k + sum of order x log2 c, for orders up to 16.
+Bar as in test_gpu_parity.py: 1e-12 of the sum of absolute terms; an exponent's
+error is at most 16 x 2^-52 (three roundings of a concentration times the order),
+which leaves two decades.
+"""
+import numpy as np
+import pytest
+
+from flint_gb300 import mechgen
+from flint_gb300.api import Chemistry
+from oracle.oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+BAR = 1e-12
+N = 700
+
+
+def states(m, seed):
+    rng = np.random.default_rng(seed)
+    T = rng.uniform(600.0, 2500.0, N)
+    p = rng.uniform(1.0, 20.0, N) * 101325.0
+    Y = rng.dirichlet(np.full(m.ns, 0.5), size=N)
+    return T, p, np.ascontiguousarray(Y)
+
+
+def compare(m, T, p, Y):
+    """wdot and chemistry_source against the oracle."""
+    chem, orc = Chemistry(m), Oracle(m)
+    w_o, ws_o, _, _ = orc.wdot_batch(T, p, Y)
+    w_o, ws_o = w_o.reshape(N, -1), ws_o.reshape(N, -1)
+    Tt, pt, Yt = (torch.from_numpy(a).cuda() for a in (T, p, Y))
+    w = chem.wdot(Tt, pt, Yt)[0].cpu().numpy()
+    W = np.array([s.mw for s in m.species])
+    rho = p / (m.r_eos * T * (Y / W).sum(1))
+    s = chem.chemistry_source(torch.from_numpy(rho[:, None] * Y).cuda(), Tt).cpu().numpy()
+    assert np.isfinite(w_o).all()
+    assert (np.abs(w - w_o) / (ws_o + 1e-300)).max() < BAR
+    # (a concentration formed from rho Y differs by two roundings from the oracle's)
+    assert (np.abs(s - w_o) / (ws_o + 1e-300)).max() < 1e-11
+    return w
+
+
+@pytest.mark.parametrize("order", [0.5, 7.9, 8.0, 8.5, 12.5, 15.9, 16.0, 20.0])
+def test_orders(order):
+    m = mechgen.load("c1")
+    m.reactions[0].orders = {"CH4": 1.0, "O2": order}
+    T, p, Y = states(m, 11)
+    compare(m, T, p, Y)
