@@ -275,7 +275,8 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
         for (int e = m.tbp[row]; e < m.tbp[row + 1]; ++e) M = fma(m.tbv[e], cs[m.tbs[e] * S], M);
       }
       double kf;
-      if (type < 2) kf = none ? 0.0 : exp2_q52(a, m.et);
+      if (none) kf = 0.0;      // (of any type: the absent factor is not in the exponent)
+      else if (type < 2) kf = exp2_q52(a, m.et);
       else kf = cell_falloff(m, r - f0, type, a, M, f, T, fix2d((int64_t)f.v, 70));
       const int sgn = ((int)(w >> 43) & 1) << 31;
       kf = __hiloint2double(__double2hiint(kf) ^ sgn, __double2loint(kf));

@@ -1,7 +1,8 @@
 """Orders in power form (small mechanisms, fixed-point image) against the oracle.
 
 An irreversible reaction whose orders are not 0 to 3 is evaluated as one
-exponential of log2 k + sum of order x log2 c, for orders up to 16.
+exponential of log2 k + sum of order x log2 c, for orders up to 16.  Falloff and
+three-body reactions in that form, also with the reactant absent.
 Bar as in test_gpu_parity.py: 1e-12 of the sum of absolute terms; an exponent's
 error is at most 16 x 2^-52 (three roundings of a concentration times the order),
 which leaves two decades.
@@ -51,3 +52,17 @@ def test_orders(order):
     m.reactions[0].orders = {"CH4": 1.0, "O2": order}
     T, p, Y = states(m, 11)
     compare(m, T, p, Y)
+
+
+@pytest.mark.parametrize("rtype", [1, 2, 3])
+def test_absent_reactant(rtype):
+    m = mechgen.load("c1")
+    r = m.reactions[0]
+    r.rtype, r.efficiencies, r.default_eff = rtype, {"H2O": 6.0}, 1.0
+    r.A0, r.b0, r.EaR0 = r.A * 50.0, r.b, r.EaR * 0.9
+    r.troe = [0.6, 100.0, 2000.0, 5000.0] if rtype == 3 else None
+    T, p, Y = states(m, 12)
+    Y[::3, m.index("CH4")] = 0.0
+    w = compare(m, T, p, Y)
+    # CH4 takes part in the first reaction alone
+    assert (w[::3, m.index("CH4")] == 0.0).all() and (w[1::3, m.index("CH4")] != 0.0).any()
