@@ -137,7 +137,8 @@ static int plain_class(const flint_mech_desc* d, int r) {
 // three concentrations a side (with the reverse Gibbs sum over the same
 // factors; irreversible reactions of up to 16 species may have any orders, which
 // only the small-mechanism kernel takes: sfix without fix), non-zero A, and every coefficient and exponent within its format
-// from fix_Tlo <= 600 K up to fix_Thi >= 3000 K.  Coefficients are formed in long double.
+// from fix_Tlo <= 600 K up to fix_Thi >= 3000 K (what the concentrations add to a power
+// form's exponent is bounded by the kernel).  Coefficients are formed in long double.
 static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, ImageLayout& L,
                      std::vector<uint8_t>& img) {
   typedef long double ld;

@@ -236,6 +236,8 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
       double Pf = 1.0;
       bool none = false;
       if (fix_power(w)) {
+        // the sum modulo 2^64 and, against leaving the format, in Q32
+        int64_t wide = a >> 20;
 #pragma unroll
         for (int sl = 0; sl < 3; ++sl) {
           const int s = fix_idx(w, sl);
@@ -258,9 +260,16 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
             ls[s * S] = l;
           }
           const uint64_t o = m.ord[sl * P + r];
-          if (l == 1) none = true;
-          else a += (int64_t)(mulhi_u(o, l) - (o >> 1)) >> 1;      // Q60 x Q57 -> Q53 -> Q52
+          if (l == 1) {
+            none = true;
+          } else {
+            const int64_t x = (int64_t)(mulhi_u(o, l) - (o >> 1));      // Q60 x Q57 -> Q53
+            a += x >> 1;
+            wide += x >> 21;
+          }
         }
+        if (wide >= 2040ll << 32) a = 2040ll << 52;
+        if (wide <= -(2040ll << 32)) a = -(2040ll << 52);
       } else {
 #pragma unroll
         for (int sl = 0; sl < 3; ++sl) {

@@ -2,7 +2,9 @@
 
 An irreversible reaction whose orders are not 0 to 3 is evaluated as one
 exponential of log2 k + sum of order x log2 c, for orders up to 16.  Falloff and
-three-body reactions in that form, also with the reactant absent.
+three-body reactions in that form, also with the reactant absent, and orders with
+concentrations so small that the sum leaves the format's 2^11 octaves.
+
 Bar as in test_gpu_parity.py: 1e-12 of the sum of absolute terms; an exponent's
 error is at most 16 x 2^-52 (three roundings of a concentration times the order),
 which leaves two decades.
@@ -66,3 +68,14 @@ def test_absent_reactant(rtype):
     w = compare(m, T, p, Y)
     # CH4 takes part in the first reaction alone
     assert (w[::3, m.index("CH4")] == 0.0).all() and (w[1::3, m.index("CH4")] != 0.0).any()
+
+
+@pytest.mark.parametrize("order,trace", [(15.0, 1e-17), (15.9, 1e-16), (11.0, 1e-17), (4.5, 1e-17)])
+def test_exponent_beyond_the_format(order, trace):
+    """Three factors of large order at trace concentrations: the rate vanishes."""
+    m = mechgen.load("c1")
+    m.reactions[0].orders = {"CH4": order, "O2": order, "N2": order}
+    T, p, Y = states(m, 13)
+    for s in ("CH4", "O2", "N2"):
+        Y[::2, m.index(s)] = trace * (1.0 + np.arange(Y[::2].shape[0]) / N)
+    compare(m, T, p, Y)
