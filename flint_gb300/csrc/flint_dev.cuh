@@ -38,7 +38,7 @@ __host__ __device__ inline int rx_ordcode(uint32_t w, int s) { return (w >> (16 
 // Offsets (in bytes) of each section of the packed image.  All sections are
 // 16-byte aligned; the image is copied to shared memory with 16-byte loads.
 struct ImageLayout {
-  int ns, nr, nrpad, nsp;        // nsp = species padded to a multiple of 32
+  int ns, nr, nrpad, nsp;        // nsp = unknowns (species and T) padded to a multiple of 32
   int ntb;                       // rows of third-body efficiencies
   int nlist;                     // CSR entries (species -> reactions)
   int bytes;                     // total image size

@@ -328,7 +328,7 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
 
 // ---------------------------------------------------------------- warp
 // SPL species per lane; GJ: the Jacobian work area is a per-warp slot of
-// global memory (mechanisms of 33-63 species, and smaller ones whose shared
+// global memory (mechanisms of 32-63 species, and smaller ones whose shared
 // memory layout would not fit a block).  FIX: the fixed-point kinetics
 // (flint_fixkin.cuh); the block then stages only that image.  RHS: rhs_out is
 // wanted.
@@ -630,7 +630,7 @@ static int64_t grid_for(const void* fn, int threads, size_t smem, int64_t work_i
 }
 
 size_t small_smem(const ImageLayout& L) { return L.bytes + 3 * SMALL_NSMAX * SMALL_THREADS * sizeof(double); }
-// Jacobian work area in global memory: 33-63 species, or a shared-memory
+// Jacobian work area in global memory: 32-63 species, or a shared-memory
 // layout too large for a block of 256 threads (the choice does not depend on
 // the block size a caller tunes, so one kernel serves every block size).
 // The image a block of the warp kernels stages.
