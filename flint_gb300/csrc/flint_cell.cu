@@ -230,6 +230,7 @@ k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
       }
     }
     // ---- outputs
+    unsigned left = __ballot_sync(FULL, lane < nc && !in);
     if (RHS) {
       // dT/dt = -T sum_k (h_k/RT) w_k / sum_k c_k cp_k/R (u and cv at constant volume)
       double Q = 0.0;
@@ -251,8 +252,9 @@ k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
         if (cpo) cpo[cell] = cpm * m.r_thermo;
         if (ho) ho[cell] = hm * m.r_thermo * Ts;
       }
+      // (cells left to the FP64 path keep their row: it may hold their Y still)
       if (layout == 1) {
-        if (lane < nc)
+        if (lane < nc && in)
           for (int k = 0; k < ns; ++k) out[(int64_t)k * n + cell] = w[k * CELL_ROW];
       } else {
         __syncwarp();
@@ -261,14 +263,13 @@ k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
         int row = 0, k = lane;
         while (k >= ns) { k -= ns; ++row; }
         for (int i = lane; i < nc * ns; i += 32) {
-          dst[i] = wr[k * CELL_ROW + row];
+          if (!(left >> row & 1u)) dst[i] = wr[k * CELL_ROW + row];
           k += 32;
           while (k >= ns) { k -= ns; ++row; }
         }
       }
     }
     // ---- cells outside the fixed-point range: the whole warp, one at a time
-    unsigned left = __ballot_sync(FULL, lane < nc && !in);
     while (left) {
       const int64_t ci = c0 + (__ffs(left) - 1);
       left &= left - 1;
