@@ -480,7 +480,13 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
         ++ri;
       }
     }
-    if (fits) L.term_len = len;
+    if (fits) {
+      L.term_len = len;
+    } else {   // the Jacobian takes the FP64 path
+      term.clear();
+      target.clear();
+      coef.resize(1);
+    }
   }
   // ---- sections
   int off = 0;

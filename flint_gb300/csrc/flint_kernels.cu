@@ -630,13 +630,24 @@ static int64_t grid_for(const void* fn, int threads, size_t smem, int64_t work_i
 }
 
 size_t small_smem(const ImageLayout& L) { return L.bytes + 3 * SMALL_NSMAX * SMALL_THREADS * sizeof(double); }
+// Whether a launch of the warp kernels takes the fixed-point form.  A Jacobian takes
+// it where the mechanism's term lists were packed and the image with them leaves a
+// block of 256 threads room, or where the FP64 image does not either: the lists grow
+// with reactions x species x third-body efficiencies (255 three-body reactions of 20
+// efficiencies each: 233 KB, the FP64 image 139).
+static bool use_fix(const ImageLayout& L, bool jac) {
+  if (!L.fix || !jac) return L.fix;
+  const size_t warps = (WARP_THREADS / 32) * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
+  const bool fp64_fits = L.bytes + warps <= device_smem_optin();
+  return !fp64_fits || (L.term_len > 0 && L.fix_bytes + warps <= device_smem_optin());
+}
+// The image a block of the warp kernels stages.
+static size_t image_bytes(const ImageLayout& L, bool jac) {
+  return use_fix(L, jac) ? (jac ? L.fix_bytes : L.fix_bytes_rate) : L.bytes;
+}
 // Jacobian work area in global memory: 32-63 species, or a shared-memory
 // layout too large for a block of 256 threads (the choice does not depend on
 // the block size a caller tunes, so one kernel serves every block size).
-// The image a block of the warp kernels stages.
-static size_t image_bytes(const ImageLayout& L, bool jac) {
-  return L.fix ? (jac ? L.fix_bytes : L.fix_bytes_rate) : L.bytes;
-}
 static bool warp_gj(const ImageLayout& L, bool jac) {
   if (L.nsp > 32) return true;
   if (!jac) return false;
@@ -662,9 +673,10 @@ typedef void (*WarpKernel)(const uint8_t*, ImageLayout, int64_t, int, const doub
 
 template <bool JAC, bool RHS>
 static WarpKernel warp_fn(const ImageLayout& L) {
-  if (L.nsp > 32) return L.fix ? k_wdot_warp<JAC, 2, true, true, RHS> : k_wdot_warp<JAC, 2, true, false, RHS>;
-  if (JAC && warp_gj(L, JAC)) return L.fix ? k_wdot_warp<JAC, 1, true, true, RHS> : k_wdot_warp<JAC, 1, true, false, RHS>;
-  return L.fix ? k_wdot_warp<JAC, 1, false, true, RHS> : k_wdot_warp<JAC, 1, false, false, RHS>;
+  const bool fix = use_fix(L, JAC);
+  if (L.nsp > 32) return fix ? k_wdot_warp<JAC, 2, true, true, RHS> : k_wdot_warp<JAC, 2, true, false, RHS>;
+  if (JAC && warp_gj(L, JAC)) return fix ? k_wdot_warp<JAC, 1, true, true, RHS> : k_wdot_warp<JAC, 1, true, false, RHS>;
+  return fix ? k_wdot_warp<JAC, 1, false, true, RHS> : k_wdot_warp<JAC, 1, false, false, RHS>;
 }
 
 // Global Jacobian work area needed by the warp kernels (doubles), for a grid
