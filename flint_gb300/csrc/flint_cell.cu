@@ -299,7 +299,7 @@ static int cell_warps(const ImageLayout& L, int staged) {
 // six or more are asked for.
 bool use_cell_kernel(const ImageLayout& L, int64_t n) {
   const int64_t sms = device_sms(), w = cell_warps(L, L.fix_bytes_cell);
-  if (!L.fix || w < 6 || scratch_small_doubles(L.nsp, L.nrpad) > cell_warp_doubles(L.ns)) return false;
+  if (!L.fix || w < 6 || scratch_small_doubles(L) > cell_warp_doubles(L.ns)) return false;
   const int64_t rounds = (n + 32 * w * sms - 1) / (32 * w * sms);
   return n >= 145 * sms * rounds;
 }

@@ -354,7 +354,7 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
     const int sd = scratch_doubles(L, JAC);
     s = carve(reinterpret_cast<double*>(smem + base) + wid * sd, L, JAC);
   } else {
-    const int sd = scratch_small_doubles(nsp, nrpad);
+    const int sd = scratch_small_doubles(L);
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
     s = carve2(reinterpret_cast<double*>(smem + base) + wid * sd,
                JAC ? gscratch + gw * scratch_jac_doubles(L) : nullptr, L);
@@ -637,7 +637,7 @@ size_t small_smem(const ImageLayout& L) { return L.bytes + 3 * SMALL_NSMAX * SMA
 // efficiencies each: 233 KB, the FP64 image 139).
 static bool use_fix(const ImageLayout& L, bool jac) {
   if (!L.fix || !jac) return L.fix;
-  const size_t warps = (WARP_THREADS / 32) * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
+  const size_t warps = (WARP_THREADS / 32) * scratch_small_doubles(L) * sizeof(double);
   const bool fp64_fits = L.bytes + warps <= device_smem_optin();
   return !fp64_fits || (L.term_len > 0 && L.fix_bytes + warps <= device_smem_optin());
 }
@@ -659,7 +659,7 @@ static int warp_block(int threads) { return threads == 64 || threads == 128 ? th
 
 size_t warp_smem(const ImageLayout& L, bool jac, int threads) {
   const int wpb = warp_block(threads) / 32;
-  if (warp_gj(L, jac)) return image_bytes(L, jac) + wpb * scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double);
+  if (warp_gj(L, jac)) return image_bytes(L, jac) + wpb * scratch_small_doubles(L) * sizeof(double);
   return image_bytes(L, jac) + wpb * scratch_doubles(L, jac) * sizeof(double);
 }
 

@@ -363,7 +363,7 @@ constexpr int REACTOR_LAYOUT_WIDE = 100, REACTOR_LAYOUT_NARROW = 101;
 constexpr int WIDE_THREADS = 384;
 
 static size_t wide_warp_doubles(const ImageLayout& L) {
-  return scratch_small_doubles(L.nsp, L.nrpad) + (((L.nsp + 1) * (L.nsp + 1) + 1) & ~1);
+  return scratch_small_doubles(L) + (((L.nsp + 1) * (L.nsp + 1) + 1) & ~1);
 }
 static size_t wide_smem(const ImageLayout& L) {
   return staged_bytes(L) + (WIDE_THREADS / 32) * (wide_warp_doubles(L) * sizeof(double) + 64 * sizeof(int));
@@ -471,7 +471,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
   WarpScratch s;
   int* pivs;
   if (WIDE) {
-    const int small = scratch_small_doubles(nsp, nrpad), sd = small + (((nsp + 1) * (nsp + 1) + 1) & ~1);
+    const int small = scratch_small_doubles(L), sd = small + (((nsp + 1) * (nsp + 1) + 1) & ~1);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
     s = carve2(wbase, Jg + JW * JW, L);
     s.Jr = wbase + small;
@@ -482,7 +482,7 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
     s = carve(wbase, L, true);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
   } else {
-    const int sd = scratch_small_doubles(nsp, nrpad);
+    const int sd = scratch_small_doubles(L);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
     s = carve2(wbase, Jg + JW * JW, L);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64 * SPL;
@@ -803,7 +803,7 @@ size_t reactor_smem(const ImageLayout& L, int layout = REACTOR_LAYOUT_AUTO) {
   if (layout == REACTOR_LAYOUT_WIDE) return wide_smem(L);
   if (!reactor_gj(L, layout)) return reactor_smem_spl1(L);
   return staged_bytes(L) + (reactor_threads(layout) / 32) *
-                       (scratch_small_doubles(L.nsp, L.nrpad) * sizeof(double) + 64 * spl_of(L) * sizeof(int));
+                       (scratch_small_doubles(L) * sizeof(double) + 64 * spl_of(L) * sizeof(int));
 }
 
 typedef void (*ReactorKernel)(const uint8_t*, ImageLayout, int64_t, double*, const double*, double*, const double*,

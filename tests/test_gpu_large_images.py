@@ -2,7 +2,8 @@
 FP64 image staged they accept with the fixed-point one.
 
 * 255 three-body reactions with 20 efficiencies each: the Jacobian's term lists grow
-  with reactions x species x efficiencies and leave no room in a block.
+  with reactions x species x efficiencies and leave no room in a block;
+* an FP64 image that leaves its block next to nothing.
 """
 import copy
 
@@ -48,3 +49,31 @@ def test_jacobian_of_many_third_bodies(per_reaction):
     assert (np.abs(J.cpu().numpy().reshape(n, -1) - J_o.reshape(n, -1)) / (Js_o.reshape(n, -1) + 1e-300)).max() < 1e-12
     _, ws_o, _, _ = Oracle(m).wdot_batch(T, p, Y)
     assert (np.abs(w.cpu().numpy().reshape(n, -1) - w_o.reshape(n, -1)) / (ws_o.reshape(n, -1) + 1e-300)).max() < 1e-12
+
+
+def test_fp64_image_at_the_limit():
+    """608 reactions on NASA-9 thermo: image and scratch fill a block's 227 KB but for
+    less than 384 bytes."""
+    m = mechgen.load("c2")
+    for s in m.species:
+        s.nasa9 = [[s.tlow, s.tmid, 0.0, 0.0] + list(s.low), [s.tmid, s.thigh, 0.0, 0.0] + list(s.high)]
+    plain = [r for r in m.reactions if r.rtype == 0]
+    while m.nr < 608:
+        m.reactions.append(copy.deepcopy(plain[m.nr % len(plain)]))
+    three = [r for r in m.reactions if r.rtype == 1]
+    for r in three:
+        r.efficiencies = {}
+    for i in range(298):
+        three[i // 30].efficiencies[m.species[i % 30].name] = 1.5 + i
+    n = 200
+    T, p, Y = mechgen.c2_states(n, m, seed=22)
+    w_o, ws_o, _, _ = Oracle(m).wdot_batch(T, p, Y)
+    Tt, pt, Yt = (torch.from_numpy(a).cuda() for a in (T, p, Y))
+    chem = Chemistry(m)
+    w = chem.wdot(Tt, pt, Yt)[0].cpu().numpy()
+    f = chem.rhs(Tt, pt, Yt).cpu().numpy()
+    W = np.array([s.mw for s in m.species])
+    rho = p / (m.r_eos * T * (Y / W).sum(1))
+    scale = ws_o.reshape(n, -1) + 1e-300
+    assert (np.abs(w - w_o.reshape(n, -1)) / scale).max() < 1e-12
+    assert (np.abs(f[:, :-1] * rho[:, None] - w_o.reshape(n, -1)) / scale).max() < 1e-12
