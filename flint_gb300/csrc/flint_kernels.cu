@@ -169,8 +169,8 @@ __device__ __noinline__ void small_cell_general(const uint8_t* __restrict__ img,
 // pipe (concentrations, sums, cp and h) where it took about 300, half of them
 // logarithms and exponentials.  The mechanism's few words are read through the
 // read-only cache: staging them cost a block more than they are worth.  A thread
-// whose temperature or concentrations leave the formats (2^-64 <= c < 2^63 for a
-// factor in power form, or c = 0) takes the FP64 path.
+// whose temperature leaves the formats, or a concentration in power form the normal
+// range (subnormal, inf or NaN), takes the FP64 path.
 __global__ void __launch_bounds__(SMALL_THREADS)
 k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L, int64_t n, int layout,
                  const double* __restrict__ Tg, const double* __restrict__ pg, const double* __restrict__ Yg,
@@ -235,6 +235,7 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
       int64_t a = fix_arrhenius(m.a[r], m.b[r], m.e[r], f);
       double Pf = 1.0;
       bool none = false;
+      int minus = 0;             // last bit: the factors' sign
       if (fix_power(w)) {
         // the sum modulo 2^64 and, against leaving the format, in Q32
         int64_t wide = a >> 20;
@@ -242,31 +243,33 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
         for (int sl = 0; sl < 3; ++sl) {
           const int s = fix_idx(w, sl);
           if (s >= ns) continue;
+          const double c = cs[s * S];
           uint64_t l = ls[s * S];
           if (l == 0) {
-            // log2 c in Q57, sign flipped
-            const double c = cs[s * S];
-            const unsigned e = (unsigned)(__double2hiint(c) >> 20);     // sign and exponent
-            if (e - 960u < 126u) {
+            // log2 |c| with its sign flipped: Q57 (last bit 0) from 2^-63 to 2^63, Q53
+            // (last bit 1) beyond; 1 where c = 0
+            const unsigned e = (unsigned)(__double2hiint(c) >> 20) & 0x7ffu;
+            l = 1;
+            if (e - 1u < 0x7feu) {
               int ex;
-              const int64_t fr = log2_q62(c, m.lt, &ex);
-              l = ((((uint64_t)(int64_t)ex) << 57) + (uint64_t)(fr >> 5)) ^ 0x8000000000000000ull;
-            } else if ((__double_as_longlong(c) << 1) == 0) {
-              l = 1;     // c = 0
-            } else {
+              const int64_t fr = log2_q62(fabs(c), m.lt, &ex);
+              l = e - 960u < 126u ? (((uint64_t)(int64_t)ex << 57) + ((uint64_t)fr >> 6 << 1)) ^ 0x8000000000000000ull
+                                  : ((((uint64_t)(int64_t)ex << 53) + ((uint64_t)fr >> 9)) ^ 0x8000000000000000ull) | 1u;
+            } else if ((__double_as_longlong(c) << 1) != 0) {
               in = false;
-              l = 1;
             }
             ls[s * S] = l;
           }
           const uint64_t o = m.ord[sl * P + r];
-          if (l == 1) {
-            none = true;
-          } else {
-            const int64_t x = (int64_t)(mulhi_u(o, l) - (o >> 1));      // Q60 x Q57 -> Q53
-            a += x >> 1;
-            wide += x >> 21;
+          // a negative c to an order of 1, 2 or 3 has a sign, to any other it is absent
+          none |= l == 1;
+          if (__double2hiint(c) < 0) {
+            none |= (o << 4) != 0 || o >> 60 > 3;
+            minus ^= (int)(o >> 60);
           }
+          const int64_t x = (int64_t)(mulhi_u(o, l) - (o >> 1));      // Q60 x Q57 -> Q53, x Q53 -> Q49
+          a += l & 1 ? (int64_t)((uint64_t)x << 3) : x >> 1;
+          wide += l & 1 ? x >> 17 : x >> 21;
         }
         if (wide >= 2040ll << 32) a = 2040ll << 52;
         if (wide <= -(2040ll << 32)) a = -(2040ll << 52);
@@ -287,7 +290,7 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
       if (none) kf = 0.0;      // (of any type: the absent factor is not in the exponent)
       else if (type < 2) kf = exp2_q52(a, m.et);
       else kf = cell_falloff(m, r - f0, type, a, M, f, T, fix2d((int64_t)f.v, 70));
-      const int sgn = ((int)(w >> 43) & 1) << 31;
+      const int sgn = (((int)(w >> 43) ^ minus) & 1) << 31;
       kf = __hiloint2double(__double2hiint(kf) ^ sgn, __double2loint(kf));
       double q = kf * Pf;
       if (fix_rev(w)) {
