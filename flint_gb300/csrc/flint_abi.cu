@@ -293,8 +293,8 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
   const ld lC = log2l((ld)d->p_ref / (ld)d->r_thermo) - 7.0L;
   if (!(fabsl(lC) < 1000.0L)) ok = false;
   if (!ok) return;
-  // ---- the range of T over which every exponent stays in format (in double:
-  // magnitudes against limits 2 % inside the formats')
+  // ---- the range of T over which every exponent stays in format and every rate
+  // constant normal (in double: magnitudes against limits 2 % inside the formats')
   double Tlo = 1e30;
   const double l2e = (double)LOG2E, lC0 = (double)(lC + 7.0L);
   std::vector<double> g(ns), lA(nr), lA0(nr);
@@ -326,10 +326,14 @@ static void pack_fix(const flint_mech_desc* d, const std::vector<int>& order, Im
         for (int i : lists_r[rr]) v -= g[i];
         v -= ((int)lists_p[rr].size() - (int)lists_r[rr].size()) * (lC0 - lg);
       }
+      // what the kernels take the exponential of: f (alone or, in power form, with more
+      // terms), f + v of a reversible reaction, v and the ratio f0 - f of a falloff one
       in = std::fabs(f) < 2000.0 && std::fabs(v) < 2000.0 && std::fabs(f + v) < 2000.0;
-      if (d->rtype[r] >= 2) {
+      const bool falloff = d->rtype[r] >= 2, power = (ix[rr] >> 46) & 1;
+      in = in && (power || f > -1020.0) && (!d->reversible[r] || (falloff ? v : f + v) > -1020.0);
+      if (falloff) {
         const double f0 = lA0[rr] + d->arrh0[3 * r + 1] * lg - l2e * d->arrh0[3 * r + 2] / T;
-        in = in && std::fabs(f0 - f) < 2000.0;
+        in = in && f0 - f > -1020.0 && f0 - f < 2000.0;
       }
     }
     if (!in) break;

@@ -121,10 +121,11 @@ __device__ __forceinline__ double troe_blend(double Fc, double Pr, const uint64_
 }
 
 // Effective rate coefficient of a falloff reaction (i-th, reaction word w) from
-// its high-pressure limit's exponent xinf (Q52).
+// its high-pressure limit's exponent xinf (Q52; SUB: below the normal range too).
+template <bool SUB = false>
 __device__ __forceinline__ double cell_falloff(const FixView& m, int i, int type, int64_t xinf, double M, const FixT& f,
                                                double T, double Tinv) {
-  const double kinf = exp2_q52(xinf, m.et);
+  const double kinf = exp2_q52<SUB>(xinf, m.et);
   const double kratio = exp2_q52(fix_arrhenius(m.ra[i], m.rb[i], m.re[i], f), m.et);
   const double Pr = kratio * M;
   const double k = kinf * (Pr * recip(1.0 + Pr));

@@ -288,8 +288,8 @@ k_wdot_small_fix(const uint8_t* __restrict__ img, const __grid_constant__ ImageL
       }
       double kf;
       if (none) kf = 0.0;      // (of any type: the absent factor is not in the exponent)
-      else if (type < 2) kf = exp2_q52(a, m.et);
-      else kf = cell_falloff(m, r - f0, type, a, M, f, T, fix2d((int64_t)f.v, 70));
+      else if (type < 2) kf = exp2_q52<true>(a, m.et);
+      else kf = cell_falloff<true>(m, r - f0, type, a, M, f, T, fix2d((int64_t)f.v, 70));
       const int sgn = (((int)(w >> 43) ^ minus) & 1) << 31;
       kf = __hiloint2double(__double2hiint(kf) ^ sgn, __double2loint(kf));
       double q = kf * Pf;

@@ -23,3 +23,8 @@ def values(tmp_path_factory):
 def test_conversion_that_rounds_up_to_a_power_of_two(values):
     assert values["fix2d_carry"] <= 2.0 ** -53
     assert (values["fix2d_one"], values["fix2d_four"], values["fix2d_minus"]) == (1.0, 4.0, -1.0)
+
+
+def test_exp2_below_the_normal_range(values):
+    """Cut to a subnormal number: less than one unit (and 2^-5 of the evaluation's)."""
+    assert values["exp2_subnormal"] <= 1.0 + 2.0 ** -5
