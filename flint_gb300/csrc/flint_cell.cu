@@ -49,7 +49,7 @@ __device__ __noinline__ void cell_general(const uint8_t* __restrict__ img, const
                                           int cv) {
   const int ns = L.ns, nv = ns + 1;
   const double* mw = reinterpret_cast<const double*>(img + L.o_mw);
-  const WarpScratch s = carve2(scratch, nullptr, L);
+  const WarpScratch s = carve2<true>(scratch, nullptr, L);
   double Yk[SPL];
 #pragma unroll
   for (int j = 0; j < SPL; ++j) {
@@ -262,11 +262,16 @@ k_wdot_cell(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
         const double* wr = w - lane;
         int row = 0, k = lane;
         while (k >= ns) { k -= ns; ++row; }
-        for (int i = lane; i < nc * ns; i += 32) {
-          if (!(left >> row & 1u)) dst[i] = wr[k * CELL_ROW + row];
-          k += 32;
-          while (k >= ns) { k -= ns; ++row; }
-        }
+        auto store = [&](bool all) {
+          for (int i = lane; i < nc * ns; i += 32) {
+            if (all || !(left >> row & 1u)) dst[i] = wr[k * CELL_ROW + row];
+            k += 32;
+            while (k >= ns) { k -= ns; ++row; }
+          }
+        };
+        // (the test in the loop of every warp costs 1 M cells 0.9 %)
+        if (left == 0) store(true);
+        else store(false);
       }
     }
     // ---- cells outside the fixed-point range: the whole warp, one at a time

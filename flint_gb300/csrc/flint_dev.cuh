@@ -325,14 +325,16 @@ struct WarpScratch {
 // rates of progress are done).
 // For the fixed-point path c, hRT and gRT have two more entries than species slots: it
 // reads index `dummy` (c = 1, g = 0) for a missing reactant or product.
-__host__ __device__ inline int species_stride(const ImageLayout& L) { return L.nsp + (L.fix ? 2 : 0); }
+// (Kernels know which path they are at compile time: read from the layout it cost the
+// reactor 1 %.)
+__host__ __device__ inline int species_stride(int nsp, bool fix) { return nsp + (fix ? 2 : 0); }
 // Thread-per-cell kernel (flint_cell.cu): a species' row of a warp holds c, g and
 // the production of the warp's 32 cells, each padded to 33 doubles.
 constexpr int CELL_PAD = 33, CELL_ROW = 3 * CELL_PAD;
 // (63 rather than 64 for the larger size: the packed index has 6 bits, and 63 species leave slot 63 free)
 __host__ __device__ inline int fix_dummy(int nsp) { return nsp == 64 ? 63 : nsp; }
 __host__ __device__ inline int scratch_small_doubles(const ImageLayout& L) {
-  return (3 * species_stride(L) + L.nrpad + 8 * 32 + 1) & ~1;   // keep 16-byte alignment
+  return (3 * species_stride(L.nsp, L.fix != 0) + L.nrpad + 8 * 32 + 1) & ~1;   // keep 16-byte alignment
 }
 __host__ __device__ inline int scratch_jac_doubles(const ImageLayout& L) {
   return (L.dq_rows * L.nrpad + (L.nsp + 1) * (L.nsp + 1) + 1) & ~1;
@@ -342,14 +344,15 @@ __host__ __device__ inline int scratch_jac_doubles(const ImageLayout& L) {
 // calls without the Jacobian (in the Jacobian call it lives in Jr), and dq only
 // inside a Jacobian call, so the two may share (dq and Jr together hold 256 doubles).
 __host__ __device__ inline int scratch_doubles(const ImageLayout& L, bool jac) {
-  return jac ? ((3 * species_stride(L) + L.nrpad + scratch_jac_doubles(L) + 1) & ~1)
+  return jac ? ((3 * species_stride(L.nsp, L.fix != 0) + L.nrpad + scratch_jac_doubles(L) + 1) & ~1)
              : scratch_small_doubles(L);
 }
 
+template <bool FIX>
 __device__ inline WarpScratch carve2(double* small, double* jacbuf, const ImageLayout& L) {
   const int nsp = L.nsp, nrpad = L.nrpad;
   WarpScratch s;
-  const int ss = species_stride(L);
+  const int ss = species_stride(nsp, FIX);
   s.c = small; s.hRT = small + ss; s.gRT = small + 2 * ss; s.q = small + 3 * ss;
   s.fo = s.q + nrpad;
   s.ldj = nsp + 1;
@@ -359,8 +362,9 @@ __device__ inline WarpScratch carve2(double* small, double* jacbuf, const ImageL
 }
 
 // Both parts contiguous in one buffer (shared memory, up to 31 species).
+template <bool FIX>
 __device__ inline WarpScratch carve(double* p, const ImageLayout& L, bool jac) {
-  return carve2(p, jac ? p + 3 * species_stride(L) + L.nrpad : nullptr, L);
+  return carve2<FIX>(p, jac ? p + 3 * species_stride(L.nsp, FIX) + L.nrpad : nullptr, L);
 }
 
 // Cell-level results held per lane: lane k (< ns) gets species k, the T-row

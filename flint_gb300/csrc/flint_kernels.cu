@@ -355,11 +355,11 @@ k_wdot_warp(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout
   WarpScratch s;
   if (!GJ) {
     const int sd = scratch_doubles(L, JAC);
-    s = carve(reinterpret_cast<double*>(smem + base) + wid * sd, L, JAC);
+    s = carve<FIX>(reinterpret_cast<double*>(smem + base) + wid * sd, L, JAC);
   } else {
     const int sd = scratch_small_doubles(L);
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + wid;
-    s = carve2(reinterpret_cast<double*>(smem + base) + wid * sd,
+    s = carve2<FIX>(reinterpret_cast<double*>(smem + base) + wid * sd,
                JAC ? gscratch + gw * scratch_jac_doubles(L) : nullptr, L);
   }
   const int ns = L.ns, nv = ns + 1;

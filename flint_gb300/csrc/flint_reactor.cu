@@ -473,18 +473,18 @@ k_reactor(const uint8_t* __restrict__ img, const __grid_constant__ ImageLayout L
   if (WIDE) {
     const int small = scratch_small_doubles(L), sd = small + (((nsp + 1) * (nsp + 1) + 1) & ~1);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
-    s = carve2(wbase, Jg + JW * JW, L);
+    s = carve2<FIX>(wbase, Jg + JW * JW, L);
     s.Jr = wbase + small;
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
   } else if (!GJ) {
     const int sd = scratch_doubles(L, true);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
-    s = carve(wbase, L, true);
+    s = carve<FIX>(wbase, L, true);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64;
   } else {
     const int sd = scratch_small_doubles(L);
     double* wbase = reinterpret_cast<double*>(smem + base) + wid * sd;
-    s = carve2(wbase, Jg + JW * JW, L);
+    s = carve2<FIX>(wbase, Jg + JW * JW, L);
     pivs = reinterpret_cast<int*>(reinterpret_cast<double*>(smem + base) + (blockDim.x >> 5) * sd) + wid * 64 * SPL;
   }
   const int ns = L.ns, nv = ns + 1;
