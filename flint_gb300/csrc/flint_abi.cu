@@ -1353,6 +1353,12 @@ int flint_selftest_log(flint_mech_t h, int64_t n, const double* x, double* y, vo
   return e == cudaSuccess ? FLINT_OK : cuda_fail(e, "flint_selftest_log");
 }
 
+int flint_selftest_recip(int64_t n, const double* x, double* y, void* stream) {
+  if (n < 0 || (n > 0 && (!x || !y))) return fail(FLINT_ERR_ARG, "bad argument");
+  cudaError_t e = launch_recip_selftest(n, x, y, (cudaStream_t)stream);
+  return e == cudaSuccess ? FLINT_OK : cuda_fail(e, "flint_selftest_recip");
+}
+
 int flint_probe_fp64_peak(double* tflops) {
   if (!tflops) return fail(FLINT_ERR_ARG, "NULL argument");
   cudaError_t e = probe_fp64(tflops);

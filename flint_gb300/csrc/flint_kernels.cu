@@ -503,6 +503,22 @@ cudaError_t launch_log_selftest(const uint8_t* img, const ImageLayout& L, int64_
   return cudaGetLastError();
 }
 
+__global__ void k_recip_selftest(int64_t n, const double* __restrict__ x, double* __restrict__ y) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    y[4 * i] = recip(x[i]);
+    y[4 * i + 1] = 1.0 / x[i];
+    y[4 * i + 2] = sqrt_fast(x[i]);
+    y[4 * i + 3] = sqrt(x[i]);
+  }
+}
+
+cudaError_t launch_recip_selftest(int64_t n, const double* x, double* y, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  k_recip_selftest<<<256, 256, 0, st>>>(n, x, y);
+  count_launch();
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- FP64 probe
 // Independent FMA chains: the FP64 pipe's throughput, the denominator of the
 // FP64 roofline the benchmarks report.

@@ -87,21 +87,6 @@ constexpr int MSBP = 20;
 constexpr int MSBJ = 50;
 constexpr int JSLOT = 32 * 32;   // doubles per saved-Jacobian slot of up to 31 species
 
-// sqrt(x) of a non-negative x: the SM's reciprocal square root (about 2^-20) and
-// one third-order (Householder) step, 5 FP64 operations where the library's takes
-// about 9 FP64-pipe slots; relative error below 2^-52.  Zero, subnormal, huge,
-// inf and NaN take the library's.
-static __device__ __noinline__ double sqrt_slow(double x) { return sqrt(x); }
-__device__ __forceinline__ double sqrt_fast(double x) {
-  const uint32_t h = (uint32_t)__double2hiint(x);
-  if (h - 0x03000000u >= 0x79000000u) return sqrt_slow(x);
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double t = x * r;
-  const double e = fma(-t, r, 1.0);                     // 1 - x r^2
-  return fma(t * e, fma(0.375, e, 0.5), t);
-}
-
 // a < b, a <= b of doubles that are not negative (NaN: false), as bit patterns:
 // an FP64 compare costs as much as a DADD.
 __device__ __forceinline__ bool lt_pos(double a, double b) {

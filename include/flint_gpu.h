@@ -511,6 +511,11 @@ int flint_selftest_exp(flint_mech_t mech, int64_t n, const double* x, double* y,
  * kernels' log against the CUDA library. */
 int flint_selftest_log(flint_mech_t mech, int64_t n, const double* x, double* y, void* stream);
 
+/* Diagnostic: y[4i] = the kernels' 1/x[i], y[4i+1] = CUDA's, y[4i+2] = the
+ * kernels' sqrt(x[i]), y[4i+3] = CUDA's (device pointers).  No reference
+ * counterpart: lets tests bound both. */
+int flint_selftest_recip(int64_t n, const double* x, double* y, void* stream);
+
 /* Number of kernels the library launched since load (instrumentation). */
 int64_t flint_kernel_launch_count(void);
 
