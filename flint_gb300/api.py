@@ -228,6 +228,12 @@ class Chemistry:
                      "flint_reactor_autotune_times")
         return {int(lays[i]): float(ms[i]) for i in range(min(cnt.value, 8))}
 
+    def wdot_kernel(self, n):
+        """Which kernel serves wdot of n cells: "small", "cell" (a thread per cell) or "warp"."""
+        k = C.c_int(0)
+        native.check(self.L.flint_wdot_kernel(self.h, n, C.byref(k)), "flint_wdot_kernel")
+        return ("small", "cell", "warp")[k.value]
+
     def wdot_autotune(self, T, p, Y):
         """Time the source-term kernels at each block size on these cells (device
         tensors, cell-major) and keep the fastest; returns the handle's tuning."""

@@ -5,7 +5,8 @@ What is tuned (all of it empirically, on a sample of the caller's own cells):
 * the reactor's layout (``flint_reactor_autotune``: shared-memory or global
   Newton matrices, 8 or 4 warps per block, one or two blocks per SM);
 * the threads per block of the warp-per-cell source-term kernels, for wdot and
-  for wdot + Jacobian (``flint_wdot_autotune``: 64, 128 or 256);
+  for wdot + Jacobian (``flint_wdot_autotune``: 64, 128 or 256; 0, the default, for
+  wdot where a thread-per-cell kernel serves the sample);
 * which kernel serves wdot, and which wdot + Jacobian: the data-driven warp
   kernels of the library or the per-mechanism generated ones (``ytf_cuda``,
   every coefficient a literal, thread per cell), when nvcc is there to build

@@ -1131,6 +1131,14 @@ int flint_tuning_set(flint_mech_t h, const flint_tuning* t) {
   return FLINT_OK;
 }
 
+int flint_wdot_kernel(flint_mech_t h, int64_t n, int* kernel) {
+  int rc = check_common(h, n, FLINT_CELL_MAJOR);
+  if (rc) return rc;
+  if (!kernel) return fail(FLINT_ERR_ARG, "NULL argument");
+  *kernel = wdot_kernel(h->L, n);
+  return FLINT_OK;
+}
+
 int flint_wdot_autotune(flint_mech_t h, int64_t n, const double* T, const double* p, const double* Y,
                         flint_tuning* out, void* stream) {
   int rc = check_common(h, n, FLINT_CELL_MAJOR);
@@ -1154,7 +1162,7 @@ int flint_wdot_autotune(flint_mech_t h, int64_t n, const double* T, const double
   int best_w = 0, best_j = 0;
   float tw = 0.f, tj = 0.f;
   for (int jac = 0; jac < 2 && !e; ++jac) {
-    if (!jac && use_small_kernel(h->L)) continue;   // the thread-per-cell kernel serves this mechanism
+    if (!jac && wdot_kernel(h->L, n) != FLINT_WDOT_WARP) continue;   // a kernel without this choice serves the sample
     for (int c = 0; c < nc && !e; ++c) {
       float ms = 0.f;
       for (int rep = 0; rep < 3 && !e; ++rep) {   // the first run of each block size warms up

@@ -71,6 +71,7 @@ cudaError_t launch_wdot_cell(const uint8_t* img, const ImageLayout& L, int64_t n
                              cudaStream_t st);
 int warp_block_candidates(int* out);
 bool use_small_kernel(const ImageLayout& L);   // wdot of <= 8 species: thread per cell
+int wdot_kernel(const ImageLayout& L, int64_t n);   // FLINT_WDOT_*: what launch_wdot takes for n cells
 cudaError_t launch_species_thermo(const uint8_t* img, const ImageLayout& L, int64_t n, const double* T, double* cp,
                                   double* h, double* s, double* g, cudaStream_t st);
 cudaError_t launch_thermo(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,

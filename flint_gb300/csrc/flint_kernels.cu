@@ -759,12 +759,17 @@ static cudaError_t launch_small(const uint8_t* img, const ImageLayout& L, int64_
 
 bool use_small_kernel(const ImageLayout& L) { return L.ns <= SMALL_NSMAX && L.ns <= 8; }
 
+int wdot_kernel(const ImageLayout& L, int64_t n) {
+  return use_small_kernel(L) ? FLINT_WDOT_SMALL : use_cell_kernel(L, n) ? FLINT_WDOT_CELL : FLINT_WDOT_WARP;
+}
+
 cudaError_t launch_wdot(const uint8_t* img, const ImageLayout& L, int64_t n, int layout, const double* T,
                         const double* p, const double* Y, double* wdot, double* cp, double* h,
                         cudaStream_t st, int threads) {
   if (n <= 0) return cudaSuccess;
-  if (use_small_kernel(L)) return launch_small(img, L, n, layout, T, p, Y, wdot, cp, h, 0, nullptr, st);
-  if (use_cell_kernel(L, n)) return launch_wdot_cell(img, L, n, layout, T, p, Y, wdot, cp, h, false, 0, st);
+  const int kernel = wdot_kernel(L, n);
+  if (kernel == FLINT_WDOT_SMALL) return launch_small(img, L, n, layout, T, p, Y, wdot, cp, h, 0, nullptr, st);
+  if (kernel == FLINT_WDOT_CELL) return launch_wdot_cell(img, L, n, layout, T, p, Y, wdot, cp, h, false, 0, st);
   return launch_warp<false, false>(img, L, n, layout, T, p, Y, wdot, cp, h, nullptr, nullptr, nullptr, st, 0, threads);
 }
 

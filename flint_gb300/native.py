@@ -124,6 +124,7 @@ def lib():
     L.flint_reactor_autotune_times.argtypes = [vp, _ip, C.POINTER(C.c_float), C.c_int, _ip]
     L.flint_tuning_get.argtypes = [vp, C.POINTER(Tuning)]
     L.flint_tuning_set.argtypes = [vp, C.POINTER(Tuning)]
+    L.flint_wdot_kernel.argtypes = [vp, i64, _ip]
     L.flint_wdot_autotune.argtypes = [vp, i64, vp, vp, vp, C.POINTER(Tuning), vp]
     L.flint_probe_fp64_peak.argtypes = [C.POINTER(C.c_double)]
     L.flint_selftest_exp.argtypes = [vp, i64, vp, vp, vp]

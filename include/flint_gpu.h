@@ -346,11 +346,20 @@ int flint_tuning_get(flint_mech_t mech, flint_tuning* tuning);
  * block size that does not fit this mechanism on the current device is
  * refused (FLINT_ERR_ARG) and nothing changes. */
 int flint_tuning_set(flint_mech_t mech, const flint_tuning* tuning);
-/* Empirical choice of the source-term kernels' block size: times
+/* Which kernel serves flint_wdot_batch for n cells of this mechanism on the
+ * current device: a thread per cell of a small mechanism, a thread per cell of a
+ * large batch, or a warp per cell.  Instrumentation, no reference counterpart. */
+#define FLINT_WDOT_SMALL 0
+#define FLINT_WDOT_CELL 1
+#define FLINT_WDOT_WARP 2
+int flint_wdot_kernel(flint_mech_t mech, int64_t n, int* kernel);
+/* Empirical choice of the warp-per-cell source-term kernels' block size: times
  * flint_wdot_batch and flint_wdot_jac_batch at every block size on a sample
  * of cells (n of them, device arrays, cell-major; outputs go to private
  * buffers), keeps the fastest for this handle and reports the handle's tuning
- * in *tuning (may be NULL).  No reference counterpart. */
+ * in *tuning (may be NULL).  Where a thread-per-cell kernel serves a sample of
+ * that size (flint_wdot_kernel) there is nothing to choose: wdot_threads is 0.
+ * No reference counterpart. */
 int flint_wdot_autotune(flint_mech_t mech, int64_t n, const double* T, const double* p, const double* Y,
                         flint_tuning* tuning, void* stream);
 
