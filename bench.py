@@ -71,6 +71,19 @@ def fp64_ops(ev, ns, mech_name="synthetic-31sp-160r"):
             + ev["newton"] * 2.0 * n * n)
 
 
+def kernel_and_flops(chem, n, jac, generated):
+    """The kernel that serves a source-term (or Jacobian) batch of n states and its
+    FP64 operations per state; None for a mechanism without a count."""
+    kf = (GENERATED_FLOPS if generated else KINETICS_FLOPS).get(chem.mech.name)
+    if kf is None:
+        return None
+    if generated:
+        return f"ytf_<mech>_{'jac_' if jac else ''}kernel", kf["jac" if jac else "rhs"]
+    if not jac and chem.wdot_kernel(n) == "cell":
+        return "k_wdot_cell", kf["cell"]
+    return f"k_wdot_warp<{int(jac)}>", kf["jac" if jac else "rhs"]
+
+
 def dist_env():
     from flint_gb300.dist import env
     return env()
@@ -691,13 +704,11 @@ def run_kernel_workload(args):
     nv = chem.ns + 1
     bytes_per_state = 8 * (2 + 2 * chem.ns) + (8 * nv * nv if jac is not None else 16)
     roof = None
-    kf = (GENERATED_FLOPS if gen else KINETICS_FLOPS).get(chem.mech.name)
-    if kf is not None and tab is None:
-        cell = jac is None and "cell" in kf and n >= 32768
-        fl = kf["jac" if jac is not None else "cell" if cell else "rhs"]
+    named = None if tab is not None else kernel_and_flops(chem, n, jac is not None, gen is not None)
+    if named is not None:
+        kernel, fl = named
         peak = chem_peak_fp64()
-        roof = {"bound": "fp64", "kernel": (f"ytf_<mech>_{'jac_' if jac is not None else ''}kernel" if gen else
-                                            "k_wdot_cell" if cell else f"k_wdot_warp<{int(jac is not None)}>"),
+        roof = {"bound": "fp64", "kernel": kernel,
                 "flops_note": ("the FP64 path's operations per state" if gen else
                                "FP64 operations per state (exponentials and polynomials are integer work)"),
                 "flops_per_state": fl, "achieved": n * fl / t / 1e12, "peak": peak, "unit": "TFLOP/s",
