@@ -162,7 +162,8 @@ def current_stream():
     global _raw_stream
     if _raw_stream is None:
         import torch
-        _raw_stream = (torch._C._cuda_getCurrentRawStream, torch.cuda.current_device)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # private: may be missing
+        _raw_stream = (raw or (lambda dev: torch.cuda.current_stream(dev).cuda_stream), torch.cuda.current_device)
     return C.c_void_p(_raw_stream[0](_raw_stream[1]()))
 
 
