@@ -38,6 +38,7 @@ struct TableLayout {
   // the thread-per-cell kernel's image (flint_table.cu, pack_cell): cell_bytes at
   // o_cell; offsets relative to it
   int o_cell, cell_bytes;
+  float us_round, us_pass;     // estimated times of the two kernels (use_general_cell)
   int c_head, c_fac, c_facx, c_w, c_wv, c_tp, c_t, c_te, c_tz, c_et, c_lt, c_ywm, c_wm, c_ri;
   // transport (when given): species viscosity and conductivity [row][nsp],
   // and Wilke's species-pair factors (W_i/W_j)^(1/4) and sqrt(8 (1 + W_i/W_j)) [ns][ns]
@@ -202,6 +203,17 @@ int table_pack(const flint_table_desc* d, TableLayout& L, std::vector<uint8_t>& 
       tbrow[r] = ntb++;
       for (int s = 0; s < S; ++s) effs.push_back(s < ns ? ep[s] : 0.0);
     }
+  }
+  {
+    int groups_tb = 0, groups_falloff = 0;
+    for (int r0 = 0; r0 < P; r0 += 32) {
+      bool t = false, f = false;
+      for (int r = r0; r < r0 + 32; ++r) { t |= tbrow[r] >= 0; f |= kind[r] != 0; }
+      groups_tb += t;
+      groups_falloff += f;
+    }
+    L.us_round = 1.6f + 4.25f * (P / 32) + 0.29f * ns * groups_tb + 33.6f * groups_falloff;
+    L.us_pass = 3.7f + 1.50f * nr + 1.84f * ntb + 3.73f * (nr - nra);
   }
   L.ntb = std::max(ntb, 1);
   if (effs.empty()) effs.assign(S, 0.0);
@@ -424,11 +436,24 @@ k_general_warp(const uint8_t* __restrict__ img, TableLayout L, const double* __r
 // The table rows differ from lane to lane; two reactions' entries are one 16-byte
 // load, fetched a pair ahead.
 constexpr int TC_MAX_WARPS = 12;
-// From how many cells per SM on it is the faster kernel.  A warp's pass takes 306 us
-// (31 species, 160 reactions) or 385 us (197) however few its cells; the
-// warp-per-cell kernel takes 73 and 140 us per 1,000 cells and passes that at 4,200
-// and 2,750 cells.
+// From where on it is the faster kernel.  The warp-per-cell kernel goes by rounds of 8
+// cells on every SM, and a round's time by the reactions in groups of 32 lanes, the
+// groups with a third body (a sum over the species) and those with falloff; a pass of
+// this kernel takes the same time for any number of cells up to 32 on every warp, by the
+// reactions, third bodies and falloff reactions.  Fits of 15 mechanisms of 5-31 species
+// and 2-197 reactions, both kernels measured at 3,600-22,000 cells, within 13 % and 8 %
+// (31 species, 160 reactions, 6 of them falloff: 72 us a round, 308 a pass; without
+// those 32 and 263; 185 without falloff 53 and 291; 28 reactions 11 and 68):
+//   round = 1.6 + 4.25 groups + 0.29 ns groups_tb + 33.6 groups_falloff   [us]
+//   pass  = 3.7 + 1.50 nr + 1.84 third bodies + 3.73 falloff
+// and from three rounds on, below which neither was measured.  (One line at three rounds
+// had cost the mechanism without falloff a factor of two up to 8,600 cells.)
 constexpr int64_t TC_CELLS_PER_SM = 24;
+
+static bool use_general_cell(const TableLayout& L, int64_t n) {
+  const int64_t sms = device_sms(), rounds = (n + 8 * sms - 1) / (8 * sms);
+  return n >= TC_CELLS_PER_SM * sms && (float)rounds * L.us_round >= L.us_pass;
+}
 
 __device__ __forceinline__ double tc_ipow(double x, int n) {
   if (n == 1) return x;
@@ -621,7 +646,7 @@ cudaError_t launch_general(const uint8_t* img, const TableLayout& L, const doubl
                            const double* roi, const double* T, double* out, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int wmax = tc_warps(L, L.cell_bytes);
-  if (wmax >= 4 && n >= TC_CELLS_PER_SM * (int64_t)device_sms()) {
+  if (wmax >= 4 && use_general_cell(L, n)) {
     const int64_t tasks = (n + 31) / 32, sms = device_sms();
     const int w = (int)std::min<int64_t>(wmax, (tasks + sms - 1) / sms);
     const size_t smc = L.cell_bytes + (size_t)w * (L.ns + 1) * TC_ROW * sizeof(double);
