@@ -299,9 +299,11 @@ static int cell_warps(const ImageLayout& L, int staged) {
 // time, about 145 per SM (thread against warp: 20,000 cells 136 against
 // 125 us, 24,000 136 against 146, 32,000 145 against 193; 197 reactions: 20,000 167
 // against 152, 24,000 167 against 177).  At 1 M cells it takes 4.6 ms against 6.1.
+// Mechanisms of 13-25 species and 44-110 reactions could change earlier: 56-112 us at
+// 22,100 cells, where the warp kernel takes 83-123 at 20,000.
 // With 4 resident warps (54 species) there is too little to hide latencies
-// behind (100,003 cells: 1.37 ms against 1.28 with the warp kernel of that time), so
-// six or more are asked for.
+// behind (100,003 cells: 1.37 ms against 0.97 with the warp kernel), so six or more are
+// asked for.
 bool use_cell_kernel(const ImageLayout& L, int64_t n) {
   const int64_t sms = device_sms(), w = cell_warps(L, L.fix_bytes_cell);
   if (!L.fix || w < 6 || scratch_small_doubles(L) > cell_warp_doubles(L.ns)) return false;

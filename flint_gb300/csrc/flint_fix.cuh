@@ -9,11 +9,16 @@
 // *absolute* error matters, which is what fixed point gives: with 52 fraction
 // bits an argument carries an absolute error of about 2^-52, where the FP64
 // chain it replaces rounds at every step to 2^-53 of a magnitude of 10-60.
-// The result is therefore closer to the exact value, not further from it.
+// The exponent is therefore closer to the exact value, not further from it.  (Outside
+// the exponents the kernels trade a division for a product by a reciprocal, two
+// roundings for one; against 64-bit references the rates, Jacobians and right-hand
+// sides come out closer all the same.)
 //
 // All logarithms are base 2.  Formats (Qn: n fraction bits in 64 bits):
 //   exponents (log2 k, g/RT in octaves)   Q52 signed   |x| < 2^11
 //   log2 T - 7                            Q61 unsigned, T in [129, 8192)
+//   log2 c of a factor to a power         Q57 signed within 2^+-63, Q53 beyond
+//   orders of such factors                Q60 unsigned, below 16
 //   1/T                                   Q70 unsigned (T > 128)
 //   T/2^13 (high range), T/2^11 (low)     Q63 unsigned
 //   E log2e (kelvin)                      Q45 signed   |x| < 2^18
@@ -145,8 +150,8 @@ __host__ __device__ __forceinline__ double fix2d(int64_t X, int q) {
   return X == 0 ? 0.0 : bits_d((int64_t)((uint64_t)bits | sgn));
 }
 
-// A double as Q52, saturated to |x| < 2^11 (rounded towards minus infinity
-// below 2^-52; NaN saturates).
+// A double as Q52, saturated to |x| < 2^11 (cut towards zero below 2^-52; NaN
+// saturates).
 __host__ __device__ __forceinline__ int64_t d2fix52(double x) {
   const int64_t b = d_bits(x);
   const int e = (int)((b >> 52) & 0x7ff) - 1023;

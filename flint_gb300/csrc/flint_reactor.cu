@@ -819,7 +819,8 @@ static int slots_of(const ImageLayout& L, int layout) {
 // WIDE's rule.  31 species, 8 against 12 warps on an SM: 89.5 / 106 ms at 2,432 cells,
 // 164 / 157 at 4,096, 298 / 287 at 8,192, 592 / 537 at 16,384 (a round of 12 warps takes
 // longer than one of 8, and 168 registers spill a little): from two rounds of 12 warps on
-// every SM.
+// every SM.  (Between 1,217 and 1,824 cells, one round of 12 warps but two of 8, neither
+// was measured against the other.)
 // Where the count is only on the device it may be far below n (the cells that a
 // surrogate leaves): 8 warps.
 static bool reactor_wide(const ImageLayout& L, int64_t n, bool n_on_device) {
